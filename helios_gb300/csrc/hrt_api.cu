@@ -546,7 +546,7 @@ const char *variant_name(int v) {
 int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *variant) {
     const int nf = ((P0.faces & 1) ? 1 : 0) + ((P0.faces & 2) ? 1 : 0);
     const long long rays = (long long)P0.count * P0.dimx * P0.dimy * nf;
-    *variant = record ? (P0.sc.nodes4 ? DV_W4 : DV_PS3) : DV_DEFAULT;
+    *variant = record ? (P0.sc.nodes4 ? DV_W4S4D16 : DV_PS3) : DV_DEFAULT;
     if (ctx->tune >= 16) {  // forced variant (tests, experiments)
         const int v = ctx->tune - 16;
         if (!(record && v == DV_SIMPLE)) *variant = v;
@@ -1731,7 +1731,7 @@ struct SweepPlan {
     bool scattering = false, any_direct = false, any_diffuse = false, any_copy0 = false, any_active = false;
     int dimx = 0, dimy = 0, ddx = 0, ddy = 0, Rd = 0, depth = 0;
     uint32_t seed = 0, rec_per = 0;
-    int rec_variant = DV_W4;
+    int rec_variant = DV_W4S4D16;
     float *d_sun = nullptr, *d_flux = nullptr, *d_sky = nullptr, *d_zero = nullptr;
     uint8_t *m_all = nullptr, *m_fold = nullptr, *m_diff = nullptr, *m_copy0 = nullptr, *m_active = nullptr;
     float *d_rho = nullptr, *d_tau = nullptr;
@@ -1839,7 +1839,7 @@ int sweep_prepare(hrt_context *ctx, const hrt_sweep *s, bool tune, SweepPlan *pl
     CU(ctx->Gd.ensure(ctx->stream, std::max<size_t>((size_t)n * nsun * 2, 1) * sizeof(double)));
     CU(ctx->fetch.ensure(ctx->stream, sizeof(unsigned long long)));
     // choose the recording kernel's variant before capture (timing cannot run inside a capture)
-    P.rec_variant = ctx->n4 > 0 ? DV_W4 : DV_PS3;
+    P.rec_variant = ctx->n4 > 0 ? DV_W4S4D16 : DV_PS3;
     if (tune && P.Rd > 0 && (P.any_diffuse || P.any_active)) {
         DiffuseParams T0{};
         T0.sc = scene_of(ctx);

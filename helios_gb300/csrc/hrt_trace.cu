@@ -720,12 +720,15 @@ static cudaError_t direct_impl(const DirectParams &p, int max_blocks, cudaStream
     return cudaGetLastError();
 }
 
-// Default diffuse variant: the persistent 4-wide traversal; HRT_TRAVERSAL=simple selects
-// the one-ray-per-thread kernel and HRT_TRAVERSAL=bvh2 the persistent binary traversal.
+// Default diffuse variant: the lean persistent 4-wide traversal with 16 shared stack entries (scenes
+// with voxels: the generic one), the tuner's choice at every size it has timed and 10-20 % faster
+// than the generic trace, which small passes, below the tuner's limit, used to run;
+// HRT_TRAVERSAL=simple selects the one-ray-per-thread kernel and HRT_TRAVERSAL=bvh2 the persistent
+// binary traversal.
 static int default_variant() {
     static const int v = [] {  // initialised once, thread-safe
         const char *e = getenv("HRT_TRAVERSAL");
-        return (e && e[0] == 's') ? DV_SIMPLE : ((e && e[0] == 'b') ? DV_PS4 : DV_W4);
+        return (e && e[0] == 's') ? DV_SIMPLE : ((e && e[0] == 'b') ? DV_PS4 : DV_W4S4D16);
     }();
     return v;
 }

@@ -142,6 +142,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
     // a lane budget retires lanes without drawing ids, so a warp could leave ids of its
     // batch untraced: batched fetch only without one
     const bool batched = KB > 1 && P.lane_budget == 0;
+    // The first ray id of a lane is its thread's index, later ones come from the counter: a launch
+    // of few rays per lane does not begin with every warp's atomic on one address.
+    bool fresh = true;
     if (KB > 1 && lane == 0) {
         s_chunk[0][tid >> 5] = 0ull;
         s_chunk[1][tid >> 5] = 0ull;
@@ -159,9 +162,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             const unsigned rank = __popc(m & ((1u << lane) - 1u));
             unsigned long long id;
             if (!batched) {
-                unsigned long long base = 0;
-                if (lane == leader) base = atomicAdd(P.fetch, (unsigned long long)__popc(m));
-                base = __shfl_sync(0xffffffffu, base, leader);
+                unsigned long long base;
+                if (fresh) {
+                    base = (unsigned long long)blockIdx.x * BLOCK + (tid & ~31);
+                    fresh = false;
+                } else {
+                    base = 0;
+                    if (lane == leader) base = atomicAdd(P.fetch, (unsigned long long)__popc(m));
+                    base = __shfl_sync(0xffffffffu, base, leader) + (unsigned long long)gridDim.x * BLOCK;
+                }
                 id = base + rank;
             } else {
                 // ids are handed out in increasing order, so every id below the end of the
@@ -478,12 +487,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         for (int i = tid; i < P.nslots; i += BLOCK)
             if (s_srays[i] && s_slot[i].sc.rays) atomicAdd(s_slot[i].sc.rays, s_srays[i]);
     } else {
-        if (P.sc.rays && nrays) atomicAdd(P.sc.rays, (unsigned long long)nrays);
+        add_rays(P.sc, nrays);
     }
-    if (STATS && P.sc.visits) {
-        atomicAdd(P.sc.visits, (unsigned long long)nvis);
-        atomicAdd(P.sc.visits + 1, (unsigned long long)ntest);
-    }
+    if (STATS) count_visits(P.sc, nvis, ntest);
 #undef POP
 #undef SC
 }
