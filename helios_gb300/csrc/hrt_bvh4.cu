@@ -39,28 +39,37 @@ __device__ __forceinline__ float half_area(const Box &b) {
     return dx * dy + dy * dz + dz * dx;
 }
 
-// Smallest step s = 2^(e-127) with p + 255 s >= hi (FP32, as decoded); e in [1, 254].
-__device__ __forceinline__ uint32_t pick_exponent(float p, float hi) {
-    float x = (hi - p) * (1.0f / 255.0f);
+// Largest FP32 p with p + S <= lo: the origin of a node frame of extent S whose plane 0 is not
+// above lo.
+__device__ __forceinline__ float frame_origin(float lo, float S) {
+    float p = lo - S;
+    while (p + S > lo) p = nextafterf(p, -INFINITY);
+    return p;
+}
+
+// Smallest extent S = 2^(e-127) whose frame over lo reaches hi at plane 255; e in [9, 254].
+__device__ __forceinline__ uint32_t pick_exponent(float lo, float hi) {
+    float x = (hi - lo) * (256.0f / 255.0f);
     uint32_t bits = __float_as_uint(x);
     uint32_t e = (bits >> 23) & 0xFFu;
     if (bits & 0x7FFFFFu) e += 1;
-    if (e < 1) e = 1;
-    while (e < 254 && !(q_decode(p, 255u, q_step(e)) >= hi)) ++e;
+    if (e < 9) e = 9;
+    while (e < 254 && !(q_decode(frame_origin(lo, q_step(e)), 255u, q_step(e)) >= hi)) ++e;
     return e;
 }
 
-__device__ __forceinline__ uint32_t quant_lo(float p, float v, float s) {
-    float f = floorf((v - p) / s);
+// Planes of a frame of origin p and extent S at or below / at or above v (lo: its plane 0's bound)
+__device__ __forceinline__ uint32_t quant_lo(float p, float lo, float v, float S) {
+    float f = floorf((v - lo) * 256.0f / S);
     int q = f < 0.f ? 0 : (f > 255.f ? 255 : (int)f);
-    while (q > 0 && q_decode(p, (uint32_t)q, s) > v) --q;
+    while (q > 0 && q_decode(p, (uint32_t)q, S) > v) --q;
     return (uint32_t)q;
 }
 
-__device__ __forceinline__ uint32_t quant_hi(float p, float v, float s) {
-    float f = ceilf((v - p) / s);
+__device__ __forceinline__ uint32_t quant_hi(float p, float lo, float v, float S) {
+    float f = ceilf((v - lo) * 256.0f / S);
     int q = f < 0.f ? 0 : (f > 255.f ? 255 : (int)f);
-    while (q < 255 && q_decode(p, (uint32_t)q, s) < v) ++q;
+    while (q < 255 && q_decode(p, (uint32_t)q, S) < v) ++q;
     return (uint32_t)q;
 }
 
@@ -110,7 +119,7 @@ __global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float
         child_box(n2, c, 1, &box[cnt]);
         ++cnt;
     }
-    // node box and steps over the children that exist
+    // node box, frame extents and origin over the children that exist
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int k = 0; k < cnt; ++k) {
         if (ref[k] == kEmptyChild) continue;
@@ -122,8 +131,11 @@ __global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float
     if (!(lo[0] <= hi[0])) {  // no child: cannot happen for a built tree
         for (int a = 0; a < 3; ++a) lo[a] = hi[a] = 0.f;
     }
-    float s[3];
-    for (int a = 0; a < 3; ++a) s[a] = q_step(pick_exponent(lo[a], hi[a]));
+    float s[3], p[3];
+    for (int a = 0; a < 3; ++a) {
+        s[a] = q_step(pick_exponent(lo[a], hi[a]));
+        p[a] = frame_origin(lo[a], s[a]);
+    }
     uint32_t wlo[3] = {0, 0, 0}, whi[3] = {0, 0, 0};
     int32_t outref[4] = {kEmptyChild, kEmptyChild, kEmptyChild, kEmptyChild};
     // The internal children of a node get consecutive indices from one allocation, padded to
@@ -144,8 +156,8 @@ __global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float
             continue;
         }
         for (int a = 0; a < 3; ++a) {
-            wlo[a] |= quant_lo(lo[a], box[k].lo[a], s[a]) << (8 * k);
-            whi[a] |= quant_hi(lo[a], box[k].hi[a], s[a]) << (8 * k);
+            wlo[a] |= quant_lo(p[a], lo[a], box[k].lo[a], s[a]) << (8 * k);
+            whi[a] |= quant_hi(p[a], lo[a], box[k].hi[a], s[a]) << (8 * k);
         }
         if (c < 0) {
             outref[k] = c;  // leaf: ~slot
@@ -161,7 +173,7 @@ __global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float
         }
     }
     float4 *o = n4 + 4 * (size_t)q;
-    o[0] = make_float4(lo[0], lo[1], lo[2], s[0]);
+    o[0] = make_float4(p[0], p[1], p[2], s[0]);
     o[1] = make_float4(__uint_as_float(wlo[0]), __uint_as_float(wlo[1]), __uint_as_float(wlo[2]),
                        __uint_as_float(whi[0]));
     o[2] = make_float4(__uint_as_float(whi[1]), __uint_as_float(whi[2]), __int_as_float(outref[0]),

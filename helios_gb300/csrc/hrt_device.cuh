@@ -311,21 +311,23 @@ __device__ __forceinline__ f3 sample_point(const float4 g[4], uint32_t type, flo
 
 // ------------------------------------------------------- compressed 4-wide BVH ---
 // Node (64 B, two 256-bit loads):
-//   q0 = (px, py, pz, sx)       origin p (the node box's lower corner) and the x step
+//   q0 = (px, py, pz, Sx)       origin p and the x extent S of the node's quantised frame
 //   q1 = (lox, loy, loz, hix)   quantised child boxes, byte k = child k (0 <= q <= 255)
 //   q2 = (hiy, hiz, c0, c1)     child refs c_k: >= 0 node, ~slot leaf, kEmptyChild none
-//   q3 = (c2, c3, sy, sz)       the y and z steps
-// Each step s = 2^(e - 127) is a power of two (e in [1, 254]), stored as a float so that the
-// test reads it without decoding.
+//   q3 = (c2, c3, Sy, Sz)       the y and z extents
+// A plane byte q stands for v = 1 + q / 256, which is a float whose bits are 1.0's plus q << 15, and
+// for the coordinate p + v S: S is a power of two and p lies S below the node box's lower corner, so
+// v = 1 is that corner and a step is S / 256.  A ray's slab test then is one dot product of two
+// bytes (q << 15 added to 1.0's bits, q_frac) and one fused multiply-add per plane.
 // An empty child slot has lo bytes 255 and hi bytes 0: an inverted box that no ray enters.
-// On every axis the slab slope a = inv * s is nonzero (|inv| >= 1 for a unit direction,
-// s >= 2^-126), so the near plane lies beyond the far plane; an infinite slope gives a NaN
-// plane, which the min/max skip, and an infinite near or far plane, which fails the test.
-// Child k's box per axis: [p + lo_k * s, p + hi_k * s] in FP32 (q * s is exact; one rounded
-// add).  The build picks the bytes so that these values enclose the child's FP32 box (itself
-// padded), so a slab test on the decoded box never culls an accepted hit (after Ylitie,
-// Karras, Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs",
-// HPG 2017, with 4 children per node).
+// On every axis the slab slope a = inv * S is nonzero (|inv| >= 1 for a unit direction,
+// S >= 2^-118), so the near plane lies beyond the far plane; an infinite slope gives a NaN or
+// infinite plane, which the min/max skip or which fails the test.
+// Child k's box per axis: [p + (1 + lo_k / 256) S, p + (1 + hi_k / 256) S] in FP32 (the product is
+// exact; one rounded add).  The build picks p, S and the bytes so that these values enclose the
+// child's FP32 box (itself padded by more than the slab test's rounding), so a slab test on the
+// decoded box never culls an accepted hit (after Ylitie, Karras, Laine, "Efficient Incoherent Ray
+// Traversal on GPUs Through Compressed Wide BVHs", HPG 2017, with 4 children per node).
 __device__ __forceinline__ float q_step(uint32_t e) { return __uint_as_float(e << 23); }
 
 // Unsigned 32-bit division by a divisor fixed for a launch, by multiplication (Granlund and
@@ -361,8 +363,18 @@ __device__ __forceinline__ void load_node64(const float4 *nodes, int32_t i, floa
         : "=f"(q2.x), "=f"(q2.y), "=f"(q2.z), "=f"(q2.w), "=f"(q3.x), "=f"(q3.y), "=f"(q3.z), "=f"(q3.w)
         : "l"(a + 2));
 }
-__device__ __forceinline__ float q_decode(float p, uint32_t q, float s) { return p + (float)q * s; }
-__device__ __forceinline__ uint32_t q_byte(uint32_t w, int k) { return (w >> (8 * k)) & 0xFFu; }
+// Plane q of a node frame of origin p and extent S (the build's and the tests' value of it).
+__device__ __forceinline__ float q_decode(float p, uint32_t q, float S) { return p + (1.0f + (float)q * 0.00390625f) * S; }
+// 1 + q / 256 of byte k of w.  The 16 x 8 bit dot product runs beside the ALU pipe, which bounds
+// the node loop; a byte permute would add to it.
+__device__ __forceinline__ float q_frac(uint32_t w, int k) {
+    const uint32_t one = 0x3F800000u;
+    const uint32_t v = k == 0   ? __dp2a_lo(0x00008000u, w, one)
+                       : k == 1 ? __dp2a_lo(0x80000000u, w, one)
+                       : k == 2 ? __dp2a_hi(0x00008000u, w, one)
+                                : __dp2a_hi(0x80000000u, w, one);
+    return __uint_as_float(v);
+}
 // Three-input minimum / maximum (PTX min.f32 / max.f32 with three sources; a NaN input
 // is ignored, as by fminf / fmaxf).
 __device__ __forceinline__ float fmin3(float a, float b, float c) {
@@ -375,11 +387,6 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-// Byte k of w as an exact float: one byte permute builds 0x4B0000qq = 2^23 + q.
-__device__ __forceinline__ float q_float(uint32_t w, int k) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, (uint32_t)k | 0x7540u)) - 8388608.0f;
-}
-
 // Packed FP32 pairs (PTX .f32x2 on sm_100 and later): one instruction applies the same
 // IEEE operation (round to nearest) to both halves of a 64-bit register pair.
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
@@ -395,16 +402,6 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// Byte k of w as the float 2^23 + q (q_float before its subtraction).
-__device__ __forceinline__ float q_biased(uint32_t w, int k) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, (uint32_t)k | 0x7540u));
-}
-
 // Leaf-box padding: each face moves out by (|x| + extent) * 2^-20.
 __device__ __forceinline__ float pad_lo(float x, float ext) { return x - (fabsf(x) + ext) * 9.5367431640625e-07f; }
 __device__ __forceinline__ float pad_hi(float x, float ext) { return x + (fabsf(x) + ext) * 9.5367431640625e-07f; }

@@ -39,3 +39,34 @@ def test_rays_through_edges_and_corners(gpu, oracle_mod, div):
     assert (h2 >= 0).any()
     assert np.array_equal(h1, h2) and np.array_equal(f1, f2)
     assert np.array_equal(t1[h1 >= 0], t2[h2 >= 0])
+
+
+@pytest.mark.parametrize("scale,offset", [(1e-3, 0.0), (1.0, 0.0), (1.0, 3.0e4), (1e4, 0.0)])
+def test_wide_nodes_enclose_their_children(gpu, oracle_mod, scale, offset):
+    """The quantised 4-wide nodes cull no accepted hit at small and large sizes and far from the
+    origin of coordinates: fluxes and ray counts of a solve over them equal the oracle's."""
+    from helios_gb300.radiation import Context, RadiationModel
+    from helpers import run_oracle
+
+    sc = scenes.mixed_canopy(700, 2.0, seed=5)
+    T = sc.T.reshape(-1, 4, 4).astype(np.float64)
+    T[:, :3, :] *= scale
+    T[:, :2, 3] += offset
+    ctx = Context()
+    uu = ctx.addPrimitives(T.reshape(-1, 16).astype(np.float32), sc.ptype, sc.area * scale ** 2, sc.twosided)
+    ctx.setPrimitiveData(uu, "reflectivity_SW", np.full(uu.size, 0.3))
+    rad = RadiationModel(ctx)
+    rad.addRadiationBand("SW")
+    rad.disableEmission("SW")
+    sun = rad.addCollimatedRadiationSource(scenes.sun_direction(40.0, 100.0))
+    rad.setSourceFlux(sun, "SW", 500.0)
+    rad.setDiffuseRadiationFlux("SW", 80.0)
+    rad.setDirectRayCount("SW", 36)
+    rad.setDiffuseRayCount("SW", 49)
+    rad.setScatteringDepth("SW", 1)
+    rad.setSeed(11)
+    got = rad.runBand("SW").astype(np.float64)
+    ref, st = run_oracle(rad, ["SW"], oracle_mod, seed=11)
+    floor = 1e-3 * float(np.abs(ref).mean())
+    assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
+    assert rad.last_stats["rays"] == st["rays"]
