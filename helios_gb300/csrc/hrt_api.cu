@@ -125,6 +125,11 @@ struct hrt_context {
     DevBuf rin, stop, sbot, otop, obot, ftop, fbot, Gd, Gt, Gb, flags, sky, fin, status, counter, emis, emis_eps, emis_T,
         fetch;
     size_t emis_eps_count = 0, emis_T_count = 0;
+    // grids across the collimated sources of a direct pass, and what they need of the geometry
+    // (ordered bounds and extent sums of the records, once per geometry)
+    DevBuf sg_cells, sg_entries, sg_grids, sg_extent, sg_done;
+    bool sg_extent_ready = false;
+    std::vector<int> h_src_type;
     DevBuf io_a, io_b, io_c;  // staging for inspection calls
     uint64_t last_rays = 0, last_kernels = 0, last_iters = 0;
     DevBuf resid;  // scattering residual: block partials and the per-band result
@@ -436,6 +441,38 @@ GlassParams glass_params(hrt_context *ctx, int Bg, int Bl) {
     return g;
 }
 
+// Buffers of the grids of `nsrc` collimated sources and the scene's extent (queued on the context's
+// stream); *nb: sources per batch.
+int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
+    const SunCaps caps = sun_caps(ctx->n);
+    *nb = std::max(1, std::min(caps.batch, nsrc));
+    CU(ctx->sg_cells.ensure(ctx->stream, (size_t)*nb * caps.cells * sizeof(uint2)));
+    CU(ctx->sg_entries.ensure(ctx->stream, (size_t)*nb * caps.entries * sizeof(uint2)));
+    CU(ctx->sg_grids.ensure(ctx->stream, (size_t)kSunBatch * sizeof(SunGrid)));
+    CU(ctx->sg_done.ensure(ctx->stream, (size_t)std::max(nsrc, 1) * sizeof(uint32_t)));
+    CU(ctx->sg_extent.ensure(ctx->stream, 9 * sizeof(uint32_t)));
+    if (!ctx->sg_extent_ready) {
+        CU(launch_scene_extent(ctx->n, ctx->rec.as<float4>(), ctx->sg_extent.as<uint32_t>(), ctx->stream));
+        ctx->sg_extent_ready = true;
+    }
+    return HRT_OK;
+}
+
+// Whether a direct pass of `rays` rays per source bins its collimated sources (hrt_sungrid.cu).
+// Statistics launches count the tree's visits and a lowered visit budget is meant for the tree.
+bool sun_grids_pay(hrt_context *ctx, unsigned long long rays) {
+    return !(ctx->measure & 1) && ctx->visit_budget == 0 && rays >= kSunMinRays;
+}
+
+void fill_sun_params(hrt_context *ctx, SunDirectParams *D) {
+    const SunCaps caps = sun_caps(ctx->n);
+    D->grids = ctx->sg_grids.as<SunGrid>();
+    D->cells = ctx->sg_cells.as<uint2>();
+    D->entries = ctx->sg_entries.as<uint2>();
+    D->cells_cap = caps.cells;
+    D->entries_cap = caps.entries;
+}
+
 // Direct pass + epilogue (__raygen__direct / __miss__direct).
 int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp, uint32_t seed, uint32_t pass, int Bg,
                 int Bc, int Bl) {
@@ -462,6 +499,7 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
     P.offset = offset;
     P.count = count;
     P.G = ctx->Gd.as<double>();
+    P.done = nullptr;
     P.gl = GlassParams{};
     const uint32_t *cov = nullptr;
     int r;
@@ -480,7 +518,42 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
     const uint32_t per = chunk_prims(ctx, (uint64_t)dimx * (uint64_t)dimy);
     if (per == 0) return HRT_EUNSUPPORTED;
     uint32_t chunks = 0;
+    const bool grids = !cov && sun_grids_pay(ctx, (unsigned long long)count * (unsigned)(dimx * dimy)) &&
+                       std::find(ctx->h_src_type.begin(), ctx->h_src_type.end(), 0) != ctx->h_src_type.end();
+    int batch = 1;
+    if (grids) {
+        if ((r = ensure_sun_grids(ctx, ctx->S, &batch))) return r;
+        CU(cudaMemsetAsync(ctx->sg_done.p, 0, (size_t)ctx->S * sizeof(uint32_t), ctx->stream));
+        P.done = ctx->sg_done.as<uint32_t>();
+    }
     CU(timed_launch(ctx, 0, [&] {
+        for (int k = 0; grids && k < ctx->S;) {
+            int e = k;
+            while (e < ctx->S && e - k < batch && ctx->h_src_type[e] == 0) ++e;
+            if (e == k) {
+                ++k;
+                continue;
+            }
+            SunDirectParams D{};
+            D.sc = P.sc;
+            D.dimx = dimx;
+            D.dimy = dimy;
+            D.seed = seed;
+            D.pass = pass;
+            D.offset = offset;
+            D.count = count;
+            D.first = k;
+            D.nb = e - k;
+            D.S = ctx->S;
+            D.G = P.G;
+            fill_sun_params(ctx, &D);
+            const cudaError_t ee = launch_direct_sun(D, ctx->src.as<SourceDev>()[k].pos, (int)(sizeof(SourceDev) / 4),
+                                                     ctx->sg_extent.as<uint32_t>(), ctx->sg_done.as<uint32_t>() + k,
+                                                     false, per, max_blocks(ctx), ctx->stream);
+            if (ee != cudaSuccess) return ee;
+            chunks += 5;
+            k = e;
+        }
         DirectParams Q = P;
         for (uint32_t done = 0; done < count; done += Q.count, ++chunks) {
             Q.offset = offset + done;
@@ -507,6 +580,8 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
     E.Gd = ctx->Gd.as<double>();
     E.Gcov = cov ? ctx->Gcov.as<double>() : nullptr;
     E.src_flux = ctx->src_flux.as<float>();
+    E.strength = 1.0 / (double)(dimx * dimy);
+    E.done = P.done;
     CU(launch_epilogue_direct(E, ctx->stream));
     ctx->last_kernels += 1 + chunks;
     return HRT_OK;
@@ -1036,6 +1111,7 @@ int hrt_build_accel(hrt_context *ctx) {
     if (r) return r;
     // compressed 4-wide nodes for the persistent diffuse trace (scratch reuses the build's)
     ctx->n4 = 0;
+    ctx->sg_extent_ready = false;
     CU(ctx->nodes4.ensure(ctx->stream, bvh4_node_capacity(n) * 4 * sizeof(float4)));
     // the traces fetch a node in two 256-bit loads, which need 32-byte aligned addresses
     if (((uintptr_t)ctx->nodes.p | (uintptr_t)ctx->nodes4.p) & 63u)
@@ -1135,10 +1211,12 @@ int hrt_update_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sou
     if (nsources > 256) return fail(ctx, HRT_EINVAL, "A maximum of 256 radiation sources are allowed.");
     CU(cudaSetDevice(ctx->device));
     std::vector<SourceDev> h((size_t)std::max(nsources, 1));
+    ctx->h_src_type.assign((size_t)nsources, 0);
     for (int k = 0; k < nsources; ++k) {
         if (sources[k].type > 4) return fail(ctx, HRT_EINVAL, "unknown source type");
         SourceDev &s = h[k];
         s.type = (int)sources[k].type;
+        ctx->h_src_type[k] = s.type;
         for (int i = 0; i < 3; ++i) s.pos[i] = sources[k].position[i];
         s.w0 = sources[k].width[0];
         s.w1 = sources[k].width[1];
@@ -1730,7 +1808,8 @@ struct SweepPlan {
     size_t m = 0;
     bool scattering = false, any_direct = false, any_diffuse = false, any_copy0 = false, any_active = false;
     int dimx = 0, dimy = 0, ddx = 0, ddy = 0, Rd = 0, depth = 0;
-    uint32_t seed = 0, rec_per = 0;
+    uint32_t seed = 0, rec_per = 0, dir_per = 0;
+    int sun_batch = 0;  // suns binned together for the direct pass (0: through the tree)
     int rec_variant = DV_W4S4D16;
     float *d_sun = nullptr, *d_flux = nullptr, *d_sky = nullptr, *d_zero = nullptr;
     uint8_t *m_all = nullptr, *m_fold = nullptr, *m_diff = nullptr, *m_copy0 = nullptr, *m_active = nullptr;
@@ -1838,6 +1917,11 @@ int sweep_prepare(hrt_context *ctx, const hrt_sweep *s, bool tune, SweepPlan *pl
     P.hits = ctx->sw_hits.as<uint32_t>();
     CU(ctx->Gd.ensure(ctx->stream, std::max<size_t>((size_t)n * nsun * 2, 1) * sizeof(double)));
     CU(ctx->fetch.ensure(ctx->stream, sizeof(unsigned long long)));
+    P.dir_per = std::max(launch_chunk_prims(std::max<uint64_t>((uint64_t)P.dimx * (uint64_t)P.dimy, 1), ctx->ray_limit), 1u);
+    if (P.any_direct && P.dimx * P.dimy > 0 &&
+        sun_grids_pay(ctx, (unsigned long long)n * (unsigned)(P.dimx * P.dimy))) {
+        if ((r = ensure_sun_grids(ctx, nsun, &P.sun_batch))) return r;
+    }
     // choose the recording kernel's variant before capture (timing cannot run inside a capture)
     P.rec_variant = ctx->n4 > 0 ? DV_W4S4D16 : DV_PS3;
     if (tune && P.Rd > 0 && (P.any_diffuse || P.any_active)) {
@@ -1864,11 +1948,12 @@ int sweep_prepare(hrt_context *ctx, const hrt_sweep *s, bool tune, SweepPlan *pl
 std::string sweep_key(const SweepPlan &P, const hrt_sweep *s) {
     hrt_context *ctx = P.ctx;
     char key[384];
-    std::snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%d/%u/%d%d%d%d/%p/%p/%p/%p/%p/%p/%p/v%d/c%u", P.n, P.nsun, P.Bl,
+    std::snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%d/%u/%d%d%d%d/%p/%p/%p/%p/%p/%p/%p/v%d/c%u/%u/g%d/%p/%p/%p/%p", P.n, P.nsun, P.Bl,
                   s->direct_rays, s->diffuse_rays, s->scattering_depth, s->seed, (int)P.any_direct,
                   (int)P.any_diffuse, (int)P.any_copy0, (int)P.any_active, ctx->sw_acc.p, ctx->sw_hits.p,
                   ctx->sw_in.p, ctx->sw_mat.p, ctx->sw_out.p, ctx->Gd.p, (void *)ctx->stream, P.rec_variant,
-                  P.rec_per);
+                  P.rec_per, P.dir_per, P.sun_batch, ctx->sg_cells.p, ctx->sg_entries.p, ctx->sg_grids.p,
+                  ctx->sg_done.p);
     return key;
 }
 
@@ -1920,12 +2005,39 @@ struct SweepStages {
                 return e;
             TraceScene sc = scene_of(ctx);
             sc.visits = nullptr;
-            SweepDirectParams D{sc, P.d_sun, P.nsun, P.dimx, P.dimy, P.seed, ctx->Gd.as<double>()};
+            SweepDirectParams D{sc, P.d_sun, P.nsun, P.dimx, P.dimy, P.seed, ctx->Gd.as<double>(), nullptr};
+            if (P.sun_batch > 0) {
+                D.done = ctx->sg_done.as<uint32_t>();
+                if ((e = cudaMemsetAsync(ctx->sg_done.p, 0, (size_t)P.nsun * sizeof(uint32_t), st)) != cudaSuccess)
+                    return e;
+                for (int k = 0; k < P.nsun; k += P.sun_batch) {
+                    SunDirectParams Q{};
+                    Q.sc = sc;
+                    Q.dimx = P.dimx;
+                    Q.dimy = P.dimy;
+                    Q.seed = P.seed;
+                    Q.pass = 0u;
+                    Q.offset = 0u;
+                    Q.count = (uint32_t)P.n;
+                    Q.first = k;
+                    Q.nb = std::min(P.sun_batch, P.nsun - k);
+                    Q.S = P.nsun;
+                    Q.G = ctx->Gd.as<double>();
+                    fill_sun_params(ctx, &Q);
+                    if ((e = launch_direct_sun(Q, P.d_sun + 3 * k, 3, ctx->sg_extent.as<uint32_t>(),
+                                               ctx->sg_done.as<uint32_t>() + k, true, P.dir_per, max_blocks(ctx),
+                                               st)) != cudaSuccess)
+                        return e;
+                    nk += 5;
+                }
+            }
             if ((e = launch_direct_sweep(D, max_blocks(ctx), st)) != cudaSuccess) return e;
             ChannelEpilogue E = epilogue();
             E.flux = P.d_flux;
             E.mask = P.m_all;
             E.Gd = ctx->Gd.as<double>();
+            E.inv_nr = 1.0 / (double)(P.dimx * P.dimy);
+            E.done = D.done;
             if ((e = launch_epilogue_direct_channels(E, st)) != cudaSuccess) return e;
             nk += 2;
         }

@@ -106,7 +106,7 @@ struct Request {
 size_t footprint(int32_t n, int32_t Bl) {
     size_t nn = (size_t)std::max(n, 1);
     return nn * (64 + 64 + 64 + 64 + 64 + 8 + 1) + nn * (size_t)std::max(Bl, 1) * (7 * 8 + 3 * 4) + nn * 200 +
-           (8u << 20);
+           nn * 192 + (8u << 20);  // 192: the grid of one sun (hrt_sungrid.cu)
 }
 
 }  // namespace

@@ -116,6 +116,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_direct(const DirectParams P) {
     const uint32_t total = P.count * R;  // < 2^31: the host plans primitive chunks
     const uint32_t stride = gridDim.x * blockDim.x;
     const double inv_nr = 1.0 / (double)R;
+    if (P.done) {  // nothing to do when grids have traced every source
+        bool left = false;
+        for (int k = 0; k < P.S; ++k) left = left || !P.done[k];
+        if (!left) return;
+    }
     for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
         const uint32_t id = base + (threadIdx.x & 31);
         const bool active = id < total;
@@ -130,6 +135,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_direct(const DirectParams P) {
             type = __float_as_uint(g[0].w);
         }
         for (int k = 0; k < P.S; ++k) {
+            if (P.done && P.done[k]) continue;
             uint32_t nv = 0, np = 0;
             double v[2] = {0.0, 0.0};  // [face0, face1]
             bool live = active;
@@ -461,6 +467,7 @@ __global__ void k_epilogue_direct(const EpilogueParams P) {
     double in = 0.0, top = 0.0, bot = 0.0;
     for (int s = 0; s < P.S; ++s) {
         double flux = (double)P.src_flux[(size_t)s * P.Bl + b];
+        if (P.done && P.done[s]) flux *= P.strength;
         double g0 = P.Gd[((size_t)p * P.S + s) * 2] * flux, g1 = P.Gd[((size_t)p * P.S + s) * 2 + 1] * flux;
         if (P.Gcov) {
             g0 += P.Gcov[(((size_t)p * P.S + s) * 2) * P.Bl + b] * flux;
@@ -524,28 +531,23 @@ __global__ void k_final(size_t nb, const double *__restrict__ rin, const double 
 
 
 // ---------------------------------------------------------------- batched sweep --
-// Shadow rays of many suns in one launch.  Ray ids are sun-major, so a warp holds
-// 32 strata of one primitive toward ONE sun (coherent rays).  Origins and strengths
+// Shadow rays of many suns in one launch, sun after sun, so a warp holds 32 strata of one primitive
+// toward ONE sun (coherent rays); suns that a grid has served (P.done) are passed over.  Origins and strengths
 // are exactly those of a plain direct pass with the same seed (source slot 0).  W4: shadow rays
 // over the compressed 4-wide nodes (sc.nodes4 set), else the binary nodes.
 template <bool W4>
 __global__ void __launch_bounds__(kBlock, 3) k_direct_sweep(const SweepDirectParams P) {
     const uint32_t R = (uint32_t)(P.dimx * P.dimy);
-    const unsigned long long per_sun = (unsigned long long)P.sc.n * R;
-    const unsigned long long total = per_sun * (unsigned long long)P.nsun;
+    const unsigned long long total = (unsigned long long)P.sc.n * R;
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
     const double inv_nr = 1.0 / (double)R;
+    for (uint32_t sun = 0; sun < (uint32_t)P.nsun; ++sun) {
+    if (P.done && P.done[sun]) continue;
     for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
          base += stride) {
         const unsigned long long id = base + (threadIdx.x & 31);
         const bool active = id < total;
-        uint32_t sun = 0, p = 0, r = 0;
-        if (active) {
-            sun = (uint32_t)(id / per_sun);
-            const unsigned long long rem = id - (unsigned long long)sun * per_sun;
-            p = (uint32_t)(rem / R);
-            r = (uint32_t)(rem % R);
-        }
+        const uint32_t p = active ? (uint32_t)(id / R) : 0u, r = active ? (uint32_t)(id % R) : 0u;
         double v[2] = {0.0, 0.0};
         bool live = false;
         if (active) {
@@ -570,6 +572,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_direct_sweep(const SweepDirectPar
         count_rays(P.sc, live);
         const uint32_t key = active ? (p * (uint32_t)P.nsun + sun) : 0xFFFFFFFFu;
         warp_segment_add<2>(key, v, 2, P.G, 2);
+    }
     }
 }
 
@@ -658,7 +661,7 @@ __global__ void k_epilogue_direct_channels(const ChannelEpilogue P, int nsun) {
     if (i >= (long long)P.n * P.C) return;
     const int p = (int)(i / P.C), c = (int)(i % P.C), b = c % P.Bl, sun = c / P.Bl;
     if (!P.mask[c]) return;
-    const double flux = (double)P.flux[c];
+    const double flux = (P.done && P.done[sun]) ? (double)P.flux[c] * P.inv_nr : (double)P.flux[c];
     const double g0 = P.Gd[((size_t)p * nsun + sun) * 2] * flux, g1 = P.Gd[((size_t)p * nsun + sun) * 2 + 1] * flux;
     const double rho = P.rho[(size_t)p * P.Bl + b], tau = P.tau[(size_t)p * P.Bl + b];
     P.rin[i] += (g0 + g1) * (1.0 - rho - tau);
@@ -916,8 +919,8 @@ cudaError_t launch_residual(int n, int Bl, const double *area, const double *rin
 }
 
 cudaError_t launch_direct_sweep(const SweepDirectParams &p, int max_blocks, cudaStream_t s) {
-    const long long total = (long long)p.sc.n * p.dimx * p.dimy * p.nsun;
-    if (total <= 0) return cudaSuccess;
+    const long long total = (long long)p.sc.n * p.dimx * p.dimy;
+    if (total <= 0 || p.nsun <= 0) return cudaSuccess;
     unsigned nb = blocks_for(total, kBlock);
     if ((int)nb > max_blocks) nb = (unsigned)max_blocks;
     if (p.sc.nodes4) k_direct_sweep<true><<<nb, kBlock, 0, s>>>(p);

@@ -320,6 +320,19 @@ __device__ __forceinline__ bool wall_closest(const TraceScene &sc, f3 o, f3 d, f
     return any;
 }
 
+// The point hp on wall `which` moved to the opposite wall.
+__device__ __forceinline__ f3 wall_wrap(const TraceScene &sc, f3 hp, int which) {
+    if ((sc.periodic_x == 1.f) && which < 2) {
+        const float width = sc.bbox[4].x - sc.bbox[0].x;
+        hp.x = hp.x + ((which == 0) ? width : -width);
+    } else {
+        const int yb = (sc.periodic_x == 1.f) ? 2 : 0;
+        const float width = sc.bbox[4 * (yb + 1)].y - sc.bbox[4 * yb].y;
+        hp.y = hp.y + ((which == yb) ? width : -width);
+    }
+    return hp;
+}
+
 // Trace with periodic wrapping (<= 10 wraps; OptiX8DeviceCode.cu:763-789, 1440-1459).
 // o_last (optional): origin of the last segment traced.  W4: over the compressed 4-wide nodes
 // (the caller checks that sc.nodes4 is set).
@@ -338,17 +351,7 @@ __device__ Hit trace_full(const TraceScene &sc, f3 o, f3 d, float tmin, float tm
         int which = -1;
         float lim = (h.prim != 0xFFFFFFFFu) ? h.t : tmax;
         if (!wall_closest(sc, o, d, tmin, lim, &tb, &which) || (h.prim != 0xFFFFFFFFu && !(tb < h.t))) return h;
-        f3 hp = add(o, scl(d, tb));
-        bool xwall = (sc.periodic_x == 1.f) && which < 2;
-        if (xwall) {
-            float width = sc.bbox[4].x - sc.bbox[0].x;
-            hp.x = hp.x + ((which == 0) ? width : -width);
-        } else {
-            int yb = (sc.periodic_x == 1.f) ? 2 : 0;
-            float width = sc.bbox[4 * (yb + 1)].y - sc.bbox[4 * yb].y;
-            hp.y = hp.y + ((which == yb) ? width : -width);
-        }
-        o = hp;
+        o = wall_wrap(sc, add(o, scl(d, tb)), which);
     }
     // The tenth trace ended on a wall again: the reference's loop stops there and no
     // miss or closest-hit program deposits anything for this ray.
@@ -384,17 +387,7 @@ __device__ Hit trace_covers(const TraceScene &sc, f3 o, f3 d, float tmin, float 
             }
         }
         if (!wall) return h;
-        f3 hp = add(o, scl(d, tb));
-        bool xwall = (sc.periodic_x == 1.f) && which < 2;
-        if (xwall) {
-            float width = sc.bbox[4].x - sc.bbox[0].x;
-            hp.x = hp.x + ((which == 0) ? width : -width);
-        } else {
-            int yb = (sc.periodic_x == 1.f) ? 2 : 0;
-            float width = sc.bbox[4 * (yb + 1)].y - sc.bbox[4 * yb].y;
-            hp.y = hp.y + ((which == yb) ? width : -width);
-        }
-        o = hp;
+        o = wall_wrap(sc, add(o, scl(d, tb)), which);
     }
     return Hit{tmax, kLost, 0};
 }
@@ -841,16 +834,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_diffuse_ps(const DiffuseParams
                 if (wraps >= 9) {
                     lost = true;
                 } else {
-                    f3 hp = add(o, scl(d, tb));
-                    if ((sc.periodic_x == 1.f) && which < 2) {
-                        float width = sc.bbox[4].x - sc.bbox[0].x;
-                        hp.x = hp.x + ((which == 0) ? width : -width);
-                    } else {
-                        int yb = (sc.periodic_x == 1.f) ? 2 : 0;
-                        float width = sc.bbox[4 * (yb + 1)].y - sc.bbox[4 * yb].y;
-                        hp.y = hp.y + ((which == yb) ? width : -width);
-                    }
-                    o = hp;
+                    o = wall_wrap(sc, add(o, scl(d, tb)), which);
                     ooi = mk(o.x * inv.x, o.y * inv.y, o.z * inv.z);
                     best = 1e38f;
                     bprim = 0xFFFFFFFFu;

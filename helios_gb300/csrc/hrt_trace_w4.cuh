@@ -414,15 +414,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                 if (wraps >= 9) {
                     lost = true;
                 } else {
-                    f3 hp = add(o, scl(d, tb));
-                    if ((sc.periodic_x == 1.f) && which < 2) {
-                        const float width = sc.bbox[4].x - sc.bbox[0].x;
-                        hp.x = hp.x + ((which == 0) ? width : -width);
-                    } else {
-                        const int yb = (sc.periodic_x == 1.f) ? 2 : 0;
-                        const float width = sc.bbox[4 * (yb + 1)].y - sc.bbox[4 * yb].y;
-                        hp.y = hp.y + ((which == yb) ? width : -width);
-                    }
+                    const f3 hp = wall_wrap(sc, add(o, scl(d, tb)), which);
                     s_ray[6][tid] = hp.x;
                     s_ray[7][tid] = hp.y;
                     s_ray[8][tid] = hp.z;

@@ -70,3 +70,86 @@ def test_wide_nodes_enclose_their_children(gpu, oracle_mod, scale, offset):
     floor = 1e-3 * float(np.abs(ref).mean())
     assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
     assert rad.last_stats["rays"] == st["rays"]
+
+
+def _direct_model(kind, suns, periodic, rays=400, seed=3):
+    """A direct-only solve of at least 0.2 M rays per source, so that collimated sources are binned."""
+    from helios_gb300.radiation import Context, RadiationModel
+
+    ctx = Context()
+    if kind == "voxels":
+        ctx.addScene(scenes.deep_scatter(n_tri=300, n_patch=150, n_disk=150, vox_div=4, domain=2.0, height=1.0, seed=seed))
+    elif kind == "far":  # coordinates far larger than the scene
+        sc = scenes.mixed_canopy(700, 2.0, seed=seed)
+        T = sc.T.copy()
+        T[:, [3, 7]] += 2.0e4
+        ctx.addPrimitives(T, sc.ptype, sc.area, sc.twosided)
+    elif kind == "wide":  # more wide primitives than a grid takes: the tree serves the source
+        ctx.addScene(scenes.mixed_canopy(2000, 2.0, seed=seed))
+        for k in range(40):
+            ctx.addPatch((0.6, 0.7, 3.1 + 0.01 * k), (1.5, 1.4), (0.1, 0.2 * k))
+    elif kind == "flat":  # one plane: no extent across a horizontal sun
+        ctx.addScene(scenes.tile_grid((0.0, 0.0, 0.0), (4.0, 4.0), (24, 24), twosided=1))
+    else:
+        ctx.addScene(scenes.mixed_canopy(700, 2.0, seed=seed))
+        if kind == "masks":
+            mask = np.zeros((8, 8), np.uint8)
+            mask[::2] = 1
+            for k in range(30):
+                ctx.addPatch((0.03 * k, 0.5, 3.2), (0.2, 0.2), (0.3, 0.1 * k), texture_mask=mask)
+    rad = RadiationModel(ctx)
+    if periodic:
+        rad.enforcePeriodicBoundary("xy")
+    rad.addRadiationBand("SW")
+    rad.disableEmission("SW")
+    for k, d in enumerate(suns):
+        s = rad.addSphereRadiationSource((0.5, 0.5, 9.0), 0.3) if d is None else rad.addCollimatedRadiationSource(d)
+        rad.setSourceFlux(s, "SW", 300.0 + 50.0 * k)
+    rad.setDirectRayCount("SW", rays)
+    rad.setDiffuseRayCount("SW", 1)
+    rad.setSeed(seed)
+    return rad
+
+
+SUNS = [(0.3, -0.4, 0.8), (0.0, 0.0, 1.0), (1.0, 0.0, 0.0), (-0.2, 0.9, -0.3)]
+
+
+@pytest.mark.parametrize("kind", ["mixed", "voxels", "masks", "far", "wide", "flat"])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_binned_shadow_rays_equal_the_tree(hrt_lib, kind, periodic):
+    """Shadow rays answered by the grid across the sun give the tree's sums: suns from above, along an
+    axis and from below, a source that is no sun between them, over every primitive form.  A set
+    visit budget sends all of them through the tree.  Strengths are summed in another order in FP64:
+    FP32 fluxes agree to two units in the last place."""
+    rad = _direct_model(kind, SUNS[:2] + [None] + SUNS[2:], periodic)
+    binned = rad.runBand("SW").astype(np.float64)
+    rays = rad.last_stats["rays"]
+    rad.ctx.set_visit_budget(1 << 30)
+    tree = rad.runBand("SW").astype(np.float64)
+    assert (tree > 0).any()
+    assert np.abs(binned - tree).max() <= 2.4e-7 * np.abs(tree).max()
+    assert np.all(np.abs(binned - tree) <= 2.4e-7 * np.abs(tree))
+    assert rad.last_stats["rays"] == rays
+    rad.ctx.set_visit_budget(0)
+    rad.ctx.set_launch_ray_limit(60000)  # several primitive chunks
+    assert np.all(np.abs(rad.runBand("SW").astype(np.float64) - tree) <= 2.4e-7 * np.abs(tree))
+
+
+@pytest.mark.parametrize("nsun", [1, 33])
+def test_binned_sweep_equals_the_tree(gpu, nsun):
+    """The sweep's suns in one batch and in two (more suns than a batch holds)."""
+    sc = scenes.mixed_canopy(2100, 2.0, seed=4)
+    rng = np.random.default_rng(1)
+    d = scenes.uniform_sphere(rng, nsun).astype(np.float32)
+    kw = dict(sun_dir=d, direct_flux=np.full((nsun, 1), 500.0), diffuse_flux=np.zeros((nsun, 1)),
+              rho=np.full((sc.n, 1), 0.1), tau=np.full((sc.n, 1), 0.05), direct_rays=100, diffuse_rays=4, depth=0, seed=9)
+    gpu.update_geometry(sc.T, sc.ptype, sc.twosided)
+    gpu.build_accel()
+    binned, rays = gpu.run_sweep(**kw), gpu.last_stats()["rays"]
+    again = gpu.run_sweep(**kw)
+    gpu.set_visit_budget(1 << 30)
+    tree = gpu.run_sweep(**kw)
+    gpu.set_visit_budget(0)
+    assert gpu.last_stats()["rays"] == rays
+    assert np.array_equal(binned, again)
+    assert np.all(np.abs(binned - tree) <= 2.4e-7 * np.abs(tree))
