@@ -1701,6 +1701,7 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
         {
             // zero diffuse flux for the scattering iterations (RadiationModel.cpp:4237-4240)
             CU(cudaMemsetAsync((void *)sky.flux, 0, (size_t)Bl * sizeof(float), st));
+            ctx->sky_any = false;
             sky0 = sky;
         }
         std::vector<uint8_t> sflags = flags, conv(Bg, 0);

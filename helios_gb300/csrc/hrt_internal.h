@@ -282,6 +282,7 @@ enum DiffuseVariant {
 bool is_w4s_variant(int v);
 cudaError_t launch_w4s(const DiffuseParams &p, int variant, cudaStream_t s);
 cudaError_t launch_w4s_record(const DiffuseParams &p, uint32_t *hits, int variant, cudaStream_t s);
+cudaError_t launch_w4s_covers(const DiffuseParams &p, cudaStream_t s);
 cudaError_t launch_w4s_stats(const DiffuseParams &p, int variant, cudaStream_t s);
 // Multi-scene recording launch: p.fetch, p.faces, p.slots / nslots / multi_total set; the
 // other scene fields of p are unused.

@@ -21,7 +21,8 @@ unsigned w4_grid(const DiffuseParams &p, int resident, int block) {
     return (unsigned)g;
 }
 
-template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB = 1, bool MULTI = false, bool LIN = false>
+template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB = 1, bool MULTI = false, bool LIN = false,
+          bool COV = false>
 cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
     // resident blocks of one wave (SMs x blocks per SM); initialised once per instantiation,
     // thread-safe (the server launches from several threads)
@@ -30,7 +31,7 @@ cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
-                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN>,
+                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV>,
                                                       BLOCK, 0);
         return (sms < 1 ? 1 : sms) * (per_sm < 1 ? 1 : per_sm);
     }();
@@ -38,7 +39,7 @@ cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     DiffuseParams q = p;
     q.refill = refill_threshold(false, true);
-    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
+    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -87,6 +88,14 @@ cudaError_t launch_w4s_multi_record(const DiffuseParams &p, cudaStream_t s) {
     DiffuseParams q = p;
     q.Bc = 1;
     return w4_launch<1, true, false, 4, 8, 256, 1, true>(q, s);
+}
+
+cudaError_t launch_w4s_covers(const DiffuseParams &p, cudaStream_t s) {
+    if (!p.sc.nodes4 || p.sc.voxels || !p.sc.cover) return cudaErrorInvalidValue;
+    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true, true>(p, s);
+    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true, true>(p, s);
+    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true, true>(p, s);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_w4s_stats(const DiffuseParams &p, int variant, cudaStream_t s) {

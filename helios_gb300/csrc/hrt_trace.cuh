@@ -298,6 +298,97 @@ __device__ Hit trace_bvh4(const TraceScene &sc, f3 o, f3 d, float tmin, float tm
     return h;
 }
 
+// The covers a ray segment crosses, nearest first (ties: the smaller primitive index), at most
+// kMaxCovers of them.
+struct CoverList {
+    int n;
+    float t[kMaxCovers];
+    uint32_t code[kMaxCovers];  // primitive << 1 | face
+    __device__ void add(float tc, uint32_t c) {
+        if (n == kMaxCovers) {
+            if (!(tc < t[n - 1] || (tc == t[n - 1] && c < code[n - 1]))) return;
+            --n;
+        }
+        int i = n++;
+        for (; i > 0 && (tc < t[i - 1] || (tc == t[i - 1] && c < code[i - 1])); --i) {
+            t[i] = t[i - 1];
+            code[i] = code[i - 1];
+        }
+        t[i] = tc;
+        code[i] = c;
+    }
+};
+
+// Closest opaque hit over the compressed 4-wide nodes of a launch with covers: covers of source bit
+// cbit are passed and, with list, the nearest of those met before the closest hit known at the time
+// are kept (never the ray's own origin `self`).  One walk finds the hit and the covers; the binary
+// form (trace_bvh with a CoverQ) walks the tree once for the hit and once more per cover.
+__device__ Hit trace_bvh4_covers(const TraceScene &sc, f3 o, f3 d, float tmin, float tmax, const VoxKey &vk,
+                                 uint32_t cbit, uint32_t self, CoverList *list) {
+    Hit h{tmax, 0xFFFFFFFFu, 0};
+    if (sc.n == 0) return h;
+    const WT w = wt_setup(d);
+    const f3 inv = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+    int32_t stack[kStack4];
+    int sp = 0;
+    int32_t cur = 0;
+    float best = tmax;
+    const uint32_t n4 = (uint32_t)sc.n4;
+    uint32_t budget = sc.visit_budget;
+    for (;;) {
+        if ((uint32_t)cur >= n4 || budget-- == 0u) {
+            raise(sc.status, budget == 0xFFFFFFFFu ? ERR_BUDGET : ERR_BOUNDS);
+            return h;
+        }
+        float4 q0, q1, q2, q3;
+        load_node64(sc.nodes4, cur, q0, q1, q2, q3);
+        float tk[4];
+        int32_t ck[4];
+        node4_children(q0, q1, q2, q3, node4_offset(q0, o, inv), inv, tmin, best, tk, ck);
+        node4_nearest(tk, ck);
+        int32_t nxt = kSentinel;
+#pragma unroll
+        for (int k = 3; k >= 0; --k) {
+            const int32_t c = ck[k];
+            if (c == kSentinel) continue;
+            if (c >= 0) {
+                if (nxt != kSentinel) {
+                    if (sp >= kStack4) {
+                        raise(sc.status, ERR_STACK);
+                        return h;
+                    }
+                    stack[sp++] = nxt;
+                }
+                nxt = c;
+                continue;
+            }
+            if ((uint32_t)(~c) >= (uint32_t)sc.n) {
+                raise(sc.status, ERR_BOUNDS);
+                continue;
+            }
+            float t;
+            int face;
+            uint32_t orig;
+            if (rec_hit(sc.rec, (uint32_t)(~c), w, o, d, inv, tmin, best, vk, &t, &face, &orig, sc.masks)) {
+                if (__ldg(sc.cover + orig) & cbit) {
+                    if (list && orig != self) list->add(t, (orig << 1) | (uint32_t)face);
+                } else if (h.prim == 0xFFFFFFFFu || t < h.t || (t == h.t && orig < h.prim)) {
+                    h.t = t;
+                    h.prim = orig;
+                    h.face = face;
+                    best = t;
+                }
+            }
+        }
+        if (nxt == kSentinel) {
+            if (sp == 0) break;
+            nxt = stack[--sp];
+        }
+        cur = nxt;
+    }
+    return h;
+}
+
 // Periodic walls: closest wall before `lim`.
 __device__ __forceinline__ bool wall_closest(const TraceScene &sc, f3 o, f3 d, float tmin, float lim, float *tb,
                                              int *which) {
@@ -362,28 +453,37 @@ __device__ Hit trace_full(const TraceScene &sc, f3 o, f3 d, float tmin, float tm
 // deterministic): the closest opaque hit with every cover of source bit `cbit` passed, then,
 // when `collect`, the covers of each periodic segment before its end in the order
 // (distance, primitive index), each reported to on_cover(prim, face).
-template <class F>
+// W4: over the compressed 4-wide nodes (sc.nodes4 set).
+template <bool W4, class F>
 __device__ Hit trace_covers(const TraceScene &sc, f3 o, f3 d, float tmin, float tmax, VoxKey vk, uint32_t cbit,
                             uint32_t self, bool collect, F &&on_cover) {
     const uint32_t c2 = vk.c2;
     const CoverQ q0{cbit, 0, -1.f, 0u, self};
     for (int wrap = 0; wrap < 10; ++wrap) {
         vk.c2 = c2 | ((uint32_t)wrap << 16);
-        Hit h = trace_bvh<false, true>(sc, o, d, tmin, tmax, false, vk, nullptr, nullptr, &q0);
+        CoverList list;
+        if (W4) list.n = 0;
+        Hit h = W4 ? trace_bvh4_covers(sc, o, d, tmin, tmax, vk, cbit, self, collect ? &list : nullptr)
+                   : trace_bvh<false, true>(sc, o, d, tmin, tmax, false, vk, nullptr, nullptr, &q0);
         const float lim = (h.prim != 0xFFFFFFFFu) ? h.t : tmax;
         float tb = lim;
         int which = -1;
         const bool wall = sc.nbbox > 0 && wall_closest(sc, o, d, tmin, lim, &tb, &which) &&
                           (h.prim == 0xFFFFFFFFu || tb < h.t);
         if (collect) {
-            CoverQ q1{cbit, 1, -1.f, 0u, self};
             const float end = wall ? tb : lim;
-            for (int c = 0; c < kMaxCovers; ++c) {
-                const Hit g = trace_bvh<false, true>(sc, o, d, tmin, end, false, vk, nullptr, nullptr, &q1);
-                if (g.prim == 0xFFFFFFFFu) break;
-                on_cover(g.prim, g.face);
-                q1.tlo = g.t;
-                q1.ilo = g.prim;
+            if (W4) {
+                for (int c = 0; c < list.n && list.t[c] <= end; ++c)
+                    on_cover(list.code[c] >> 1, (int)(list.code[c] & 1u));
+            } else {
+                CoverQ q1{cbit, 1, -1.f, 0u, self};
+                for (int c = 0; c < kMaxCovers; ++c) {
+                    const Hit g = trace_bvh<false, true>(sc, o, d, tmin, end, false, vk, nullptr, nullptr, &q1);
+                    if (g.prim == 0xFFFFFFFFu) break;
+                    on_cover(g.prim, g.face);
+                    q1.tlo = g.t;
+                    q1.ilo = g.prim;
+                }
             }
         }
         if (!wall) return h;

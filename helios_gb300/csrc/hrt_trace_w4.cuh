@@ -77,8 +77,10 @@ struct LinStack {
 // MULTI (recording mode only): the launch traces several scenes -- P.slots[0..P.nslots) each
 // give a scene, a primitive chunk, ray counts, seed, pass and hit buffer, with consecutive
 // ranges of the launch's ray ids (id_begin) -- so one persistent launch covers the pass of
-// every scene of a multi-scene sweep.  LIN: the LinStack layout, else RingStack.
-template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB, bool MULTI = false, bool LIN = false>
+// every scene of a multi-scene sweep.  LIN: the LinStack layout, else RingStack.  COV: translucent
+// covers of source 0 (P.sc.cover) are passed as if they were not there.
+template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB, bool MULTI = false, bool LIN = false,
+          bool COV = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams P) {
     static_assert(!MULTI || (RECORD && !STATS), "multi-scene launches record hits only");
     __shared__ double s_sum[RECORD ? 1 : NB][BLOCK];            // running sums of the lane's origin
@@ -379,7 +381,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                     float t;
                     int fc;
                     uint32_t orig;
-                    if (rec_hit<false>(sc.rec, slot, w, o, d, inv, 1e-4f, best, vk, &t, &fc, &orig, sc.masks)) {
+                    if (rec_hit<false>(sc.rec, slot, w, o, d, inv, 1e-4f, best, vk, &t, &fc, &orig, sc.masks) &&
+                        !(COV && (__ldg(sc.cover + orig) & 1u))) {
                         if (bcode == kMissCode || t < best || (t == best && orig < (bcode >> 1))) {
                             best = t;
                             bcode = (orig << 1) | (uint32_t)fc;

@@ -153,3 +153,40 @@ def test_binned_sweep_equals_the_tree(gpu, nsun):
     assert gpu.last_stats()["rays"] == rays
     assert np.array_equal(binned, again)
     assert np.all(np.abs(binned - tree) <= 2.4e-7 * np.abs(tree))
+
+
+@pytest.mark.parametrize("panes,voxels", [(1, False), (16, False), (20, False), (3, True)])
+@pytest.mark.parametrize("depth", [0, 2])
+def test_stacked_covers_vs_oracle(oracle_mod, panes, voxels, depth):
+    """Rays through a stack of covers, up to and beyond the sixteen that a segment takes, with a sky
+    (covers take deposits) and scattering (covers are passed by): fluxes of covers and leaves."""
+    from helios_gb300.radiation import Context, RadiationModel
+    from helpers import run_oracle
+
+    ctx = Context()
+    if voxels:
+        ctx.addScene(scenes.deep_scatter(n_tri=100, n_patch=60, n_disk=60, vox_div=3, domain=1.0, height=1.0, seed=6))
+    else:
+        ctx.addScene(scenes.mixed_canopy(200, 2.0, seed=6, height=1.0))
+    leaves = np.arange(1, ctx.getPrimitiveCount())
+    for k in range(panes):
+        u = ctx.addPatch((0.5, 0.5, 1.3 + 0.02 * k), (1.2, 1.2), (0.02 * (k % 3), 0.3 * k))
+        ctx.setPrimitiveData(u, "glass_n_SW", 1.3 + 0.01 * k)
+        ctx.setPrimitiveData(u, "glass_KL_SW", 0.02)
+    ctx.setPrimitiveData(leaves, "reflectivity_SW", np.full(leaves.size, 0.3))
+    ctx.setPrimitiveData(leaves, "transmissivity_SW", np.full(leaves.size, 0.2))
+    rad = RadiationModel(ctx)
+    rad.addRadiationBand("SW")
+    rad.disableEmission("SW")
+    s = rad.addCollimatedRadiationSource(scenes.sun_direction(25.0, 60.0))
+    rad.setSourceFlux(s, "SW", 600.0)
+    rad.setDiffuseRadiationFlux("SW", 100.0)
+    rad.setDirectRayCount("SW", 49)
+    rad.setDiffuseRayCount("SW", 64)
+    rad.setScatteringDepth("SW", depth)
+    rad.setSeed(21)
+    got = rad.runBand("SW").astype(np.float64)
+    ref, st = run_oracle(rad, ["SW"], oracle_mod, seed=21)
+    floor = 1e-3 * float(np.abs(ref).mean())
+    assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
+    assert rad.last_stats["rays"] == st["rays"]
