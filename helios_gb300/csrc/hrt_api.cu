@@ -107,6 +107,7 @@ struct hrt_context {
     // geometry
     int n = 0, nbbox = 0;
     float px = 0.f, py = 0.f;
+    float wall_scale = 0.f;  // TraceScene::wall_scale
     bool have_geometry = false, built = false;
     std::vector<int8_t> h_twosided;
     std::vector<uint32_t> h_voxels;  // original indices of voxel primitives
@@ -213,6 +214,7 @@ TraceScene scene_of(hrt_context *ctx) {
     sc.bbox = ctx->nbbox ? ctx->bbox.as<float4>() : nullptr;
     sc.n = ctx->n;
     sc.nbbox = ctx->nbbox;
+    sc.wall_scale = ctx->wall_scale;
     sc.voxels = ctx->h_voxels.empty() ? 0 : 1;
     sc.periodic_x = ctx->px;
     sc.periodic_y = ctx->py;
@@ -1067,6 +1069,22 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     ctx->nbbox = g->nbbox;
     ctx->px = g->periodic_x;
     ctx->py = g->periodic_y;
+    // Walls on the planes of an axis-aligned box, as RadiationModel lays them out (x walls, then y
+    // walls), pass the traces' plane test; other quads are always tested as they are.
+    ctx->wall_scale = 0.f;
+    if (g->nbbox) {
+        bool planes = g->nbbox == 4 ? (g->periodic_x == 1.f) : true;
+        float scale = 0.f;
+        const int nx = g->periodic_x == 1.f ? 2 : 0;
+        for (int b = 0; b < g->nbbox; ++b)
+            for (int k = 0; k < 4; ++k) {
+                const float *v = g->bbox_vertices + 3 * (4 * b + k), *v0 = g->bbox_vertices + 12 * b;
+                const int a = b < nx ? 0 : 1;
+                planes = planes && v[a] == v0[a];
+                for (int i = 0; i < 3; ++i) scale = std::max(scale, std::fabs(v[i]));
+            }
+        if (planes && std::isfinite(scale)) ctx->wall_scale = 2.f * scale;
+    }
     if (g->nbbox) {
         std::vector<float4> q((size_t)g->nbbox * 4);
         for (int i = 0; i < g->nbbox * 4; ++i)

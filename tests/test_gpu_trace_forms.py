@@ -190,3 +190,33 @@ def test_stacked_covers_vs_oracle(oracle_mod, panes, voxels, depth):
     floor = 1e-3 * float(np.abs(ref).mean())
     assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
     assert rad.last_stats["rays"] == st["rays"]
+
+
+@pytest.mark.parametrize("boundary", ["x", "y", "xy", "tilted"])
+def test_periodic_walls_vs_oracle(oracle_mod, boundary):
+    """Walls across x, across y and both, and walls that are not the planes of a box (which take no part
+    in the plane test): fluxes and ray counts against the oracle."""
+    from helios_gb300.radiation import Context, RadiationModel
+    from helpers import run_oracle
+
+    ctx = Context()
+    ctx.addScene(scenes.mixed_canopy(400, 1.0, seed=8))
+    rad = RadiationModel(ctx)
+    rad.enforcePeriodicBoundary("xy" if boundary == "tilted" else boundary)
+    if boundary == "tilted":
+        faces = rad._bbox_faces()
+        faces[1, 2, 0] += np.float32(0.01)
+        rad._bbox_faces = lambda: faces
+    rad.addRadiationBand("SW")
+    rad.disableEmission("SW")
+    s = rad.addCollimatedRadiationSource(scenes.sun_direction(55.0, 30.0))
+    rad.setSourceFlux(s, "SW", 600.0)
+    rad.setDiffuseRadiationFlux("SW", 100.0)
+    rad.setDirectRayCount("SW", 25)
+    rad.setDiffuseRayCount("SW", 64)
+    rad.setSeed(5)
+    got = rad.runBand("SW").astype(np.float64)
+    ref, st = run_oracle(rad, ["SW"], oracle_mod, seed=5)
+    floor = 1e-3 * float(np.abs(ref).mean())
+    assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
+    assert rad.last_stats["rays"] == st["rays"]
