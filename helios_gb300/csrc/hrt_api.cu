@@ -97,6 +97,78 @@ double prim_area(const float *T, uint32_t type, float lad) {
     return a;
 }
 
+// Do the voxels form a regular lattice?  Boxes as the records hold them (make_records, FP32): equal
+// sides, corners on the planes of one lattice within a thousandth of a cell, no cell twice, and not
+// so sparse that the table of cells outgrows them 16 times.  Fills g but for its device pointer and
+// the cells [x fastest] as the march reads them.
+bool find_lattice(const float *T, const std::vector<uint32_t> &vox, const float *lad, float far, VoxGrid *g,
+                  std::vector<float4> *cells) {
+    if (vox.empty()) return false;
+    const size_t nv = vox.size();
+    std::vector<float> lo(3 * nv), hi(3 * nv);
+    double size[3] = {0, 0, 0}, org[3], end[3];
+    for (int a = 0; a < 3; ++a) {
+        org[a] = INFINITY;
+        end[a] = -INFINITY;
+    }
+    for (size_t i = 0; i < nv; ++i) {
+        const float *t = T + 16 * (size_t)vox[i];
+        for (int a = 0; a < 3; ++a) {
+            const float c = t[4 * a + 3], h = std::fabs(t[5 * a]) * 0.5f;
+            lo[3 * i + a] = c - h;
+            hi[3 * i + a] = c + h;
+            if (!(h > 0.f) || !std::isfinite(c) || !std::isfinite(h)) return false;
+            org[a] = std::min(org[a], (double)lo[3 * i + a]);
+            end[a] = std::max(end[a], (double)hi[3 * i + a]);
+            size[a] += 2.0 * (double)h;
+        }
+    }
+    double cellsn = 1.0, ext = 0.0;
+    for (int a = 0; a < 3; ++a) {
+        size[a] /= (double)nv;
+        const double n = std::round((end[a] - org[a]) / size[a]);
+        if (!(n >= 1.0 && n <= 1024.0)) return false;  // cell indices of 10 bits
+        g->n[a] = (int)n;
+        size[a] = (end[a] - org[a]) / n;
+        cellsn *= n;
+        ext = std::max(ext, end[a] - org[a]);
+    }
+    if (cellsn > 16.0 * (double)nv + 64.0) return false;
+    double off = 0.0;
+    cells->assign(2 * (size_t)cellsn, make_float4(0.f, 0.f, 0.f, 0.f));
+    for (size_t i = 0; i < nv; ++i) {
+        size_t at = 0;
+        for (int a = 2; a >= 0; --a) {
+            const double q = std::round(((double)lo[3 * i + a] - org[a]) / size[a]);
+            if (!(q >= 0.0 && q < (double)g->n[a])) return false;
+            const double e0 = std::fabs((double)lo[3 * i + a] - (org[a] + q * size[a]));
+            const double e1 = std::fabs((double)hi[3 * i + a] - (org[a] + (q + 1.0) * size[a]));
+            if (e0 > 1e-3 * size[a] || e1 > 1e-3 * size[a]) return false;
+            off = std::max(off, std::max(e0, e1));
+            at = at * (size_t)g->n[a] + (size_t)q;
+        }
+        float4 &c0 = (*cells)[2 * at], &c1 = (*cells)[2 * at + 1];
+        if (c1.x != 0.f || c1.y != 0.f || c1.z != 0.f || c1.w != 0.f || c0.w != 0.f) return false;
+        uint32_t id = vox[i];
+        float idf;
+        std::memcpy(&idf, &id, sizeof idf);
+        c0 = make_float4(lo[3 * i], lo[3 * i + 1], lo[3 * i + 2], kVoxelG * lad[vox[i]]);
+        c1 = make_float4(hi[3 * i], hi[3 * i + 1], hi[3 * i + 2], idf);
+        if (c1.x == 0.f && c1.y == 0.f && c1.z == 0.f && id == 0u) return false;  // reads as an unused cell
+    }
+    // the march's crossings and the tests' round by about 2^-22 of the coordinates
+    const double tol = off * 2.0 + ((double)far + ext) * 3.814697265625e-06;
+    for (int a = 0; a < 3; ++a) {
+        g->org[a] = (float)org[a];
+        g->size[a] = (float)size[a];
+        g->inv[a] = (float)(1.0 / size[a]);
+        g->tolf[a] = (float)(tol / size[a]);
+        if (!(g->tolf[a] < 0.1f)) return false;
+    }
+    g->tol = (float)tol;
+    return true;
+}
+
 }  // namespace
 
 struct hrt_context {
@@ -115,6 +187,10 @@ struct hrt_context {
     DevBuf mask_id, mask_uv_id, mask_uv, mask_size, mask_offset, mask_data;
     bool masks = false;
     int n4 = 0;  // compressed 4-wide nodes built
+    // a lattice of voxels: its description, cells and the 4-wide nodes over the other primitives
+    bool have_lattice = false, use_lattice = false;
+    DevBuf vg, vg_cells, nodes4s;
+    int n4s = 0;
     // materials and sources
     int mS = 0, mN = 0, mB = 0;
     DevBuf rho, tau, src, src_flux;
@@ -210,6 +286,9 @@ TraceScene scene_of(hrt_context *ctx) {
     sc.nodes = ctx->nodes.as<float4>();
     sc.nodes4 = ctx->n4 > 0 ? ctx->nodes4.as<float4>() : nullptr;
     sc.n4 = ctx->n4;
+    sc.nodes4s = ctx->use_lattice ? ctx->nodes4s.as<float4>() : nullptr;
+    sc.n4s = ctx->use_lattice ? ctx->n4s : 0;
+    sc.vgrid = ctx->use_lattice ? ctx->vg.as<VoxGrid>() : nullptr;
     sc.rgen = ctx->rgen.as<float4>();
     sc.bbox = ctx->nbbox ? ctx->bbox.as<float4>() : nullptr;
     sc.n = ctx->n;
@@ -630,6 +709,7 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
         return HRT_OK;
     }
     if (!ctx->tune || rays < kTuneMinRays) return HRT_OK;
+    if (!record && P0.sc.vgrid) return HRT_OK;  // a marched lattice has one kernel
     char key[160];
     std::snprintf(key, sizeof key, "%s n=%d count=%u rays_per_face=%d faces=%d bands=%d voxels=%d",
                   record ? "record" : "accumulate", ctx->n, P0.count, P0.dimx * P0.dimy, P0.faces, P0.Bc,
@@ -1029,6 +1109,24 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
         CU(ctx->lad.ensure(ctx->stream, n * sizeof(float)));
         CU(cudaMemcpyAsync(ctx->lad.p, g->voxel_lad, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
+    ctx->have_lattice = ctx->use_lattice = false;
+    if (!voxels.empty() && voxels.size() + 2 <= n) {
+        float far = 0.f;  // periodic wraps stay within the walls, which hold the scene
+        for (size_t i = 0; i < n; ++i)
+            for (int a = 0; a < 3; ++a) far = std::max(far, std::fabs(g->transform[16 * i + 4 * a + 3]));
+        std::vector<float4> cells;
+        VoxGrid vg{};
+        if (find_lattice(g->transform, voxels, g->voxel_lad, far, &vg, &cells)) {
+            CU(ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4)));
+            CU(ctx->vg.ensure(ctx->stream, sizeof(VoxGrid)));
+            vg.cells = ctx->vg_cells.as<float4>();
+            CU(cudaMemcpyAsync(ctx->vg_cells.p, cells.data(), cells.size() * sizeof(float4), cudaMemcpyHostToDevice,
+                               ctx->stream));
+            CU(cudaMemcpyAsync(ctx->vg.p, &vg, sizeof vg, cudaMemcpyHostToDevice, ctx->stream));
+            CU(cudaStreamSynchronize(ctx->stream));  // the host copies end here
+            ctx->have_lattice = true;
+        }
+    }
     ctx->h_voxels.swap(voxels);
     // texture masks
     ctx->masks = false;
@@ -1148,6 +1246,18 @@ int hrt_build_accel(hrt_context *ctx) {
     }
     CU(bvh4_build(src2, n, ctx->nodes4.as<float4>(), ctx->bvh_scratch.p, ctx->status.as<uint32_t>(), &n4,
                   ctx->stream));
+    // a lattice of voxels is marched: a second tree holds the surfaces alone, which are the first
+    // leaves (voxel codes sort last)
+    const int ns = n - (int)ctx->h_voxels.size();
+    ctx->use_lattice = false;
+    if (ctx->have_lattice && ns >= 2) {
+        CU(ctx->nodes4s.ensure(ctx->stream, bvh4_node_capacity(ns) * 4 * sizeof(float4)));
+        if ((uintptr_t)ctx->nodes4s.p & 63u) return fail(ctx, HRT_ECUDA, "node arrays are not 64-byte aligned");
+        CU(ploc_build(b.leafbox, ns, ploc_nodes.as<float4>(), ploc_scratch.p, ctx->stream));
+        CU(bvh4_build(ploc_nodes.as<float4>(), ns, ctx->nodes4s.as<float4>(), ctx->bvh_scratch.p,
+                      ctx->status.as<uint32_t>(), &ctx->n4s, ctx->stream));
+        ctx->use_lattice = ctx->n4s > 0;
+    }
     ploc_nodes.free_on(ctx->stream);
     ploc_scratch.free_on(ctx->stream);
     if ((r = sync_and_status(ctx))) return r;

@@ -8,12 +8,23 @@
 
 namespace hrt {
 
+// Voxels that are cells of one lattice (hrt_voxgrid.cuh).
+struct VoxGrid {
+    float org[3], size[3], inv[3];  // lower corner, cell sides and their inverses
+    int n[3];                       // cells per axis
+    float tol, tolf[3];             // closeness to a cell face: a length, and per axis in cells
+    const float4 *cells;            // [n0*n1*n2*2] (lo.xyz, extinction), (hi.xyz, original index); extinction 0: empty
+};
+
 // Scene as the trace kernels see it.
 struct TraceScene {
     const float4 *rec;    // [n*4] intersection records, BVH leaf order
     const float4 *nodes;  // [max(n-1,1)*4] BVH2 nodes
     const float4 *nodes4; // [n4*4] compressed 4-wide nodes (hrt_device.cuh), root 0
     int n4;
+    const float4 *nodes4s; // [n4s*4] 4-wide nodes over the surfaces alone (scenes with a voxel lattice)
+    int n4s;
+    const VoxGrid *vgrid; // the lattice (null: none; voxels are leaves of the tree)
     const float4 *rgen;   // [n*4] ray-origin records, original order
     const float4 *bbox;   // [nbbox*4] periodic wall corners (xyz, w unused)
     int n;
@@ -283,6 +294,8 @@ enum DiffuseVariant {
 bool is_w4s_variant(int v);
 cudaError_t launch_w4s(const DiffuseParams &p, int variant, cudaStream_t s);
 cudaError_t launch_w4s_record(const DiffuseParams &p, uint32_t *hits, int variant, cudaStream_t s);
+// Scenes with a voxel lattice (sc.vgrid).
+cudaError_t launch_w4s_voxels(const DiffuseParams &p, cudaStream_t s);
 cudaError_t launch_w4s_covers(const DiffuseParams &p, cudaStream_t s);
 cudaError_t launch_w4s_stats(const DiffuseParams &p, int variant, cudaStream_t s);
 // Multi-scene recording launch: p.fetch, p.faces, p.slots / nslots / multi_total set; the

@@ -22,7 +22,7 @@ unsigned w4_grid(const DiffuseParams &p, int resident, int block) {
 }
 
 template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB = 1, bool MULTI = false, bool LIN = false,
-          bool COV = false>
+          bool COV = false, bool VG = false>
 cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
     // resident blocks of one wave (SMs x blocks per SM); initialised once per instantiation,
     // thread-safe (the server launches from several threads)
@@ -31,15 +31,15 @@ cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
-                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV>,
+                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV, VG>,
                                                       BLOCK, 0);
         return (sms < 1 ? 1 : sms) * (per_sm < 1 ? 1 : per_sm);
     }();
     cudaError_t e = cudaMemsetAsync(p.fetch, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
     DiffuseParams q = p;
-    q.refill = refill_threshold(false, true);
-    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
+    q.refill = refill_threshold(false, true, VG);
+    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV, VG><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -95,6 +95,14 @@ cudaError_t launch_w4s_covers(const DiffuseParams &p, cudaStream_t s) {
     if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true, true>(p, s);
     if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true, true>(p, s);
     if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true, true>(p, s);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_w4s_voxels(const DiffuseParams &p, cudaStream_t s) {
+    if (!p.sc.vgrid) return cudaErrorInvalidValue;
+    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
+    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
+    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
     return cudaErrorInvalidValue;
 }
 

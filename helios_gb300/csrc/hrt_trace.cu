@@ -744,7 +744,11 @@ static cudaError_t diffuse_impl(const DiffuseParams &p, int variant, int max_blo
     if (total <= 0 || p.Bc <= 0) return cudaSuccess;
     if (variant == DV_DEFAULT) variant = default_variant();
     if ((variant == DV_W4 || variant == DV_W43 || is_w4s_variant(variant)) && !p.sc.nodes4) variant = DV_PS4;
-    if (is_w4s_variant(variant) && p.sc.voxels) variant = DV_W4;  // the lean kernel has no voxel code
+    // voxels that form a lattice: the lean trace marches them; others are leaves of the generic one
+    if (is_w4s_variant(variant) && p.sc.voxels) {
+        if (!STATS && p.sc.vgrid && p.fetch) return launch_w4s_voxels(p, s);
+        variant = DV_W4;
+    }
     if (p.fetch && variant != DV_SIMPLE) {
         if (STATS) {
             if (p.Bc <= 4 && is_w4s_variant(variant)) return launch_w4s_stats(p, variant, s);

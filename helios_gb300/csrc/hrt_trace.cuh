@@ -700,14 +700,17 @@ constexpr int kRefillDefault = 8;
 // vote: 8 162.5 ms, 10 160.4 ms, 12 160.2 ms, 14 161.2 ms, 16 162.7 ms, 18 161.8 ms, 20 161.1 ms,
 // 24 170.6 ms (run to run on one box within 0.02 ms).
 constexpr int kRefillLean = 12;
-inline int refill_threshold(bool voxels, bool lean = false) {
+// With a lattice of voxels to march a refill costs more code: on the deep-scattering section 4 362 ms of
+// diffuse launches, 6 364 ms, 8 369 ms, 12 377 ms.
+constexpr int kRefillLattice = 4;
+inline int refill_threshold(bool voxels, bool lean = false, bool lattice = false) {
     static const int env = [] {  // initialised once, thread-safe; -1: not set
         const char *e = getenv("HRT_REFILL");
         const int v = e ? atoi(e) : -1;
         return (v < -1 || v > 32) ? -1 : v;
     }();
     if (env >= 0) return env;
-    return voxels ? 0 : (lean ? kRefillLean : kRefillDefault);
+    return voxels ? 0 : (lattice ? kRefillLattice : (lean ? kRefillLean : kRefillDefault));
 }
 
 // Blocks of a persistent launch: one resident wave; with a lane budget, enough blocks

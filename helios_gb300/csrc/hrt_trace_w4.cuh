@@ -1,5 +1,5 @@
 // hrt_trace_w4.cuh -- the persistent diffuse trace over compressed 4-wide nodes for scenes
-// without voxels, laid out for occupancy.
+// without voxels or with a lattice of them, laid out for occupancy.
 //
 // The trace is bound by the latency of node fetches (L1/L2 hits) and by issue slots, not by
 // DRAM.  More resident warps hide more of that latency, so this kernel keeps only the state
@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "hrt_trace.cuh"
+#include "hrt_voxgrid.cuh"
 
 namespace hrt {
 
@@ -78,14 +79,16 @@ struct LinStack {
 // give a scene, a primitive chunk, ray counts, seed, pass and hit buffer, with consecutive
 // ranges of the launch's ray ids (id_begin) -- so one persistent launch covers the pass of
 // every scene of a multi-scene sweep.  LIN: the LinStack layout, else RingStack.  COV: translucent
-// covers of source 0 (P.sc.cover) are passed as if they were not there.
+// covers of source 0 (P.sc.cover) are passed as if they were not there.  VG: the scene's voxels form a
+// lattice (P.sc.vgrid): each ray segment marches it first and then walks the tree of the surfaces
+// (P.sc.nodes4s), bounded by the interception.
 template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB, bool MULTI = false, bool LIN = false,
-          bool COV = false>
+          bool COV = false, bool VG = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams P) {
     static_assert(!MULTI || (RECORD && !STATS), "multi-scene launches record hits only");
     __shared__ double s_sum[RECORD ? 1 : NB][BLOCK];            // running sums of the lane's origin
     __shared__ float s_ray[9][BLOCK];                            // d.xyz, Sx, Sy, Sz, o.xyz
-    __shared__ uint32_t s_lane[5][BLOCK];                        // see the L_* slots below
+    __shared__ uint32_t s_lane[VG ? 8 : 5][BLOCK];               // see the L_* slots below
     __shared__ int32_t s_stack[SD][BLOCK];
     __shared__ unsigned long long s_rid[RECORD ? BLOCK : 1];     // record: hit-buffer index
     __shared__ unsigned long long s_chunk[2][KB > 1 ? BLOCK / 32 : 1];  // per warp: next id, end
@@ -96,6 +99,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
     constexpr int L_HIT = 2;   // best hit so far: prim << 1 | face, or kMissCode
     constexpr int L_KEY = 3;   // running-sum key 2p + face, or 0xFFFFFFFF
     constexpr int L_TAKEN = 4; // rays taken (lane budget)
+    constexpr int L_RR = VG ? 5 : 0;    // VG: the ray's index in its primitive
+    constexpr int L_CELL = VG ? 6 : 0;  // VG: the march's state (VoxMarch)
+    constexpr int L_T0 = VG ? 7 : 0;
+    constexpr int32_t kMarch = kSentinel + 1;  // VG: the current node of a lane whose segment is marching
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const uint32_t R = (uint32_t)(P.dimx * P.dimy);
@@ -250,7 +257,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                         load_rgen(sc, p, g);
                         const uint32_t type = __float_as_uint(g[0].w);
                         f3 o, d;
-                        diffuse_ray_cell<false>(g, type, r, p, face, (int)ti, (int)pi, dxk, dyk, seedk, passk, &o, &d,
+                        diffuse_ray_cell<VG>(g, type, r, p, face, (int)ti, (int)pi, dxk, dyk, seedk, passk, &o, &d,
                                                 sc.masks);
                         const WT w = wt_setup(d);
                         s_ray[0][tid] = d.x;
@@ -268,7 +275,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                         inv = mk(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
                         ooi = mk(o.x * inv.x, o.y * inv.y, o.z * inv.z);
                         best = 1e38f;
-                        cur = (sc.n > 0) ? 0 : kSentinel;
+                        if (VG) {
+                            s_lane[L_RR][tid] = r;
+                            s_lane[L_CELL][tid] = kMarchNew;
+                        }
+                        cur = VG ? kMarch : ((sc.n > 0) ? 0 : kSentinel);
                         leaf = 0;
                         leaf2 = 0;
                         sp = kSp0;
@@ -289,9 +300,43 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         const unsigned lm = __ballot_sync(0xffffffffu, live);
         if (!live) continue;
 
+        // ---- lattice of voxels: lanes whose segment has not passed it step through its cells, together
+        // until fewer than four are left at it; then the surfaces are walked (with 4, 8, 14, 20 lanes the
+        // deep-scattering section took 450, 470, 535, 673 ms of diffuse launches)
+        if (VG && cur == kMarch) {
+            const VoxGrid &vg = *P.sc.vgrid;
+            const f3 o = mk(s_ray[6][tid], s_ray[7][tid], s_ray[8][tid]);
+            const f3 d = mk(s_ray[0][tid], s_ray[1][tid], s_ray[2][tid]);
+            const uint32_t ax = s_lane[L_AXES][tid];
+            const VoxKey vk{s_lane[L_RR][tid], s_lane[L_P][tid], ((ax >> 6) & 1u) | ((ax >> 8) << 16), P.seed, P.pass};
+            uint32_t code = s_lane[L_HIT][tid];
+            VoxMarch m{s_lane[L_CELL][tid], __uint_as_float(s_lane[L_T0][tid])};
+            float ta;
+            const float tb = vox_exit(vg, o, inv, &ta);
+            bool on = true;
+            if (m.cell == kMarchNew) {
+                on = ta <= tb;
+                if (on) vox_begin(vg, o, d, ta, &m);
+            }
+            // a segment steps through at most n0 + n1 + n2 cells, every round through one or more
+            while (on) {
+                on = vox_step(vg, o, ooi, inv, vk, tb, &m, &best, &code);
+                if (__popc(__activemask()) < 4) break;
+            }
+            s_lane[L_HIT][tid] = code;
+            if (on) {
+                s_lane[L_CELL][tid] = m.cell;
+                s_lane[L_T0][tid] = __float_as_uint(m.t0);
+            } else {
+                cur = P.sc.n4s > 0 ? 0 : kSentinel;
+            }
+        }
+
+        if (VG) __syncwarp(lm);
+
         // ---- internal nodes; up to two leaves per lane are postponed to the primitive tests below
         const TraceScene &sc = SC;
-        const uint32_t n4 = (uint32_t)sc.n4;
+        const uint32_t n4 = (uint32_t)(VG ? sc.n4s : sc.n4);
         // cur is an internal node: 0 <= cur < kSentinel in one unsigned compare (leaves are
         // negative; indices at or above n4 fail the bounds test inside)
         while ((uint32_t)cur < (uint32_t)kSentinel) {
@@ -307,7 +352,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             --budget;
             if (STATS) ++nvis;
             float4 q0, q1, q2, q3;
-            load_node64(sc.nodes4, cur, q0, q1, q2, q3);
+            load_node64(VG ? sc.nodes4s : sc.nodes4, cur, q0, q1, q2, q3);
             float tk[4];
             int32_t ck[4];  // every slot's reference: a child is hit when its tk < INFINITY
             node4_children<false>(q0, q1, q2, q3, node4_offset_ooi(q0, ooi, inv), inv, 1e-4f, best, tk, ck);
@@ -378,7 +423,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             w.Sy = s_ray[4][tid];
             w.Sz = s_ray[5][tid];
             uint32_t bcode = s_lane[L_HIT][tid];
-            const VoxKey vk{0u, 0u, 0u, 0u, 0u};  // no voxels in this kernel's scenes
+            const VoxKey vk{0u, 0u, 0u, 0u, 0u};  // no voxels among this kernel's leaves
             while (leaf != 0) {
                 const uint32_t slot = (uint32_t)(~leaf);
                 if (STATS) ++ntest;
@@ -434,7 +479,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                     best = 1e38f;
                     s_lane[L_HIT][tid] = kMissCode;
                     s_lane[L_AXES][tid] = (ax & 0xFFu) | ((wraps + 1u) << 8);
-                    cur = 0;
+                    if (VG) s_lane[L_CELL][tid] = kMarchNew;
+                    cur = VG ? kMarch : 0;
                     sp = kSp0;
                     budget = sc.visit_budget;
                     continue;

@@ -220,3 +220,56 @@ def test_periodic_walls_vs_oracle(oracle_mod, boundary):
     floor = 1e-3 * float(np.abs(ref).mean())
     assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
     assert rad.last_stats["rays"] == st["rays"]
+
+
+def _voxel_scene(form, seed=2):
+    """Leaves among voxels that are a full lattice, a lattice with holes, one layer, off the planes of
+    any lattice, and a lattice far from the origin of coordinates."""
+    rng = np.random.default_rng(seed)
+    leaves = scenes.mixed_canopy(300, 1.0, seed=seed, height=1.0)
+    div = (5, 4, 1) if form == "layer" else (5, 4, 3)
+    vox = scenes.voxel_grid((0.0, 0.0, 0.05), (0.85, 0.85, 1.0), div, rng.uniform(0.0, 3.0, int(np.prod(div))))
+    T, lad = vox.T.copy(), vox.lad
+    if form == "holes":
+        keep = rng.random(T.shape[0]) < 0.5
+        T, lad = T[keep], lad[keep]
+    if form == "shifted":
+        T[::3, 3] += 0.03
+    ty = np.concatenate([leaves.ptype, np.full(T.shape[0], scenes.VOXEL, np.uint32)])
+    T = np.concatenate([leaves.T, T])
+    if form == "far":
+        T[:, [3, 7]] += 500.0
+    return T, ty, np.concatenate([leaves.twosided, np.ones(lad.size, np.int8)]), np.concatenate([np.zeros(leaves.n), lad])
+
+
+@pytest.mark.parametrize("form", ["full", "holes", "layer", "shifted", "far"])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_voxel_lattices_vs_oracle(oracle_mod, form, periodic):
+    """Voxels that are marched as a lattice, and some that are not one: fluxes and ray counts."""
+    from helios_gb300.radiation import Context, RadiationModel
+    from helpers import run_oracle
+
+    T, ty, ts, lad = _voxel_scene(form)
+    ctx = Context()
+    uu = ctx.addPrimitives(T, ty, 1.0, ts)
+    ctx.setPrimitiveData(uu, "leaf_area_density", lad)
+    ctx.setPrimitiveData(uu[1:], "reflectivity_SW", np.full(uu.size - 1, 0.4))
+    ctx.setPrimitiveData(uu[1:], "transmissivity_SW", np.full(uu.size - 1, 0.3))
+    rad = RadiationModel(ctx)
+    if periodic:
+        rad.enforcePeriodicBoundary("xy")
+    rad.addRadiationBand("SW")
+    rad.disableEmission("SW")
+    s = rad.addCollimatedRadiationSource(scenes.sun_direction(35.0, 200.0))
+    rad.setSourceFlux(s, "SW", 600.0)
+    rad.setDiffuseRadiationFlux("SW", 100.0)
+    rad.setDirectRayCount("SW", 25)
+    rad.setDiffuseRayCount("SW", 100)
+    rad.setScatteringDepth("SW", 3)
+    rad.setSeed(7)
+    got = rad.runBand("SW").astype(np.float64)
+    ref, st = run_oracle(rad, ["SW"], oracle_mod, seed=7)
+    floor = 1e-3 * float(np.abs(ref).mean())
+    assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
+    assert rad.last_stats["rays"] == st["rays"]
+    assert rad.ctx.device_status() == 0
