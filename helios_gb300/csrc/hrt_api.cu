@@ -80,23 +80,6 @@ void keep_pool(int device) {
     done.push_back(device);
 }
 
-// Surface area of a primitive in FP64 from its FP32 transform (a voxel's: its leaf area,
-// LAD x volume).  Triangles span half the parallelogram of their two edges, disks are
-// the unit disk scaled by the transform.
-double prim_area(const float *T, uint32_t type, float lad) {
-    double ax = T[0], ay = T[4], az = T[8], bx = T[1], by = T[5], bz = T[9];
-    if (type == PT_VOXEL) {
-        double cx = T[2], cy = T[6], cz = T[10];
-        double det = ax * (by * cz - bz * cy) - bx * (ay * cz - az * cy) + cx * (ay * bz - az * by);
-        return (double)lad * std::fabs(det);
-    }
-    double x = ay * bz - az * by, y = az * bx - ax * bz, z = ax * by - ay * bx;
-    double a = std::sqrt(x * x + y * y + z * z);
-    if (type == PT_TRI) return 0.5 * a;
-    if (type == PT_DISK) return M_PI * a;
-    return a;
-}
-
 // Do the voxels form a regular lattice?  Boxes as the records hold them (make_records, FP32): equal
 // sides, corners on the planes of one lattice within a thousandth of a cell, no cell twice, and not
 // so sparse that the table of cells outgrows them 16 times.  Fills g but for its device pointer and
@@ -1095,20 +1078,18 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     CU(ctx->area.ensure(ctx->stream, std::max<size_t>(n, 1) * sizeof(double)));
     ctx->h_twosided.assign(g->twosided, g->twosided + n);
     for (uint32_t i : voxels) ctx->h_twosided[i] = 1;  // a voxel launches both directions of each sample
-    // primitive areas (voxels: leaf area) weight the scattering residual
-    std::vector<double> area(n);
-    for (size_t i = 0; i < n; ++i)
-        area[i] = prim_area(g->transform + 16 * i, g->type[i], g->type[i] == PT_VOXEL ? g->voxel_lad[i] : 0.f);
     if (n) {
         CU(cudaMemcpyAsync(ctx->T.p, g->transform, n * 16 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(ctx->type.p, g->type, n * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(ctx->twosided.p, ctx->h_twosided.data(), n, cudaMemcpyHostToDevice, ctx->stream));
-        CU(cudaMemcpyAsync(ctx->area.p, area.data(), n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     }
     if (!voxels.empty()) {
         CU(ctx->lad.ensure(ctx->stream, n * sizeof(float)));
         CU(cudaMemcpyAsync(ctx->lad.p, g->voxel_lad, n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
+    // primitive areas (voxels: leaf area) weight the scattering residual
+    CU(launch_prim_area((int)n, ctx->T.as<float>(), ctx->type.as<uint32_t>(), ctx->lad.as<float>(),
+                        ctx->area.as<double>(), ctx->stream));
     ctx->have_lattice = ctx->use_lattice = false;
     if (!voxels.empty() && voxels.size() + 2 <= n) {
         float far = 0.f;  // periodic wraps stay within the walls, which hold the scene
@@ -1223,8 +1204,7 @@ int hrt_build_accel(hrt_context *ctx) {
     b.status = ctx->status.as<uint32_t>();
     CU(bvh_build(ctx->T.as<float>(), ctx->type.as<uint32_t>(), ctx->h_voxels.empty() ? nullptr : ctx->lad.as<float>(), n,
                  b, ctx->stream));
-    int r = sync_and_status(ctx);
-    if (r) return r;
+    int r;
     // compressed 4-wide nodes for the persistent diffuse trace (scratch reuses the build's)
     ctx->n4 = 0;
     ctx->sg_extent_ready = false;

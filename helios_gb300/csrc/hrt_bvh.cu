@@ -92,16 +92,25 @@ __global__ void k_bounds_partial(int n, const float *__restrict__ aabb, float *_
 }
 
 // Final bounds: out[0..2] clo, [3..5] chi, [6..8] blo, [9..11] bhi, [12..14] Morton scale, [15] extent.
-__global__ void k_bounds_final(int nparts, const float *__restrict__ partial, float *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float v[12];
-    for (int k = 0; k < 12; ++k) v[k] = partial[k];
-    for (int p = 1; p < nparts; ++p)
-        for (int k = 0; k < 12; ++k) {
-            float b = partial[12 * p + k];
-            bool mx = (k >= 3 && k < 6) || k >= 9;
-            v[k] = mx ? fmaxf(v[k], b) : fminf(v[k], b);
-        }
+// One warp per value (one thread looping over the partials took 170 us at 783 of them).
+__global__ void __launch_bounds__(384) k_bounds_final(int nparts, const float *__restrict__ partial,
+                                                      float *__restrict__ out) {
+    __shared__ float v[12];
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool mx = (k >= 3 && k < 6) || k >= 9;
+    float x = partial[k];
+    for (int p = 1 + lane; p < nparts; p += 32) {
+        const float b = partial[12 * p + k];
+        x = mx ? fmaxf(x, b) : fminf(x, b);
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const float b = __shfl_down_sync(0xffffffffu, x, d);
+        x = mx ? fmaxf(x, b) : fminf(x, b);
+    }
+    if (lane == 0) v[k] = x;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     float ext = 0.f;
     for (int k = 0; k < 3; ++k) {
         out[k] = v[k];
@@ -212,6 +221,33 @@ __global__ void k_scan_blocks(const uint32_t *__restrict__ in, uint32_t *__restr
     if (threadIdx.x == 0 && sums) sums[blockIdx.x] = tot;
 }
 
+// Exclusive scan of a few tiles by one block, tile after tile: one launch where three short ones would
+// follow each other.
+__global__ void __launch_bounds__(1024) k_scan_one(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
+                                                   int count) {
+    __shared__ uint32_t shw[32];
+    uint32_t carry = 0;
+    for (int base = 0; base < count; base += 1024 * kItems) {
+        uint32_t v[kItems];
+        uint32_t loc = 0;
+#pragma unroll
+        for (int j = 0; j < kItems; ++j) {
+            const int i = base + threadIdx.x * kItems + j;
+            v[j] = (i < count) ? in[i] : 0u;
+            loc += v[j];
+        }
+        uint32_t tot;
+        uint32_t run = carry + block_excl_scan(loc, &tot, shw);
+#pragma unroll
+        for (int j = 0; j < kItems; ++j) {
+            const int i = base + threadIdx.x * kItems + j;
+            if (i < count) out[i] = run;
+            run += v[j];
+        }
+        carry += tot;
+    }
+}
+
 __global__ void k_scan_add(uint32_t *__restrict__ out, int count, const uint32_t *__restrict__ sums) {
     int base = blockIdx.x * kSortTile;
     uint32_t add = sums[blockIdx.x];
@@ -292,8 +328,8 @@ __global__ void k_scatter(int n, const uint64_t *__restrict__ kin, const uint32_
 // Exclusive scan of `count` u32 values (count <= kSortTile^2).
 cudaError_t scan_u32(const uint32_t *in, uint32_t *out, int count, uint32_t *tmp, cudaStream_t s) {
     int nb = (count + kSortTile - 1) / kSortTile;
-    if (nb <= 1) {
-        k_scan_blocks<<<1, kThreads, 0, s>>>(in, out, count, nullptr);
+    if (count <= 32768) {  // four tiles of the one block
+        k_scan_one<<<1, 1024, 0, s>>>(in, out, count);
         return cudaGetLastError();
     }
     uint32_t *sums = tmp, *sums_scan = tmp + nb;
@@ -420,6 +456,28 @@ __global__ void k_single(const float *__restrict__ leafbox, float4 *__restrict__
     write_node(nodes, 0, b0, b1, ~0, kEmptyChild);
 }
 
+// Surface area of a primitive in FP64 from its FP32 transform (a voxel's: its leaf area, LAD x
+// volume).  Triangles span half the parallelogram of their two edges, disks are the unit disk scaled
+// by the transform.
+__global__ void k_prim_area(int n, const float *__restrict__ T, const uint32_t *__restrict__ type,
+                            const float *__restrict__ lad, double *__restrict__ area) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 *t = reinterpret_cast<const float4 *>(T) + 4 * (size_t)i;
+    const float4 r0 = __ldg(t), r1 = __ldg(t + 1), r2 = __ldg(t + 2);
+    const double ax = r0.x, ay = r1.x, az = r2.x, bx = r0.y, by = r1.y, bz = r2.y;
+    const uint32_t ty = type[i];
+    if (ty == PT_VOXEL) {
+        const double cx = r0.z, cy = r1.z, cz = r2.z;
+        const double det = ax * (by * cz - bz * cy) - bx * (ay * cz - az * cy) + cx * (ay * bz - az * by);
+        area[i] = (double)lad[i] * fabs(det);
+        return;
+    }
+    const double x = ay * bz - az * by, y = az * bx - ax * bz, z = ax * by - ay * bx;
+    const double a = sqrt(x * x + y * y + z * z);
+    area[i] = ty == PT_TRI ? 0.5 * a : (ty == PT_DISK ? 3.14159265358979323846 * a : a);
+}
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // ---------------------------------------------------------------- PLOC
@@ -434,6 +492,20 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // 32 39.4 / 1.93, 64 38.9 / 1.98, 128 38.2 / 1.97.  HRT_PLOC_RADIUS overrides (1-256).
 constexpr int kPlocRadius = 64;
 
+// A round is three launches and nothing waits for the host: the cluster count lives on the device, and
+// rounds are queued ahead with grids for the count expected (every kernel strides over what there is).
+// From kPlocTail clusters on one block finishes the tree in shared memory.  With some ten launches and
+// a host synchronisation in each of about 45 rounds the clustering was 3.5 of the 4.8 ms of a build of
+// 200,004 primitives.
+constexpr int kPlocTail = 1024;
+constexpr int kPlocTile = 1024;      // clusters per block of the counting and merging kernels
+constexpr int kPlocRounds = 64;      // rounds that one batch may queue
+constexpr int kPlocMaxRadius = 256;
+
+struct PlocState {
+    int m, next_free, cur;  // clusters, node index the next merge takes, buffer that holds the clusters
+};
+
 __device__ __forceinline__ float merged_area(const float *a, const float *b) {
     const float dx = fmaxf(a[3], b[3]) - fminf(a[0], b[0]);
     const float dy = fmaxf(a[4], b[4]) - fminf(a[1], b[1]);
@@ -442,82 +514,238 @@ __device__ __forceinline__ float merged_area(const float *a, const float *b) {
 }
 
 __global__ void k_ploc_init(int n, const float *__restrict__ leafbox, float *__restrict__ cbox,
-                            int32_t *__restrict__ cid) {
+                            int32_t *__restrict__ cid, PlocState *st) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *st = PlocState{n, n - 2, 0};
     if (i >= n) return;
 #pragma unroll
     for (int k = 0; k < 6; ++k) cbox[6 * (size_t)i + k] = leafbox[6 * (size_t)i + k];
     cid[i] = ~i;
 }
 
-__global__ void k_ploc_nn(int m, int radius, const float *__restrict__ cbox, int32_t *__restrict__ nn) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    float a[6];
+// Nearest neighbour of every cluster: a block's clusters and the radius on both sides of them in
+// shared memory (each box is read from there up to 2 x radius times).
+__global__ void __launch_bounds__(kThreads) k_ploc_nn(const PlocState *__restrict__ st, int radius,
+                                                      const float *box0, const float *box1, int32_t *__restrict__ nn) {
+    __shared__ float sh[6][kThreads + 2 * kPlocMaxRadius];
+    const int m = st->m;
+    if (m <= kPlocTail) return;
+    const float *cbox = st->cur ? box1 : box0;
+    for (int base = blockIdx.x * kThreads; base < m; base += gridDim.x * kThreads) {
+        const int first = base - radius < 0 ? 0 : base - radius;
+        const int last = base + kThreads + radius > m ? m : base + kThreads + radius;  // exclusive
+        __syncthreads();
+        for (int t = threadIdx.x; t < 6 * (last - first); t += kThreads) sh[t % 6][t / 6] = cbox[6 * (size_t)first + t];
+        __syncthreads();
+        const int i = base + threadIdx.x;
+        if (i < m) {
+            float a[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) a[k] = cbox[6 * (size_t)i + k];
-    float best = INFINITY;
-    int bj = -1;
-    const int lo = i - radius < 0 ? 0 : i - radius;
-    const int hi = i + radius > m - 1 ? m - 1 : i + radius;
-    for (int j = lo; j <= hi; ++j) {
-        if (j == i) continue;
-        float b[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) b[k] = __ldg(cbox + 6 * (size_t)j + k);
-        const float d = merged_area(a, b);
-        if (d < best) {  // j ascends: equal areas keep the smaller index
-            best = d;
-            bj = j;
+            for (int k = 0; k < 6; ++k) a[k] = sh[k][i - first];
+            float best = INFINITY;
+            int bj = -1;
+            const int lo = i - radius < 0 ? 0 : i - radius;
+            const int hi = i + radius > m - 1 ? m - 1 : i + radius;
+            for (int j = lo; j <= hi; ++j) {
+                const int q = j - first;
+                const float b[6] = {sh[0][q], sh[1][q], sh[2][q], sh[3][q], sh[4][q], sh[5][q]};
+                const float d = merged_area(a, b);
+                if (d < best && j != i) {  // j ascends: equal areas keep the smaller index
+                    best = d;
+                    bj = j;
+                }
+            }
+            nn[i] = bj;
         }
     }
-    nn[i] = bj;
 }
 
-// create[i] = 1 when cluster i starts a mutual pair (i < nn[i]); keep[i] = 0 for the partner.
-__global__ void k_ploc_flags(int m, const int32_t *__restrict__ nn, uint32_t *__restrict__ create,
-                             uint32_t *__restrict__ keep) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
+// 1: cluster i starts a mutual pair (i < nn[i]) and becomes a new node; 2: it stays as it is; 0: it is
+// the partner of a pair.
+__device__ __forceinline__ int ploc_role(int i, int m, const int32_t *nn) {
     const int j = nn[i];
     const bool mutual = j >= 0 && j < m && nn[j] == i;
-    create[i] = (mutual && i < j) ? 1u : 0u;
-    keep[i] = (mutual && i > j) ? 0u : 1u;
+    return mutual ? (i < j ? 1 : 0) : 2;
 }
 
-__global__ void k_ploc_merge(int m, const int32_t *__restrict__ nn, const uint32_t *__restrict__ create,
-                             const uint32_t *__restrict__ rank, int next_free, float *__restrict__ cbox,
-                             int32_t *__restrict__ cid, float4 *__restrict__ nodes) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !create[i]) return;
-    const int j = nn[i];
-    const int node = next_free - (int)rank[i];
-    float a[6], b[6], u[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        a[k] = cbox[6 * (size_t)i + k];
-        b[k] = cbox[6 * (size_t)j + k];
+// New nodes (low half) and clusters left (high half) of each tile.
+__global__ void __launch_bounds__(kThreads) k_ploc_count(const PlocState *__restrict__ st,
+                                                         const int32_t *__restrict__ nn, uint2 *__restrict__ tiles) {
+    __shared__ uint32_t sc, sk;
+    const int m = st->m;
+    if (m <= kPlocTail) return;
+    const int ntile = (m + kPlocTile - 1) / kPlocTile;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        __syncthreads();
+        if (threadIdx.x == 0) sc = sk = 0u;
+        __syncthreads();
+        uint32_t c = 0, k = 0;
+        for (int q = threadIdx.x; q < kPlocTile; q += kThreads) {
+            const int i = tile * kPlocTile + q;
+            if (i >= m) break;
+            const int role = ploc_role(i, m, nn);
+            c += role == 1;
+            k += role != 0;
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        k = __reduce_add_sync(0xffffffffu, k);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&sc, c);
+            atomicAdd(&sk, k);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) tiles[tile] = make_uint2(sc, sk);
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        u[k] = fminf(a[k], b[k]);
-        u[3 + k] = fmaxf(a[3 + k], b[3 + k]);
-    }
-    write_node(nodes, node, a, b, cid[i], cid[j]);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) cbox[6 * (size_t)i + k] = u[k];
-    cid[i] = node;
 }
 
-__global__ void k_ploc_compact(int m, const uint32_t *__restrict__ keep, const uint32_t *__restrict__ pos,
-                               const float *__restrict__ cbox, const int32_t *__restrict__ cid,
-                               float *__restrict__ cbox2, int32_t *__restrict__ cid2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !keep[i]) return;
-    const uint32_t o = pos[i];
+// Merge the pairs and move the clusters left to the other buffer, in order: a tile's places follow
+// the sums over the tiles before it, which every block adds up for itself.
+__global__ void __launch_bounds__(kThreads) k_ploc_merge(const PlocState *__restrict__ st, PlocState *next,
+                                                         const int32_t *__restrict__ nn, const uint2 *__restrict__ tiles,
+                                                         float *box0, float *box1, int32_t *cid0, int32_t *cid1,
+                                                         float4 *__restrict__ nodes) {
+    __shared__ uint32_t shw[32];
+    const int m = st->m;
+    if (m <= kPlocTail) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *next = *st;
+        return;
+    }
+    const bool flip = st->cur != 0;
+    const float *ibox = flip ? box1 : box0;
+    const int32_t *icid = flip ? cid1 : cid0;
+    float *obox = flip ? box0 : box1;
+    int32_t *ocid = flip ? cid0 : cid1;
+    const int ntile = (m + kPlocTile - 1) / kPlocTile;
+    constexpr int kPer = kPlocTile / kThreads;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        uint32_t c = 0, k = 0;
+        for (int t = threadIdx.x; t < tile; t += kThreads) {
+            const uint2 v = __ldg(tiles + t);
+            c += v.x;
+            k += v.y;
+        }
+        uint32_t before_c, before_k;
+        block_excl_scan(c, &before_c, shw);
+        block_excl_scan(k, &before_k, shw);
+        int role[kPer];
+        uint32_t lc = 0, lk = 0;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) cbox2[6 * (size_t)o + k] = cbox[6 * (size_t)i + k];
-    cid2[o] = cid[i];
+        for (int q = 0; q < kPer; ++q) {
+            const int i = tile * kPlocTile + threadIdx.x * kPer + q;
+            role[q] = i < m ? ploc_role(i, m, nn) : 0;
+            lc += role[q] == 1;
+            lk += role[q] != 0;
+        }
+        uint32_t tot_c, tot_k;
+        uint32_t rank = before_c + block_excl_scan(lc, &tot_c, shw);
+        uint32_t pos = before_k + block_excl_scan(lk, &tot_k, shw);
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            if (role[q] == 0) continue;
+            const int i = tile * kPlocTile + threadIdx.x * kPer + q;
+            float a[6];
+#pragma unroll
+            for (int x = 0; x < 6; ++x) a[x] = ibox[6 * (size_t)i + x];
+            int32_t id = icid[i];
+            if (role[q] == 1) {
+                const int j = nn[i];
+                float b[6];
+#pragma unroll
+                for (int x = 0; x < 6; ++x) b[x] = ibox[6 * (size_t)j + x];
+                const int node = st->next_free - (int)rank++;
+                write_node(nodes, node, a, b, id, icid[j]);
+                id = node;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    a[x] = fminf(a[x], b[x]);
+                    a[3 + x] = fmaxf(a[3 + x], b[3 + x]);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 6; ++x) obox[6 * (size_t)pos + x] = a[x];
+            ocid[pos] = id;
+            ++pos;
+        }
+        if (tile == ntile - 1 && threadIdx.x == 0)
+            *next = PlocState{(int)(before_k + tot_k), st->next_free - (int)(before_c + tot_c), flip ? 0 : 1};
+        __syncthreads();
+    }
+}
+
+// The last kPlocTail clusters by one block: the same rounds, a thread a cluster, in shared memory.
+__global__ void __launch_bounds__(kPlocTail) k_ploc_tail(PlocState *st, int radius, const float *box0, const float *box1,
+                                                         const int32_t *cid0, const int32_t *cid1,
+                                                         float4 *__restrict__ nodes) {
+    __shared__ float sh[6][kPlocTail];
+    __shared__ int32_t sid[kPlocTail], snn[kPlocTail];
+    __shared__ uint32_t shw[32];
+    int m = st->m, next_free = st->next_free;
+    if (m > kPlocTail) return;
+    const float *ibox = st->cur ? box1 : box0;
+    const int32_t *icid = st->cur ? cid1 : cid0;
+    const int i = threadIdx.x;
+    for (int t = i; t < 6 * m; t += kPlocTail) sh[t % 6][t / 6] = ibox[t];
+    if (i < m) sid[i] = icid[i];
+    __syncthreads();
+    while (m > 1) {
+        if (i < m) {
+            float a[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) a[k] = sh[k][i];
+            float best = INFINITY;
+            int bj = -1;
+            const int lo = i - radius < 0 ? 0 : i - radius;
+            const int hi = i + radius > m - 1 ? m - 1 : i + radius;
+            for (int j = lo; j <= hi; ++j) {
+                const float b[6] = {sh[0][j], sh[1][j], sh[2][j], sh[3][j], sh[4][j], sh[5][j]};
+                const float d = merged_area(a, b);
+                if (d < best && j != i) {
+                    best = d;
+                    bj = j;
+                }
+            }
+            snn[i] = bj;
+        }
+        __syncthreads();
+        const int role = i < m ? ploc_role(i, m, snn) : 0;
+        uint32_t made, left;
+        const uint32_t rank = block_excl_scan(role == 1 ? 1u : 0u, &made, shw);
+        const uint32_t pos = block_excl_scan(role != 0 ? 1u : 0u, &left, shw);
+        if (made == 0) break;  // no mutual pair (boxes that are not finite): the host sees m > 1
+        float a[6];
+        int32_t id = 0;
+        if (role != 0) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) a[k] = sh[k][i];
+            id = sid[i];
+            if (role == 1) {
+                const int j = snn[i], node = next_free - (int)rank;
+                float b[6];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) b[k] = sh[k][j];
+                write_node(nodes, node, a, b, id, sid[j]);
+                id = node;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    a[k] = fminf(a[k], b[k]);
+                    a[3 + k] = fmaxf(a[3 + k], b[3 + k]);
+                }
+            }
+        }
+        __syncthreads();
+        if (role != 0) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) sh[k][pos] = a[k];
+            sid[pos] = id;
+        }
+        next_free -= (int)made;
+        m = (int)left;
+        __syncthreads();
+    }
+    if (i == 0) {
+        st->m = m;
+        st->next_free = next_free;
+    }
 }
 
 }  // namespace
@@ -552,6 +780,13 @@ void bvh_carve(BvhBuffers &bb, void *scratch, int n) {
     bb.flags = (uint32_t *)take(ni * sizeof(uint32_t));
 }
 
+cudaError_t launch_prim_area(int n, const float *T, const uint32_t *type, const float *lad, double *area,
+                             cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    k_prim_area<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, T, type, lad, area);
+    return cudaGetLastError();
+}
+
 cudaError_t bvh_build(const float *T, const uint32_t *type, const float *lad, int n, BvhBuffers &b, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     if (n > 33000000) return cudaErrorInvalidValue;  // radix-sort offset scan covers 2048^2 bins
@@ -559,7 +794,7 @@ cudaError_t bvh_build(const float *T, const uint32_t *type, const float *lad, in
     k_records<<<grid, kThreads, 0, s>>>(n, T, type, lad, b.rec_tmp, b.rgen, b.aabb);
     int nparts = grid < 1024 ? grid : 1024;
     k_bounds_partial<<<nparts, kThreads, 0, s>>>(n, b.aabb, b.partial);
-    k_bounds_final<<<1, 32, 0, s>>>(nparts, b.partial, b.bounds);
+    k_bounds_final<<<1, 384, 0, s>>>(nparts, b.partial, b.bounds);
     k_morton<<<grid, kThreads, 0, s>>>(n, b.aabb, b.bounds, type, b.codes, b.perm);
     // 8 LSD passes; even pass count leaves the result in (codes, perm).
     const int nblk = (n + kSortTile - 1) / kSortTile;
@@ -596,36 +831,10 @@ cudaError_t bvh_build(const float *T, const uint32_t *type, const float *lad, in
     return cudaGetLastError();
 }
 
-// Exclusive scan of any length (tiles of kSortTile, sums scanned recursively); tmp holds
-// ploc_scan_tmp(count) words.
-static size_t scan_tmp_words(int count) {
-    size_t w = 64;
-    for (int c = count; c > kSortTile;) {
-        const int nb = (c + kSortTile - 1) / kSortTile;
-        w += 2 * (size_t)nb;
-        c = nb;
-    }
-    return w;
-}
-
-static cudaError_t scan_any(const uint32_t *in, uint32_t *out, int count, uint32_t *tmp, cudaStream_t s) {
-    const int nb = (count + kSortTile - 1) / kSortTile;
-    if (nb <= 1) {
-        k_scan_blocks<<<1, kThreads, 0, s>>>(in, out, count, nullptr);
-        return cudaGetLastError();
-    }
-    uint32_t *sums = tmp, *sums_scan = tmp + nb;
-    k_scan_blocks<<<nb, kThreads, 0, s>>>(in, out, count, sums);
-    cudaError_t e = scan_any(sums, sums_scan, nb, tmp + 2 * nb, s);
-    if (e != cudaSuccess) return e;
-    k_scan_add<<<nb, kThreads, 0, s>>>(out, count, sums_scan);
-    return cudaGetLastError();
-}
-
 size_t ploc_scratch_bytes(int n) {
     const size_t nn = (size_t)(n > 1 ? n : 1);
-    return 2 * align256(nn * 6 * sizeof(float)) + 2 * align256(nn * sizeof(int32_t)) +
-           4 * align256(nn * sizeof(uint32_t)) + align256(scan_tmp_words(n) * sizeof(uint32_t));
+    return 2 * align256(nn * 6 * sizeof(float)) + 3 * align256(nn * sizeof(int32_t)) +
+           align256((nn / kPlocTile + 1) * sizeof(uint2)) + align256((kPlocRounds + 1) * sizeof(PlocState));
 }
 
 static int ploc_radius() {
@@ -650,37 +859,38 @@ cudaError_t ploc_build(const float *leafbox, int n, float4 *nodes, void *scratch
     float *box[2] = {(float *)take(nn * 6 * sizeof(float)), (float *)take(nn * 6 * sizeof(float))};
     int32_t *cid[2] = {(int32_t *)take(nn * sizeof(int32_t)), (int32_t *)take(nn * sizeof(int32_t))};
     int32_t *nn_idx = (int32_t *)take(nn * sizeof(int32_t));
-    uint32_t *create = (uint32_t *)take(nn * sizeof(uint32_t));
-    uint32_t *rank = (uint32_t *)take(nn * sizeof(uint32_t));
-    uint32_t *keep = (uint32_t *)take(nn * sizeof(uint32_t));
-    uint32_t *tmp = (uint32_t *)take(scan_tmp_words(n) * sizeof(uint32_t));
-    uint32_t *pos = create;  // reused after the merge
-    k_ploc_init<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, leafbox, box[0], cid[0]);
-    int m = n, cur = 0, next_free = n - 2;
-    for (int iter = 0; m > 1; ++iter) {
-        if (iter > 4 * 1024) return cudaErrorInvalidValue;  // each round merges at least one pair
-        const int g = (m + kThreads - 1) / kThreads;
-        k_ploc_nn<<<g, kThreads, 0, s>>>(m, radius, box[cur], nn_idx);
-        k_ploc_flags<<<g, kThreads, 0, s>>>(m, nn_idx, create, keep);
-        cudaError_t e = scan_any(create, rank, m, tmp, s);
+    uint2 *tiles = (uint2 *)take((nn / kPlocTile + 1) * sizeof(uint2));
+    PlocState *st = (PlocState *)take((kPlocRounds + 1) * sizeof(PlocState));
+    k_ploc_init<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, leafbox, box[0], cid[0], st);
+    PlocState h{n, n - 2, 0};
+    for (int queued = 0; h.m > 1;) {
+        // boxes that all tie merge one pair a round: such scenes are refused, not clustered for minutes
+        if (queued > 4 * 1024) return cudaErrorInvalidValue;
+        // A round leaves about 0.73 of the clusters; a batch queues the rounds that lead to the tail at
+        // 0.8 (grids sized for that, which a slower round outgrows only by striding).
+        int rounds = 0;
+        double expect = (double)h.m;
+        for (; expect > kPlocTail && rounds < kPlocRounds; ++rounds, expect *= 0.8) {
+            const long long m = (long long)expect;
+            const unsigned gn = (unsigned)((m + kThreads - 1) / kThreads);
+            const unsigned gt = (unsigned)((m + kPlocTile - 1) / kPlocTile);
+            k_ploc_nn<<<gn, kThreads, 0, s>>>(st + rounds, radius, box[0], box[1], nn_idx);
+            k_ploc_count<<<gt, kThreads, 0, s>>>(st + rounds, nn_idx, tiles);
+            k_ploc_merge<<<gt, kThreads, 0, s>>>(st + rounds, st + rounds + 1, nn_idx, tiles, box[0], box[1], cid[0],
+                                                 cid[1], nodes);
+        }
+        queued += rounds;
+        k_ploc_tail<<<1, kPlocTail, 0, s>>>(st + rounds, radius, box[0], box[1], cid[0], cid[1], nodes);
+        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        uint32_t h[2];  // merges this round: last rank + last flag
-        if ((e = cudaMemcpyAsync(&h[0], rank + (m - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+        const int before = h.m;
+        if ((e = cudaMemcpyAsync(&h, st + rounds, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+        if (rounds > 0 && (e = cudaMemcpyAsync(st, st + rounds, sizeof h, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
             return e;
-        if ((e = cudaMemcpyAsync(&h[1], create + (m - 1), sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-            return e;
-        k_ploc_merge<<<g, kThreads, 0, s>>>(m, nn_idx, create, rank, next_free, box[cur], cid[cur], nodes);
-        if ((e = scan_any(keep, pos, m, tmp, s)) != cudaSuccess) return e;
-        k_ploc_compact<<<g, kThreads, 0, s>>>(m, keep, pos, box[cur], cid[cur], box[1 - cur], cid[1 - cur]);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        const int merged = (int)(h[0] + h[1]);
-        if (merged <= 0) return cudaErrorInvalidValue;
-        next_free -= merged;
-        m -= merged;
-        cur = 1 - cur;
+        if (h.m > 1 && h.m >= before) return cudaErrorInvalidValue;  // each round merges at least one pair
     }
-    return next_free == -1 ? cudaSuccess : cudaErrorInvalidValue;
+    return h.next_free == -1 ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 }  // namespace hrt

@@ -73,16 +73,11 @@ __device__ __forceinline__ uint32_t quant_hi(float p, float lo, float v, float S
     return (uint32_t)q;
 }
 
-// One wave: item i turns binary node in[i].x into 4-wide node in[i].y.
-// cap: 4-wide nodes n4 holds; qcap: items the wave queues hold.
-__global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float4 *__restrict__ n2,
-                                                        const int2 *__restrict__ in, int nin, int2 *__restrict__ out,
-                                                        unsigned *__restrict__ nout, unsigned *__restrict__ nnodes,
-                                                        int cap, int qcap, float4 *__restrict__ n4,
-                                                        uint32_t *__restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nin) return;
-    const int32_t b = in[i].x, q = in[i].y;
+// Binary node b as 4-wide node q.
+__device__ __forceinline__ void collapse_one(int n2count, const float4 *__restrict__ n2, int32_t b, int32_t q,
+                                             int2 *__restrict__ out, unsigned *__restrict__ nout,
+                                             unsigned *__restrict__ nnodes, int cap, int qcap, float4 *__restrict__ n4,
+                                             uint32_t *__restrict__ status) {
     if (b < 0 || b >= n2count || q < 0 || q >= cap) {
         atomicOr(status, ERR_BOUNDS);
         return;
@@ -181,14 +176,38 @@ __global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float
     o[3] = make_float4(__int_as_float(outref[2]), __int_as_float(outref[3]), s[1], s[2]);
 }
 
+// One wave: item i turns binary node in[i].x into 4-wide node in[i].y; waves are queued ahead, so the
+// count of items is read on the device (*nin, at most qcap) and the grid strides over them.
+// cap: 4-wide nodes n4 holds; qcap: items the wave queues hold.
+__global__ void __launch_bounds__(kThreads4) k_collapse(int n2count, const float4 *__restrict__ n2,
+                                                        const int2 *__restrict__ in, const unsigned *__restrict__ nin_ptr, int2 *__restrict__ out,
+                                                        unsigned *__restrict__ nout, unsigned *__restrict__ nnodes,
+                                                        int cap, int qcap, float4 *__restrict__ n4,
+                                                        uint32_t *__restrict__ status) {
+    const int nin = (int)min(*nin_ptr, (unsigned)qcap);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nin; i += gridDim.x * blockDim.x)
+        collapse_one(n2count, n2, in[i].x, in[i].y, out, nout, nnodes, cap, qcap, n4, status);
+}
+
 }  // namespace
+
+constexpr int kWaves = 64;      // waves that one batch may queue
+constexpr int kMaxWaves = 264;  // levels of a tree: deeper than any over distinct Morton codes
 
 size_t bvh4_scratch_bytes(int n) {
     const size_t ni = (size_t)(n > 1 ? n - 1 : 1);
-    return 2 * ni * sizeof(int2) + 256;
+    return 2 * ni * sizeof(int2) + (kWaves + 2) * sizeof(unsigned) + 256;
 }
 
 size_t bvh4_node_capacity(int n) { return (size_t)(n > 1 ? n - 1 : 1) + 8; }
+
+// counters: [0] nodes allocated, [1 + w] items of wave w; the root is the one item of wave 0.
+// Node 0 is the root; node 1 pads the root's line, so the first allocation starts at 2.
+__global__ void k_collapse_init(int2 *queue, unsigned *counters) {
+    const int i = threadIdx.x;
+    if (i == 0) queue[0] = make_int2(0, 0);
+    if (i < kWaves + 2) counters[i] = i == 0 ? 2u : (i == 1 ? 1u : 0u);
+}
 
 cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratch, uint32_t *status, int *count_out,
                        cudaStream_t s) {
@@ -196,33 +215,45 @@ cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratc
     if (n <= 0) return cudaSuccess;
     const int ni = n > 1 ? n - 1 : 1;
     int2 *qa = (int2 *)scratch, *qb = qa + ni;
-    unsigned *counters = (unsigned *)(qb + ni);  // [0] next-wave items, [1] nodes allocated
-    const int2 root = make_int2(0, 0);
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(qa, &root, sizeof(int2), cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-    // node 0 is the root; node 1 pads the root's line, so the first allocation starts at 2
-    const unsigned first = 2;
-    if ((e = cudaMemcpyAsync(counters + 1, &first, sizeof(unsigned), cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
+    unsigned *counters = (unsigned *)(qb + ni);
     const int cap = (int)bvh4_node_capacity(n);
-    int nin = 1, waves = 0;
-    while (nin > 0) {
-        if (++waves > 4 * 64 + 8) return cudaErrorInvalidValue;  // deeper than any LBVH of 2^32 leaves
-        if ((e = cudaMemsetAsync(counters, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
-        k_collapse<<<(nin + kThreads4 - 1) / kThreads4, kThreads4, 0, s>>>(ni, nodes2, qa, nin, qb, counters,
-                                                                           counters + 1, cap, ni, nodes4, status);
+    cudaError_t e;
+    k_collapse_init<<<1, 128, 0, s>>>(qa, counters);
+    // A wave is a level of the 4-wide tree; a clustered tree of n leaves has little more than log2(n) of
+    // them.  Waves are queued without waiting for their counts (a host synchronisation in each was
+    // 0.5 ms of a build of 200,004 primitives) and the last one's count says whether more are needed.
+    int waves = 6, done = 0;
+    for (int c = n; c > 1; c >>= 1) ++waves;
+    if (waves > kWaves) waves = kWaves;
+    unsigned h[2] = {0, 0};  // nodes, items left
+    do {
+        long long most = 1;  // items of wave w: at most 4^w
+        for (int w = 0; w < waves; ++w) {
+            const long long items = done == 0 && most < ni ? most : ni;
+            unsigned grid = (unsigned)((items + kThreads4 - 1) / kThreads4);
+            if (grid > 1216) grid = 1216;
+            k_collapse<<<grid, kThreads4, 0, s>>>(ni, nodes2, qa, counters + 1 + w, qb, counters + 2 + w, counters, cap,
+                                                  ni, nodes4, status);
+            int2 *t = qa;
+            qa = qb;
+            qb = t;
+            if (most < ni) most *= 4;
+        }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        unsigned next = 0;
-        if ((e = cudaMemcpyAsync(&next, counters, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(&h[0], counters, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(&h[1], counters + 1 + waves, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+            return e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        nin = (int)std::min<unsigned>(next, (unsigned)ni);
-        int2 *t = qa;
-        qa = qb;
-        qb = t;
-    }
-    unsigned total = 0;
-    if ((e = cudaMemcpyAsync(&total, counters + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    *count_out = (int)std::min<unsigned>(total, (unsigned)cap);
+        done += waves;
+        if (h[1] > 0) {
+            if (done >= kMaxWaves) return cudaErrorInvalidValue;
+            waves = std::min(waves, kMaxWaves - done);
+            const unsigned left = h[1];
+            if ((e = cudaMemsetAsync(counters + 1, 0, (kWaves + 1) * sizeof(unsigned), s)) != cudaSuccess) return e;
+            if ((e = cudaMemcpyAsync(counters + 1, &left, sizeof left, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
+        }
+    } while (h[1] > 0);
+    *count_out = (int)std::min<unsigned>(h[0], (unsigned)cap);
     return cudaSuccess;
 }
 

@@ -273,6 +273,9 @@ size_t bvh4_node_capacity(int n);
 cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratch, uint32_t *status, int *count_out,
                        cudaStream_t s);
 // lad: [n] leaf area density of voxels (original order), or null (voxels then hold no leaves).
+// Primitive areas (voxels: leaf area), T 16-byte aligned; lad read for voxels.
+cudaError_t launch_prim_area(int n, const float *T, const uint32_t *type, const float *lad, double *area,
+                             cudaStream_t s);
 cudaError_t bvh_build(const float *T, const uint32_t *type, const float *lad, int n, BvhBuffers &b, cudaStream_t s);
 constexpr int kSortTile = 2048;
 

@@ -273,3 +273,38 @@ def test_voxel_lattices_vs_oracle(oracle_mod, form, periodic):
     assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
     assert rad.last_stats["rays"] == st["rays"]
     assert rad.ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [2, 3, 65, 1023, 1024, 1025, 1026, 5000, 140001])
+@pytest.mark.parametrize("spread", ["uniform", "line", "same"])
+def test_trees_of_all_sizes_hit_what_the_binary_tree_hits(gpu, n, spread):
+    """The clustered tree and its 4-wide nodes at the sizes around the last block's and the tiles' limits,
+    with equal areas everywhere ("same": all primitives in one place, refused beyond a depth as before):
+    a solve over it equals the one over the binary tree, whose nodes the host build pins."""
+    rng = np.random.default_rng(n)
+    c = rng.uniform(0.0, max(1.0, (n / 50.0) ** (1.0 / 3.0)), (n, 3))
+    if spread == "line":
+        c[:, 1:] = 0.0
+    if spread == "same":
+        c[:] = 0.5
+    nrm = np.tile([0.0, 0.0, 1.0], (n, 1)) if spread == "same" else scenes.uniform_sphere(rng, n)
+    T = scenes.frame_T(c, np.full(n, 0.1), np.full(n, 0.1), nrm, np.zeros(n) if spread == "same" else rng.uniform(0, 6, n))
+    gpu.update_geometry(T, np.zeros(n, np.uint32), np.ones(n, np.int8))
+    if spread == "same" and n > 1000:  # boxes that all tie chain up, deeper than a tree may be: refused
+        with pytest.raises(_hrt.HrtError, match="invalid argument"):
+            gpu.build_accel()
+        return
+    gpu.build_accel()
+    assert gpu.device_status() == 0
+    R = max(4, 4000 // n)
+    solve = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 1, "position": (2.0, 1.0, 9.0), "width": (0.4, 0.0)}],
+             "source_flux": np.array([[500.0]]), "rho": np.zeros((1, n, 1)), "tau": np.zeros((1, n, 1)),
+             "diffuse_flux": np.array([50.0]), "direct_rays": np.array([R]), "diffuse_rays": np.array([4]),
+             "depth": np.array([0]), "emission": np.array([0], np.uint8), "seed": 3}
+    wide = gpu.run_band(solve).astype(np.float64)
+    rays = gpu.last_stats()["rays"]
+    gpu.set_tuning(16 + 1)  # binary nodes for the diffuse pass
+    binary = gpu.run_band(solve).astype(np.float64)
+    gpu.set_tuning(1)
+    assert gpu.last_stats()["rays"] == rays and gpu.device_status() == 0
+    assert np.all(np.abs(wide - binary) <= 2.4e-7 * np.abs(binary))
