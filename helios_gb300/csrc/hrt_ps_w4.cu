@@ -21,8 +21,8 @@ unsigned w4_grid(const DiffuseParams &p, int resident, int block) {
     return (unsigned)g;
 }
 
-template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB = 1, bool MULTI = false, bool LIN = false,
-          bool COV = false, bool VG = false>
+template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB = 1, bool MULTI = false, bool COV = false,
+          bool VG = false>
 cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
     // resident blocks of one wave (SMs x blocks per SM); initialised once per instantiation,
     // thread-safe (the server launches from several threads)
@@ -31,7 +31,7 @@ cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
-                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV, VG>,
+                                                      k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, COV, VG>,
                                                       BLOCK, 0);
         return (sms < 1 ? 1 : sms) * (per_sm < 1 ? 1 : per_sm);
     }();
@@ -39,19 +39,18 @@ cudaError_t w4_launch(const DiffuseParams &p, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     DiffuseParams q = p;
     q.refill = refill_threshold(false, true, VG);
-    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, LIN, COV, VG><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
+    k_diffuse_w4<NB, RECORD, STATS, MINB, SD, BLOCK, KB, MULTI, COV, VG><<<w4_grid(q, resident, BLOCK), BLOCK, 0, s>>>(q);
     return cudaGetLastError();
 }
 
 // The tuner's shapes: threads per block x resident blocks per SM (all 64 registers a thread
-// but lean5, 48), shared stack entries per lane (a ring over local memory, or with LIN the
-// bottom entries) and the warp's ray-id batch.
+// but lean5, 48), shared stack entries per lane and the warp's ray-id batch.
 template <int NB, bool RECORD, bool STATS>
 cudaError_t w4_shape(const DiffuseParams &p, int variant, cudaStream_t s) {
     switch (variant) {
         case DV_W4S5: return w4_launch<NB, RECORD, STATS, 5, 8, 256>(p, s);
-        case DV_W4S4D16: return w4_launch<NB, RECORD, STATS, 4, 16, 256, 1, false, true>(p, s);
-        case DV_W4S4D32: return w4_launch<NB, RECORD, STATS, 4, 32, 256, 1, false, true>(p, s);
+        case DV_W4S4D16: return w4_launch<NB, RECORD, STATS, 4, 16, 256, 1>(p, s);
+        case DV_W4S4D32: return w4_launch<NB, RECORD, STATS, 4, 32, 256, 1>(p, s);
         case DV_W4B128: return w4_launch<NB, RECORD, STATS, 8, 8, 128>(p, s);
         case DV_W4B512: return w4_launch<NB, RECORD, STATS, 2, 8, 512>(p, s);
         case DV_W4K4: return w4_launch<NB, RECORD, STATS, 4, 8, 256, 4>(p, s);
@@ -87,22 +86,22 @@ cudaError_t launch_w4s_multi_record(const DiffuseParams &p, cudaStream_t s) {
     if (p.multi_total == 0) return cudaSuccess;
     DiffuseParams q = p;
     q.Bc = 1;
-    return w4_launch<1, true, false, 4, 8, 256, 1, true>(q, s);
+    return w4_launch<1, true, false, 4, 16, 256, 1, true>(q, s);
 }
 
 cudaError_t launch_w4s_covers(const DiffuseParams &p, cudaStream_t s) {
     if (!p.sc.nodes4 || p.sc.voxels || !p.sc.cover) return cudaErrorInvalidValue;
-    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true, true>(p, s);
-    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true, true>(p, s);
-    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true, true>(p, s);
+    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true>(p, s);
+    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true>(p, s);
+    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true>(p, s);
     return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_w4s_voxels(const DiffuseParams &p, cudaStream_t s) {
     if (!p.sc.vgrid) return cudaErrorInvalidValue;
-    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
-    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
-    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, true, false, true>(p, s);
+    if (p.Bc <= 1) return w4_launch<1, false, false, 4, 16, 256, 1, false, false, true>(p, s);
+    if (p.Bc <= 4) return w4_launch<4, false, false, 4, 16, 256, 1, false, false, true>(p, s);
+    if (p.Bc <= 16) return w4_launch<16, false, false, 4, 16, 256, 1, false, false, true>(p, s);
     return cudaErrorInvalidValue;
 }
 

@@ -17,19 +17,12 @@
 // when fewer than P.refill lanes remain; ray ids are split into face, primitive, ray and
 // stratum by multiplication (FastDiv).
 // The traversal stack keeps SD entries per lane in shared memory (indexed [entry][lane], so
-// the 32 lanes of a warp always hit 32 different banks) over a local overflow array, in one
-// of two layouts.  RingStack: the top SD entries in a ring, entries deeper than SD below the
-// top moved to local memory on push and brought back on pop.  LinStack (LIN): the bottom SD
-// entries in shared memory, deeper ones in local memory, and a visit whose pushes all stay
-// below SD writes them with no overflow test.  Local memory is touched only by rays whose
-// stack is deeper than SD.  On the 1 M-triangle orchard LinStack with SD = 16 is the faster
-// (180 against 184 ms per diffuse launch for the ring at SD = 16, 186-189 at SD = 8).
+// the 32 lanes of a warp always hit 32 different banks); they move to local memory all at once when
+// they run out (LaneStack).  Local memory is touched only by rays whose stack is deeper than SD.
 //
 // Hits equal those of trace_bvh / k_diffuse_ps: the same node and primitive tests, the same
 // tie rule (closest, then smaller original index); only the order of work differs.
 #pragma once
-#include <type_traits>
-
 #include "hrt_trace.cuh"
 #include "hrt_voxgrid.cuh"
 
@@ -37,38 +30,72 @@ namespace hrt {
 
 namespace {
 
+// The stack's top in shared memory ([entry][lane]) at a byte address per lane: entry 0 holds
+// kSentinel, so a pop needs no empty-stack test -- popping it ends the ray's traversal.  When a visit
+// could push past the SD entries, the lane's entries move to local memory and entry 0 becomes kMore;
+// a lane that pops kMore leaves the node loop and takes them back.  A pop is one load and a push one
+// predicated store, with no other test (before, every pop and push compared its place with SD and
+// computed its address): per solve 1 M-triangle orchard 850 -> 800 ms of diffuse launches, 20,001-patch
+// canopy 16.3 -> 14.7 ms, periodic stand of 63,458 primitives 36.6 -> 35.1 ms.
+constexpr int32_t kMore = kSentinel + 2;
 template <int SD, int BLOCK>
-struct RingStack {
-    static_assert((SD & (SD - 1)) == 0 && SD >= 2, "shared stack depth must be a power of two");
-    int32_t (*ring)[BLOCK];   // [SD][BLOCK] in shared memory
-    int tid;
-    int32_t spill[kStack4];   // local memory, entries below the top SD
-    __device__ __forceinline__ void push(int sp, int32_t v) {
-        const int slot = sp & (SD - 1);
-        if (sp >= SD) spill[sp - SD] = ring[slot][tid];
-        ring[slot][tid] = v;
+struct LaneStack {
+    uint32_t base, top;         // shared addresses: entry 0, and the next free entry
+    int32_t spill[kStack4 + 1]; // [0] entries held (while entry 0 is kMore), then the entries
+    static constexpr uint32_t kStep = 4u * BLOCK, kFull = (uint32_t)SD * kStep;
+    __device__ __forceinline__ static void put(uint32_t at, int32_t v) {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(v));
     }
-    // value of entry sp (the entry just below the old top), restoring the ring window
-    __device__ __forceinline__ int32_t pop(int sp) {
-        const int slot = sp & (SD - 1);
-        const int32_t v = ring[slot][tid];
-        if (sp >= SD) ring[slot][tid] = spill[sp - SD];
+    __device__ __forceinline__ static int32_t take(uint32_t at) {
+        int32_t v;
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(at));
         return v;
     }
-};
-
-// The bottom SD entries in shared memory ([entry][lane]), deeper ones in local memory (the
-// kernel keeps a sentinel in entry 0, so SD - 1 of them hold nodes).
-template <int SD, int BLOCK>
-struct LinStack {
-    int32_t (*ring)[BLOCK];   // [SD][BLOCK] in shared memory (not a ring: entry i at row i)
-    int tid;
-    int32_t spill[kStack4];
-    __device__ __forceinline__ void push(int sp, int32_t v) {
-        if (sp < SD) ring[sp][tid] = v;
-        else spill[sp - SD] = v;
+    __device__ __forceinline__ void init(const int32_t *entry0) {
+        base = (uint32_t)__cvta_generic_to_shared(entry0);
+        clear();
     }
-    __device__ __forceinline__ int32_t pop(int sp) { return sp < SD ? ring[sp][tid] : spill[sp - SD]; }
+    __device__ __forceinline__ void clear() {
+        put(base, kSentinel);
+        restart();
+    }
+    // For a new segment: one whose traversal ended has popped entry 0 with kSentinel in it (and nothing
+    // in local memory), so the entry is still there.
+    __device__ __forceinline__ void restart() { top = base + kStep; }
+    __device__ __forceinline__ void push_if(float tk, int32_t v) {
+        asm volatile(
+            "{\n .reg .pred p;\n setp.lt.f32 p, %1, 0f7F800000;\n @p st.shared.b32 [%0], %2;\n"
+            " @p add.u32 %0, %0, %3;\n}"
+            : "+r"(top)
+            : "f"(tk), "r"(v), "n"(kStep));
+    }
+    __device__ __forceinline__ int32_t pop() {
+        top -= kStep;
+        return take(top);
+    }
+    __device__ __forceinline__ bool room() const { return top + 3u * kStep <= base + kFull; }
+    // Entries above entry 0 to local memory; false: no room there.
+    __device__ __noinline__ bool spill_out() {
+        int held = take(base) == kMore ? spill[0] : 0;
+        const int n = (int)((top - base) / kStep) - 1;
+        if (held + n > kStack4) return false;
+        for (int i = 0; i < n; ++i) spill[1 + held + i] = take(base + kStep * (uint32_t)(1 + i));
+        spill[0] = held + n;
+        put(base, kMore);
+        top = base + kStep;
+        return true;
+    }
+    // The last entries held back to shared memory (kMore was popped); the top one.
+    __device__ __noinline__ int32_t spill_in() {
+        int held = spill[0];
+        const int n = held < SD - 4 ? held : SD - 4;
+        held -= n;
+        for (int i = 0; i < n; ++i) put(base + kStep * (uint32_t)(1 + i), spill[1 + held + i]);
+        spill[0] = held;
+        put(base, held > 0 ? kMore : kSentinel);
+        top = base + kStep * (uint32_t)(1 + n);
+        return pop();
+    }
 };
 
 // BLOCK: threads per block; MINB: resident blocks per SM the register allocation must allow.
@@ -78,12 +105,11 @@ struct LinStack {
 // MULTI (recording mode only): the launch traces several scenes -- P.slots[0..P.nslots) each
 // give a scene, a primitive chunk, ray counts, seed, pass and hit buffer, with consecutive
 // ranges of the launch's ray ids (id_begin) -- so one persistent launch covers the pass of
-// every scene of a multi-scene sweep.  LIN: the LinStack layout, else RingStack.  COV: translucent
-// covers of source 0 (P.sc.cover) are passed as if they were not there.  VG: the scene's voxels form a
+// every scene of a multi-scene sweep.  COV: translucent covers of source 0 (P.sc.cover) are passed as if they were not there.  VG: the scene's voxels form a
 // lattice (P.sc.vgrid): each ray segment marches it first and then walks the tree of the surfaces
 // (P.sc.nodes4s), bounded by the interception.
-template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB, bool MULTI = false, bool LIN = false,
-          bool COV = false, bool VG = false>
+template <int NB, bool RECORD, bool STATS, int MINB, int SD, int BLOCK, int KB, bool MULTI = false, bool COV = false,
+          bool VG = false>
 __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams P) {
     static_assert(!MULTI || (RECORD && !STATS), "multi-scene launches record hits only");
     __shared__ double s_sum[RECORD ? 1 : NB][BLOCK];            // running sums of the lane's origin
@@ -126,21 +152,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         __syncthreads();
     }
 
-    typename std::conditional<LIN, LinStack<SD, BLOCK>, RingStack<SD, BLOCK>>::type stk;
-    stk.ring = s_stack;
-    stk.tid = tid;
+    LaneStack<SD, BLOCK> stk;
+    stk.init(&s_stack[0][tid]);
     uint32_t nvis = 0, ntest = 0;  // statistics builds only
     uint32_t nrays = 0;
     bool live = false, exhausted = false;
     f3 ooi = mk(0.f, 0.f, 0.f), inv = ooi;
     float best = 1e38f;
     int32_t cur = kSentinel, leaf = 0, leaf2 = 0;  // current node, up to two postponed leaves
-    // LIN: entry 0 of the shared stack holds kSentinel for good and a ray starts with sp = 1, so a
-    // pop needs no empty-stack test: popping the sentinel ends the ray's traversal (168.7 against
-    // 173.2 ms per diffuse launch of the 1 M-triangle orchard)
-    constexpr int kSp0 = LIN ? 1 : 0;
-    if (kSp0) s_stack[0][tid] = kSentinel;
-    int sp = kSp0;
     uint32_t budget = 0;
     if (!RECORD) {
 #pragma unroll
@@ -159,7 +178,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         s_chunk[1][tid >> 5] = 0ull;
     }
     __syncwarp();
-#define POP() (kSp0 ? stk.pop(--sp) : (sp > 0 ? stk.pop(--sp) : kSentinel))
+    // ends the traversal of the lane's ray after an error
+    auto give_up = [&](uint32_t bit) {
+        raise(P.sc.status, bit);
+        cur = kSentinel;
+        leaf = 0;
+        leaf2 = 0;
+        stk.clear();
+    };
 
     for (;;) {
         // ---- refill lanes without a ray (warp-vote compaction of the fetch)
@@ -282,7 +308,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                         cur = VG ? kMarch : ((sc.n > 0) ? 0 : kSentinel);
                         leaf = 0;
                         leaf2 = 0;
-                        sp = kSp0;
+                        stk.restart();
                         budget = sc.visit_budget;
                         live = true;
                         if (MULTI) atomicAdd(&s_srays[lslot], 1ull);
@@ -337,16 +363,19 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         // ---- internal nodes; up to two leaves per lane are postponed to the primitive tests below
         const TraceScene &sc = SC;
         const uint32_t n4 = (uint32_t)(VG ? sc.n4s : sc.n4);
-        // cur is an internal node: 0 <= cur < kSentinel in one unsigned compare (leaves are
-        // negative; indices at or above n4 fail the bounds test inside)
-        while ((uint32_t)cur < (uint32_t)kSentinel) {
-            // both tests evaluated (no short-circuit branch), then the visit is counted
-            if (((uint32_t)cur >= n4) | (budget == 0u)) {
-                raise(sc.status, (uint32_t)cur >= n4 ? ERR_BOUNDS : ERR_BUDGET);
-                cur = kSentinel;
-                leaf = 0;
-                leaf2 = 0;
-                sp = kSp0;
+        if (cur >= (int32_t)n4 && cur != kSentinel && !(VG && cur == kMarch)) {
+            if (cur != kMore) {
+                give_up(ERR_BOUNDS);
+            } else if ((cur = stk.spill_in()) < 0) {  // no leaf is postponed here
+                leaf = cur;
+                cur = stk.pop();
+            }
+        }
+        // one unsigned compare says that cur is an internal node (leaves are negative, the special
+        // values and any index out of range above n4: the check above handles those)
+        while ((uint32_t)cur < n4) {
+            if (budget == 0u) {
+                give_up(ERR_BUDGET);
                 break;
             }
             --budget;
@@ -357,55 +386,25 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
             int32_t ck[4];  // every slot's reference: a child is hit when its tk < INFINITY
             node4_children<false>(q0, q1, q2, q3, node4_offset_ooi(q0, ooi, inv), inv, 1e-4f, best, tk, ck);
             node4_nearest(tk, ck);
-            if (LIN) {
-                // hit children other than the nearest pushed (predicated: a visit that hits
-                // nothing pushes nothing), then the nearest entered or, with no hit, the top of
-                // the stack taken -- no branch between the two cases
-                const bool any = tk[0] < INFINITY;
-                if (sp + 3 <= SD) {  // the whole push in shared memory
-#pragma unroll
-                    for (int k = 3; k >= 1; --k)
-                        if (tk[k] < INFINITY) s_stack[sp++][tid] = ck[k];
-                } else {
-                    if (any && sp + 3 > SD + kStack4) {
-                        raise(sc.status, ERR_STACK);
-                        cur = kSentinel;
-                        leaf = 0;
-                        leaf2 = 0;
-                        sp = kSp0;
-                        break;
-                    }
-#pragma unroll
-                    for (int k = 3; k >= 1; --k)
-                        if (tk[k] < INFINITY) stk.push(sp++, ck[k]);
-                }
-                int32_t nxt = ck[0];
-                if (!any) nxt = POP();
-                cur = nxt;
-            } else if (!(tk[0] < INFINITY)) {
-                cur = POP();
-            } else {
-                if (sp + 3 > SD + kStack4) {
-                    raise(sc.status, ERR_STACK);
-                    cur = kSentinel;
-                    leaf = 0;
-                    leaf2 = 0;
-                    sp = kSp0;
-                    break;
-                }
-#pragma unroll
-                for (int k = 3; k >= 1; --k)
-                    if (tk[k] < INFINITY) stk.push(sp++, ck[k]);
-                cur = ck[0];
+            // hit children other than the nearest pushed (predicated: a visit that hits nothing pushes
+            // nothing), then the nearest entered or, with no hit, the top of the stack taken
+            if (__builtin_expect(!stk.room(), 0) && !stk.spill_out()) {
+                give_up(ERR_STACK);
+                break;
             }
+            stk.push_if(tk[3], ck[3]);
+            stk.push_if(tk[2], ck[2]);
+            stk.push_if(tk[1], ck[1]);
+            cur = ck[0];
+            if (!(tk[0] < INFINITY)) cur = stk.pop();
             // a leaf is postponed while one of the two slots is free; a lane with both full stops
             // at its third leaf.  The warp leaves the loop only when fewer than P.refill lanes
             // remain in it (no vote on the leaves): 162.7 against 167.4 ms per diffuse launch of
             // the 1 M-triangle orchard with one slot and a leave-when-all-have-a-leaf vote
             if (cur < 0 && leaf2 == 0) {
-                if (leaf == 0) leaf = cur;
-                else leaf2 = cur;
-                cur = POP();
+                leaf2 = leaf;
+                leaf = cur;
+                cur = stk.pop();
             }
             if (__popc(__activemask()) < P.refill) break;
         }
@@ -445,7 +444,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                 leaf2 = 0;
                 if (leaf == 0 && cur < 0) {
                     leaf = cur;
-                    cur = POP();
+                    cur = stk.pop();
                 }
             }
             s_lane[L_HIT][tid] = bcode;
@@ -481,7 +480,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
                     s_lane[L_AXES][tid] = (ax & 0xFFu) | ((wraps + 1u) << 8);
                     if (VG) s_lane[L_CELL][tid] = kMarchNew;
                     cur = VG ? kMarch : 0;
-                    sp = kSp0;
+                    stk.restart();
                     budget = sc.visit_budget;
                     continue;
                 }
@@ -540,7 +539,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         add_rays(P.sc, nrays);
     }
     if (STATS) count_visits(P.sc, nvis, ntest);
-#undef POP
 #undef SC
 }
 
