@@ -703,16 +703,16 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
         return HRT_OK;
     }
     if (ctx->measure & 1) return HRT_OK;  // statistics launches count on a tuned choice, never time one
+    // The candidates are the shapes that have been fastest or within 3 % of it on some scene timed since
+    // the stack went to shared memory; the others (binary and generic traces, one ray per thread, batched
+    // fetches) lost by 10-250 % everywhere and only cost a shape's first pass time: 38 of the 92 ms of a
+    // periodic stand's first solve.  hrt_set_tuning still forces any of them.
     std::vector<int> cand;
     const bool w4 = P0.sc.nodes4 != nullptr;
-    if (record)
-        cand = w4 ? std::vector<int>{DV_W4, DV_W43, DV_W4S4, DV_W4S5, DV_W4S4D16, DV_W4S4D32, DV_W4B128, DV_W4B512,
-                                     DV_W4K4, DV_W4K16, DV_PS3, DV_PS4}
-                  : std::vector<int>{DV_PS3, DV_PS4};
-    else if (P0.sc.voxels) cand = w4 ? std::vector<int>{DV_W4, DV_PS4, DV_SIMPLE} : std::vector<int>{DV_PS4, DV_SIMPLE};
-    else cand = w4 ? std::vector<int>{DV_W4, DV_W43, DV_W4S4, DV_W4S5, DV_W4S4D16, DV_W4S4D32, DV_W4B128, DV_W4B512,
-                                      DV_W4K4, DV_W4K16, DV_PS4, DV_PS3, DV_SIMPLE}
-                   : std::vector<int>{DV_PS4, DV_PS3, DV_SIMPLE};
+    if (!record && P0.sc.voxels) cand = w4 ? std::vector<int>{DV_W4, DV_PS4} : std::vector<int>{DV_PS4, DV_SIMPLE};
+    else if (w4) cand = {DV_W4S4D16, DV_W4S4D32, DV_W4S4};
+    else if (record) cand = {DV_PS3, DV_PS4};
+    else cand = {DV_PS4, DV_PS3, DV_SIMPLE};
     DiffuseParams P = P0;
     P.count = std::min(P0.count, std::max(P0.count / 32u, 4096u));
     // the sample is one launch: keep it within the per-launch ray limit
