@@ -182,7 +182,7 @@ struct hrt_context {
     std::vector<float> h_src_flux;
     // radiation buffers
     int Bl = 0;
-    DevBuf rin, stop, sbot, otop, obot, ftop, fbot, Gd, Gt, Gb, flags, sky, fin, status, counter, emis, emis_eps, emis_T,
+    DevBuf rin, stop, sbot, otop, obot, Gd, Gt, Gb, flags, sky, fin, status, counter, emis, emis_eps, emis_T,
         fetch;
     size_t emis_eps_count = 0, emis_T_count = 0;
     // grids across the collimated sources of a direct pass, and what they need of the geometry
@@ -192,6 +192,7 @@ struct hrt_context {
     std::vector<int> h_src_type;
     DevBuf io_a, io_b, io_c;  // staging for inspection calls
     uint64_t last_rays = 0, last_kernels = 0, last_iters = 0;
+    unsigned long long *pinned = nullptr;  // [0] ray count, [1] device error word
     DevBuf resid;  // scattering residual: block partials and the per-band result
     // measurement: bit 0 counts traversal work, bit 1 times trace launches
     int measure = 0;
@@ -377,10 +378,7 @@ int check_built(hrt_context *ctx) {
     return HRT_OK;
 }
 
-int sync_and_status(hrt_context *ctx) {
-    uint32_t st = 0;
-    CU(cudaMemcpyAsync(&st, ctx->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
+int status_result(hrt_context *ctx, uint32_t st) {
     if (st) {
         CU(cudaMemsetAsync(ctx->status.p, 0, sizeof(uint32_t), ctx->stream));
         char buf[200];
@@ -393,6 +391,17 @@ int sync_and_status(hrt_context *ctx) {
     return HRT_OK;
 }
 
+// Waits for the stream and turns the device error word into a result.  The word (and a solve's ray
+// count) come through pinned memory: a copy to pageable memory waits for the stream by itself, and
+// each such wait cost a small solve some 10 us.
+int sync_and_status(hrt_context *ctx) {
+    CU(cudaMemcpyAsync(ctx->pinned + 1, ctx->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    CU(cudaStreamSynchronize(ctx->stream));
+    uint32_t st;
+    std::memcpy(&st, ctx->pinned + 1, sizeof st);
+    return status_result(ctx, st);
+}
+
 // Radiation buffers for n x Bl values.
 int ensure_buffers(hrt_context *ctx, int Bl) {
     size_t m = (size_t)std::max(ctx->n, 1) * (size_t)std::max(Bl, 1);
@@ -401,8 +410,6 @@ int ensure_buffers(hrt_context *ctx, int Bl) {
     CU(ctx->sbot.ensure(ctx->stream, m * sizeof(double)));
     CU(ctx->otop.ensure(ctx->stream, m * sizeof(float)));
     CU(ctx->obot.ensure(ctx->stream, m * sizeof(float)));
-    CU(ctx->ftop.ensure(ctx->stream, m * sizeof(double)));
-    CU(ctx->fbot.ensure(ctx->stream, m * sizeof(double)));
     CU(ctx->Gt.ensure(ctx->stream, m * sizeof(double)));
     CU(ctx->Gb.ensure(ctx->stream, m * sizeof(double)));
     CU(ctx->fin.ensure(ctx->stream, m * sizeof(float)));
@@ -435,9 +442,12 @@ int upload_sky(hrt_context *ctx, int Bl, const float *flux, const float *K, cons
 }
 
 int upload_flags(hrt_context *ctx, int Bg, const uint8_t *flags) {
-    ctx->h_flags.assign(flags, flags + Bg);
+    if (ctx->flags.p && ctx->h_flags.size() == (size_t)Bg && std::equal(flags, flags + Bg, ctx->h_flags.begin()))
+        return HRT_OK;  // on the device already
+    ctx->h_flags.clear();
     CU(ctx->flags.ensure(ctx->stream, (size_t)std::max(Bg, 1)));
     CU(cudaMemcpyAsync(ctx->flags.p, flags, (size_t)Bg, cudaMemcpyHostToDevice, ctx->stream));
+    ctx->h_flags.assign(flags, flags + Bg);
     return HRT_OK;
 }
 
@@ -765,7 +775,7 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
 }
 
 int diffuse_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp, uint32_t seed, uint32_t pass, int faces,
-                 int Bg, int Bc, int Bl, const SkyParams &sky) {
+                 int Bg, int Bc, int Bl, const SkyParams &sky, bool zeroed = false) {
     int dimx, dimy;
     strata(rpp, &dimx, &dimy);
     if (dimx * dimy == 0 || count == 0 || Bc == 0) return HRT_OK;
@@ -776,8 +786,10 @@ int diffuse_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp
     const uint32_t per = chunk_prims(ctx, (uint64_t)dimx * (uint64_t)dimy * (uint64_t)nfaces);
     if (per == 0) return HRT_EUNSUPPORTED;
     size_t m = (size_t)ctx->n * Bl;
-    CU(cudaMemsetAsync(ctx->Gt.p, 0, m * sizeof(double), ctx->stream));
-    CU(cudaMemsetAsync(ctx->Gb.p, 0, m * sizeof(double), ctx->stream));
+    if (!zeroed) {
+        CU(cudaMemsetAsync(ctx->Gt.p, 0, m * sizeof(double), ctx->stream));
+        CU(cudaMemsetAsync(ctx->Gb.p, 0, m * sizeof(double), ctx->stream));
+    }
     DiffuseParams P;
     P.sc = scene_of(ctx);
     P.dimx = dimx;
@@ -985,6 +997,78 @@ int count_flags(int Bg, const uint8_t *f) {
     return c;
 }
 
+// Uploads of materials, sources and source fluxes.  wait: return when the caller's arrays may change
+// (a solve waits once, at its end).
+int set_materials(hrt_context *ctx, int32_t nsources, int32_t nprims, int32_t nbands_global, const float *rho,
+                         const float *tau, bool wait) {
+    if (!ctx || nsources < 0 || nprims < 0 || nbands_global < 0) return HRT_EINVAL;
+    size_t m = (size_t)nsources * nprims * nbands_global;
+    if (m && (!rho || !tau)) return fail(ctx, HRT_EINVAL, "null material array");
+    CU(cudaSetDevice(ctx->device));
+    CU(ctx->rho.ensure(ctx->stream, std::max<size_t>(m, 1) * sizeof(float)));
+    CU(ctx->tau.ensure(ctx->stream, std::max<size_t>(m, 1) * sizeof(float)));
+    std::vector<float> vr, vt;
+    if (m && !ctx->h_voxels.empty() && nprims == ctx->n) {
+        // A voxel's leaves scatter rho + tau into one isotropic field: half of it is routed
+        // to each face, so both faces emit the same radiance.
+        vr.assign(rho, rho + m);
+        vt.assign(tau, tau + m);
+        for (int32_t src = 0; src < nsources; ++src)
+            for (uint32_t p : ctx->h_voxels)
+                for (int32_t b = 0; b < nbands_global; ++b) {
+                    size_t i = ((size_t)src * nprims + p) * nbands_global + b;
+                    float h = 0.5f * (vr[i] + vt[i]);
+                    vr[i] = h;
+                    vt[i] = h;
+                }
+        rho = vr.data();
+        tau = vt.data();
+    }
+    if (m) {
+        CU(cudaMemcpyAsync(ctx->rho.p, rho, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+        CU(cudaMemcpyAsync(ctx->tau.p, tau, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    }
+    ctx->mS = nsources;
+    ctx->mN = nprims;
+    ctx->mB = nbands_global;
+    if (wait) CU(cudaStreamSynchronize(ctx->stream));
+    return HRT_OK;
+}
+
+int set_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sources, bool wait) {
+    if (!ctx || nsources < 0 || (nsources > 0 && !sources)) return HRT_EINVAL;
+    if (nsources > 256) return fail(ctx, HRT_EINVAL, "A maximum of 256 radiation sources are allowed.");
+    CU(cudaSetDevice(ctx->device));
+    std::vector<SourceDev> h((size_t)std::max(nsources, 1));
+    ctx->h_src_type.assign((size_t)nsources, 0);
+    for (int k = 0; k < nsources; ++k) {
+        if (sources[k].type > 4) return fail(ctx, HRT_EINVAL, "unknown source type");
+        SourceDev &s = h[k];
+        s.type = (int)sources[k].type;
+        ctx->h_src_type[k] = s.type;
+        for (int i = 0; i < 3; ++i) s.pos[i] = sources[k].position[i];
+        s.w0 = sources[k].width[0];
+        s.w1 = sources[k].width[1];
+        rotation3(sources[k].rotation, s.R);
+    }
+    CU(ctx->src.ensure(ctx->stream, h.size() * sizeof(SourceDev)));
+    CU(cudaMemcpyAsync(ctx->src.p, h.data(), h.size() * sizeof(SourceDev), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->S = nsources;
+    if (wait) CU(cudaStreamSynchronize(ctx->stream));
+    return HRT_OK;
+}
+
+int set_source_fluxes(hrt_context *ctx, const float *fluxes, size_t count, bool wait) {
+    if (!ctx || (count && !fluxes)) return HRT_EINVAL;
+    CU(cudaSetDevice(ctx->device));
+    CU(ctx->src_flux.ensure(ctx->stream, std::max<size_t>(count, 1) * sizeof(float)));
+    if (count) CU(cudaMemcpyAsync(ctx->src_flux.p, fluxes, count * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->src_flux_count = count;
+    ctx->h_src_flux.assign(fluxes, fluxes + count);
+    if (wait) CU(cudaStreamSynchronize(ctx->stream));
+    return HRT_OK;
+}
+
 }  // namespace
 
 // ============================================================== C ABI ===
@@ -1009,7 +1093,13 @@ int hrt_create(hrt_context **out, int device) {
     }
     ctx->stream = ctx->own;
     keep_pool(device);
+    if (cudaHostAlloc((void **)&ctx->pinned, 2 * sizeof(unsigned long long), cudaHostAllocPortable) != cudaSuccess) {
+        cudaStreamDestroy(ctx->own);
+        delete ctx;
+        return HRT_ENOMEM;
+    }
     if (ctx->status.ensure(ctx->stream, sizeof(uint32_t)) != cudaSuccess || ctx->counter.ensure(ctx->stream, sizeof(unsigned long long)) != cudaSuccess) {
+        cudaFreeHost(ctx->pinned);
         cudaStreamDestroy(ctx->own);
         delete ctx;
         return HRT_ENOMEM;
@@ -1017,6 +1107,7 @@ int hrt_create(hrt_context **out, int device) {
     cudaMemsetAsync(ctx->status.p, 0, sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(ctx->counter.p, 0, sizeof(unsigned long long), ctx->stream);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaFreeHost(ctx->pinned);
         cudaStreamDestroy(ctx->own);
         delete ctx;
         return HRT_ECUDA;
@@ -1034,9 +1125,11 @@ int hrt_destroy(hrt_context *ctx) {
     if (ctx->mw_exec) cudaGraphExecDestroy(ctx->mw_exec);
     collect_timings(ctx);
     g_release_stream = s;  // buffers are released on the context's stream
+    unsigned long long *pinned = ctx->pinned;
     delete ctx;
     g_release_stream = nullptr;
     cudaStreamSynchronize(s);
+    cudaFreeHost(pinned);
     if (own) cudaStreamDestroy(own);
     return HRT_OK;
 }
@@ -1248,38 +1341,7 @@ int hrt_build_accel(hrt_context *ctx) {
 
 int hrt_update_materials(hrt_context *ctx, int32_t nsources, int32_t nprims, int32_t nbands_global, const float *rho,
                          const float *tau) {
-    if (!ctx || nsources < 0 || nprims < 0 || nbands_global < 0) return HRT_EINVAL;
-    size_t m = (size_t)nsources * nprims * nbands_global;
-    if (m && (!rho || !tau)) return fail(ctx, HRT_EINVAL, "null material array");
-    CU(cudaSetDevice(ctx->device));
-    CU(ctx->rho.ensure(ctx->stream, std::max<size_t>(m, 1) * sizeof(float)));
-    CU(ctx->tau.ensure(ctx->stream, std::max<size_t>(m, 1) * sizeof(float)));
-    std::vector<float> vr, vt;
-    if (m && !ctx->h_voxels.empty() && nprims == ctx->n) {
-        // A voxel's leaves scatter rho + tau into one isotropic field: half of it is routed
-        // to each face, so both faces emit the same radiance.
-        vr.assign(rho, rho + m);
-        vt.assign(tau, tau + m);
-        for (int32_t src = 0; src < nsources; ++src)
-            for (uint32_t p : ctx->h_voxels)
-                for (int32_t b = 0; b < nbands_global; ++b) {
-                    size_t i = ((size_t)src * nprims + p) * nbands_global + b;
-                    float h = 0.5f * (vr[i] + vt[i]);
-                    vr[i] = h;
-                    vt[i] = h;
-                }
-        rho = vr.data();
-        tau = vt.data();
-    }
-    if (m) {
-        CU(cudaMemcpyAsync(ctx->rho.p, rho, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-        CU(cudaMemcpyAsync(ctx->tau.p, tau, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-    }
-    ctx->mS = nsources;
-    ctx->mN = nprims;
-    ctx->mB = nbands_global;
-    CU(cudaStreamSynchronize(ctx->stream));
-    return HRT_OK;
+    return set_materials(ctx, nsources, nprims, nbands_global, rho, tau, true);
 }
 
 int hrt_update_glass(hrt_context *ctx, int32_t nsources, int32_t nprims, int32_t nbands_global, const int8_t *is_glass,
@@ -1315,37 +1377,11 @@ int hrt_update_glass(hrt_context *ctx, int32_t nsources, int32_t nprims, int32_t
 }
 
 int hrt_update_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sources) {
-    if (!ctx || nsources < 0 || (nsources > 0 && !sources)) return HRT_EINVAL;
-    if (nsources > 256) return fail(ctx, HRT_EINVAL, "A maximum of 256 radiation sources are allowed.");
-    CU(cudaSetDevice(ctx->device));
-    std::vector<SourceDev> h((size_t)std::max(nsources, 1));
-    ctx->h_src_type.assign((size_t)nsources, 0);
-    for (int k = 0; k < nsources; ++k) {
-        if (sources[k].type > 4) return fail(ctx, HRT_EINVAL, "unknown source type");
-        SourceDev &s = h[k];
-        s.type = (int)sources[k].type;
-        ctx->h_src_type[k] = s.type;
-        for (int i = 0; i < 3; ++i) s.pos[i] = sources[k].position[i];
-        s.w0 = sources[k].width[0];
-        s.w1 = sources[k].width[1];
-        rotation3(sources[k].rotation, s.R);
-    }
-    CU(ctx->src.ensure(ctx->stream, h.size() * sizeof(SourceDev)));
-    CU(cudaMemcpyAsync(ctx->src.p, h.data(), h.size() * sizeof(SourceDev), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->S = nsources;
-    CU(cudaStreamSynchronize(ctx->stream));
-    return HRT_OK;
+    return set_sources(ctx, nsources, sources, true);
 }
 
 int hrt_upload_source_fluxes(hrt_context *ctx, const float *fluxes, size_t count) {
-    if (!ctx || (count && !fluxes)) return HRT_EINVAL;
-    CU(cudaSetDevice(ctx->device));
-    CU(ctx->src_flux.ensure(ctx->stream, std::max<size_t>(count, 1) * sizeof(float)));
-    if (count) CU(cudaMemcpyAsync(ctx->src_flux.p, fluxes, count * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->src_flux_count = count;
-    ctx->h_src_flux.assign(fluxes, fluxes + count);
-    CU(cudaStreamSynchronize(ctx->stream));
-    return HRT_OK;
+    return set_source_fluxes(ctx, fluxes, count, true);
 }
 
 int hrt_zero_radiation_buffers(hrt_context *ctx, size_t launch_band_count) {
@@ -1657,8 +1693,10 @@ int hrt_query_memory(hrt_context *ctx, size_t *free_bytes, size_t *total_bytes) 
     return HRT_OK;
 }
 
+}  // extern "C"
+
 // ------------------------------------------------------------ runBand ----
-int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
+static int run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
     if (!ctx || !s) return HRT_EINVAL;
     int r = check_built(ctx);
     if (r) return r;
@@ -1676,13 +1714,13 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
     // materials / sources: NULL keeps what is resident on the device
     if (s->rho || s->tau) {
         if (!s->rho || !s->tau) return fail(ctx, HRT_EINVAL, "rho and tau must be given together");
-        if ((r = hrt_update_materials(ctx, std::max(s->nsources, 1), n, Bg, s->rho, s->tau))) return r;
+        if ((r = set_materials(ctx, std::max(s->nsources, 1), n, Bg, s->rho, s->tau, false))) return r;
     }
     if (s->sources) {
-        if ((r = hrt_update_sources(ctx, s->nsources, s->sources))) return r;
+        if ((r = set_sources(ctx, s->nsources, s->sources, false))) return r;
     }
     if (s->source_flux && s->nsources > 0) {
-        if ((r = hrt_upload_source_fluxes(ctx, s->source_flux, (size_t)s->nsources * Bl))) return r;
+        if ((r = set_source_fluxes(ctx, s->source_flux, (size_t)s->nsources * Bl, false))) return r;
     }
     if (ctx->mN != n || ctx->mB < Bg || ctx->mS < 1) return fail(ctx, HRT_EINVAL, "materials do not match the scene");
     const int S = ctx->S;
@@ -1704,14 +1742,10 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
     ctx->Bl = Bl;
     const size_t m = (size_t)n * Bl;
     cudaStream_t st = ctx->stream;
-    CU(cudaMemsetAsync(ctx->rin.p, 0, m * sizeof(double), st));
-    CU(cudaMemsetAsync(ctx->stop.p, 0, m * sizeof(double), st));
-    CU(cudaMemsetAsync(ctx->sbot.p, 0, m * sizeof(double), st));
-    CU(cudaMemsetAsync(ctx->ftop.p, 0, m * sizeof(double), st));
-    CU(cudaMemsetAsync(ctx->fbot.p, 0, m * sizeof(double), st));
-    CU(cudaMemsetAsync(ctx->otop.p, 0, m * sizeof(float), st));
-    CU(cudaMemsetAsync(ctx->obot.p, 0, m * sizeof(float), st));
-    CU(cudaMemsetAsync(ctx->counter.p, 0, sizeof(unsigned long long), st));
+    CU(launch_begin_solve(m, ctx->rin.as<double>(), ctx->stop.as<double>(), ctx->sbot.as<double>(),
+                          ctx->otop.as<float>(), ctx->obot.as<float>(), ctx->Gt.as<double>(), ctx->Gb.as<double>(),
+                          ctx->counter.as<unsigned long long>(), st));
+    ctx->last_kernels += 1;
     std::vector<uint8_t> flags(s->band_launch, s->band_launch + Bg);
     if ((r = upload_flags(ctx, Bg, flags.data()))) return r;
     // Camera view of the primitives: the scatter of every pass plus emission, accumulated
@@ -1756,14 +1790,16 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
         if ((r = direct_pass(ctx, 0, (uint32_t)n, (uint32_t)dirN, s->seed, 0u, Bg, Bl, Bl))) return r;
     }
     // ---- scattered direct energy becomes the outgoing flux (one-sided prims fold top+bottom)
-    if (scattering && rundirect) {
-        if ((r = cam_add_scatter())) return r;
-        CU(launch_fold_onesided(n, Bl, ctx->twosided.as<int8_t>(), ctx->stop.as<double>(), ctx->sbot.as<double>(),
-                                ctx->ftop.as<double>(), ctx->fbot.as<double>(), st));
-        CU(cudaMemsetAsync(ctx->stop.p, 0, m * sizeof(double), st));
-        CU(cudaMemsetAsync(ctx->sbot.p, 0, m * sizeof(double), st));
+    const bool fold = scattering && rundirect;
+    if (fold && (r = cam_add_scatter())) return r;
+    auto outgoing = [&](bool em) -> int {
+        CU(launch_outgoing(n, Bl, ctx->twosided.as<int8_t>(), fold ? 1 : 0, ctx->stop.as<double>(),
+                           ctx->sbot.as<double>(), em ? ctx->emis.as<uint8_t>() : nullptr,
+                           (const int32_t *)(ctx->emis.as<char>() + 64), ctx->emis_eps.as<float>(),
+                           ctx->emis_T.as<float>(), ctx->otop.as<float>(), ctx->obot.as<float>(), st));
         ctx->last_kernels += 1;
-    }
+        return HRT_OK;
+    };
     uint32_t rpp_d = 0;
     {
         double c = std::ceil(std::sqrt((double)difN));
@@ -1774,37 +1810,19 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
                         s->sky_radiance_params, &sky)))
         return r;
     if (emission || diffuse) {
-        if (emission) {
+        if (emission && cams) {
             CU(launch_emission(n, Bl, ctx->emis.as<uint8_t>(), (const int32_t *)(ctx->emis.as<char>() + 64),
                                ctx->emis_eps.as<float>(), ctx->emis_T.as<float>(), ctx->twosided.as<int8_t>(),
-                               ctx->ftop.as<double>(), ctx->fbot.as<double>(), st));
+                               ctx->ctop.as<double>(), ctx->cbot.as<double>(), st));
             ctx->last_kernels += 1;
-            if (cams) {
-                CU(launch_emission(n, Bl, ctx->emis.as<uint8_t>(), (const int32_t *)(ctx->emis.as<char>() + 64),
-                                   ctx->emis_eps.as<float>(), ctx->emis_T.as<float>(), ctx->twosided.as<int8_t>(),
-                                   ctx->ctop.as<double>(), ctx->cbot.as<double>(), st));
-                ctx->last_kernels += 1;
-            }
         }
-        CU(launch_to_float(ctx->ftop.as<double>(), ctx->otop.as<float>(), m, st));
-        CU(launch_to_float(ctx->fbot.as<double>(), ctx->obot.as<float>(), m, st));
-        ctx->last_kernels += 2;
-        if ((r = diffuse_pass(ctx, 0, (uint32_t)n, rpp_d, s->seed, 1u, 3, Bg, Bl, Bl, sky))) return r;
+        if ((r = outgoing(emission))) return r;
+        if ((r = diffuse_pass(ctx, 0, (uint32_t)n, rpp_d, s->seed, 1u, 3, Bg, Bl, Bl, sky, true))) return r;
         if ((r = cam_add_scatter())) return r;
-    } else if (scattering && rundirect) {
-        CU(launch_to_float(ctx->ftop.as<double>(), ctx->otop.as<float>(), m, st));
-        CU(launch_to_float(ctx->fbot.as<double>(), ctx->obot.as<float>(), m, st));
-        ctx->last_kernels += 2;
-    }
-    if (scattering && (emission || diffuse) && !rundirect) {
-        CU(launch_to_float(ctx->stop.as<double>(), ctx->otop.as<float>(), m, st));
-        CU(launch_to_float(ctx->sbot.as<double>(), ctx->obot.as<float>(), m, st));
-        CU(cudaMemsetAsync(ctx->stop.p, 0, m * sizeof(double), st));
-        CU(cudaMemsetAsync(ctx->sbot.p, 0, m * sizeof(double), st));
-        ctx->last_kernels += 2;
+    } else if (fold) {
+        if ((r = outgoing(false))) return r;
     }
     if (scattering && (emission || diffuse || rundirect)) {
-        std::vector<float> zero((size_t)Bl, 0.f);
         SkyParams sky0;
         {
             // zero diffuse flux for the scattering iterations (RadiationModel.cpp:4237-4240)
@@ -1823,15 +1841,14 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
                 if (it + 1 > s->scattering_depth[b] || conv[bg]) sflags[bg] = 0;
             }
             if ((r = upload_flags(ctx, Bg, sflags.data()))) return r;
-            if (it > 0 || (emission && rundirect)) {
-                CU(launch_to_float(ctx->stop.as<double>(), ctx->otop.as<float>(), m, st));
-                CU(launch_to_float(ctx->sbot.as<double>(), ctx->obot.as<float>(), m, st));
-                ctx->last_kernels += 2;
-            }
-            CU(cudaMemsetAsync(ctx->stop.p, 0, m * sizeof(double), st));
-            CU(cudaMemsetAsync(ctx->sbot.p, 0, m * sizeof(double), st));
+            // the first iteration gathers what the primary pass left outgoing, unless emission and direct
+            // energy were both in it, or there was no direct pass (then its scatter goes out)
+            const bool copy = it > 0 || (emission && rundirect) || !rundirect;
+            CU(launch_next_pass(m, copy ? 1 : 0, ctx->stop.as<double>(), ctx->sbot.as<double>(), ctx->otop.as<float>(),
+                                ctx->obot.as<float>(), ctx->Gt.as<double>(), ctx->Gb.as<double>(), st));
+            ctx->last_kernels += 1;
             int Bc = count_flags(Bg, sflags.data());
-            if ((r = diffuse_pass(ctx, 0, (uint32_t)n, rpp_d, s->seed, 2u + (uint32_t)it, 3, Bg, Bc, Bl, sky0))) return r;
+            if ((r = diffuse_pass(ctx, 0, (uint32_t)n, rpp_d, s->seed, 2u + (uint32_t)it, 3, Bg, Bc, Bl, sky0, true))) return r;
             if ((r = cam_add_scatter())) return r;
             iters = it + 1;
             if (residual) {
@@ -1858,7 +1875,6 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
     }
     CU(launch_final_flux(m, ctx->rin.as<double>(), ctx->stop.as<double>(), ctx->sbot.as<double>(), ctx->fin.as<float>(), st));
     ctx->last_kernels += 1;
-    if (flux_out) CU(cudaMemcpyAsync(flux_out, ctx->fin.p, m * sizeof(float), cudaMemcpyDeviceToHost, st));
     // ---- cameras (RadiationModel.cpp:4358-4616), rendered from the accumulated camera view
     if (cams) {
         const bool render = scattering && (emission || diffuse || rundirect);
@@ -1896,16 +1912,26 @@ int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
             if (c.depths) CU(cudaMemcpyAsync(c.depths, ctx->cam_dep.p, npx * sizeof(float), cudaMemcpyDeviceToHost, st));
         }
     }
-    unsigned long long rays = 0;
-    CU(cudaMemcpyAsync(&rays, ctx->counter.p, sizeof(rays), cudaMemcpyDeviceToHost, st));
-    r = sync_and_status(ctx);
-    ctx->last_rays = rays;
+    CU(cudaMemcpyAsync(ctx->pinned, ctx->counter.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    CU(cudaMemcpyAsync(ctx->pinned + 1, ctx->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    // the fluxes last: a copy to pageable memory waits for all before it
+    if (flux_out) CU(cudaMemcpyAsync(flux_out, ctx->fin.p, m * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CU(cudaStreamSynchronize(st));
+    uint32_t word;
+    std::memcpy(&word, ctx->pinned + 1, sizeof word);
+    ctx->last_rays = ctx->pinned[0];
     ctx->last_iters = (uint64_t)iters;
+    return status_result(ctx, word);
+}
+
+extern "C" int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
+    const int r = run_band(ctx, s, flux_out);
+    // a call that failed on its way may have uploads from the caller's arrays in flight
+    if (r != HRT_OK && ctx) cudaStreamSynchronize(ctx->stream);
     return r;
 }
 
 // ------------------------------------------------------------ batched sweep --
-}  // extern "C"
 
 namespace {
 

@@ -386,8 +386,13 @@ cudaError_t launch_epilogue_diffuse(const EpilogueParams &p, cudaStream_t s);
 
 // Buffer bookkeeping (OptiX8Backend.cpp:1168-1250 semantics).
 cudaError_t launch_to_float(const double *a, float *out, size_t n, cudaStream_t s);
-cudaError_t launch_fold_onesided(int n, int Bl, const int8_t *twosided, const double *stop, const double *sbot,
-                                 double *ftop, double *fbot, cudaStream_t s);
+cudaError_t launch_begin_solve(size_t m, double *rin, double *stop, double *sbot, float *otop, float *obot, double *Gt,
+                               double *Gb, unsigned long long *counter, cudaStream_t s);
+cudaError_t launch_outgoing(int n, int Bl, const int8_t *twosided, int fold, double *stop, double *sbot,
+                            const uint8_t *emission, const int32_t *depth, const float *eps, const float *temperature,
+                            float *otop, float *obot, cudaStream_t s);
+cudaError_t launch_next_pass(size_t m, int copy, double *stop, double *sbot, float *otop, float *obot, double *Gt,
+                             double *Gb, cudaStream_t s);
 cudaError_t launch_emission(int n, int Bl, const uint8_t *emission, const int32_t *depth, const float *eps,
                             const float *temperature, const int8_t *twosided, double *ftop, double *fbot,
                             cudaStream_t s);

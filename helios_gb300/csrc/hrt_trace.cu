@@ -492,20 +492,65 @@ __global__ void k_to_float(const double *__restrict__ a, float *__restrict__ out
     if (i < n) out[i] = (float)a[i];
 }
 
-__global__ void k_fold(int n, int Bl, const int8_t *__restrict__ ts, const double *__restrict__ stop,
-                       const double *__restrict__ sbot, double *__restrict__ ftop, double *__restrict__ fbot) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Emitted flux of one face: eps sigma T^4, with emissivity 1 in a band that does not scatter.
+__device__ __forceinline__ float emitted(float e, int depth, float temperature) {
+    const float sigma = 5.6703744e-8f;
+    if (depth == 0 && e != 1.f) e = 1.f;
+    const double T = (double)temperature;
+    return (float)((double)(sigma * e) * (T * T * T * T));
+}
+
+// Between two passes of a solve, one launch each where a copy, fold, conversion or zeroing of one
+// buffer at a time made six to nine: a solve of a few thousand primitives spends its time in launches.
+
+// Start of a solve: every radiation buffer, the diffuse sums and the ray counter to zero.
+__global__ void k_begin_solve(size_t m, double *__restrict__ rin, double *__restrict__ stop, double *__restrict__ sbot,
+                              float *__restrict__ otop, float *__restrict__ obot, double *__restrict__ Gt,
+                              double *__restrict__ Gb, unsigned long long *counter) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *counter = 0ull;
+    if (i >= m) return;
+    rin[i] = stop[i] = sbot[i] = Gt[i] = Gb[i] = 0.0;
+    otop[i] = obot[i] = 0.f;
+}
+
+// Outgoing flux of the first diffuse or scattering pass: the scattered direct energy (fold; top and
+// bottom together on one-sided primitives; the scatter sums go back to zero) plus emission (em set).
+__global__ void k_outgoing(int n, int Bl, const int8_t *__restrict__ ts, int fold, double *__restrict__ stop,
+                           double *__restrict__ sbot, const uint8_t *__restrict__ em, const int32_t *__restrict__ depth,
+                           const float *__restrict__ eps, const float *__restrict__ temp, float *__restrict__ otop,
+                           float *__restrict__ obot) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)n * Bl) return;
-    int p = (int)(i / Bl);
-    double a = stop[i], b = sbot[i];
-    if (ts[p] == 0) {
-        double t = a + b;
-        ftop[i] = t;
-        fbot[i] = t;
-    } else {
-        ftop[i] = a;
-        fbot[i] = b;
+    const int p = (int)(i / Bl), b = (int)(i % Bl);
+    double t = 0.0, u = 0.0;
+    if (fold) {
+        t = stop[i];
+        u = sbot[i];
+        if (ts[p] == 0) t = u = t + u;
+        stop[i] = sbot[i] = 0.0;
     }
+    if (em && em[b]) {
+        const float out = emitted(eps[i], depth[b], temp[p]);
+        t += out;
+        if (ts[p] != 0) u += out;
+    }
+    otop[i] = (float)t;
+    obot[i] = (float)u;
+}
+
+// Before a scattering pass: the last pass's scatter becomes the outgoing flux (copy), and the scatter
+// and diffuse sums go to zero.
+__global__ void k_next_pass(size_t m, int copy, double *__restrict__ stop, double *__restrict__ sbot,
+                            float *__restrict__ otop, float *__restrict__ obot, double *__restrict__ Gt,
+                            double *__restrict__ Gb) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    if (copy) {
+        otop[i] = (float)stop[i];
+        obot[i] = (float)sbot[i];
+    }
+    stop[i] = sbot[i] = Gt[i] = Gb[i] = 0.0;
 }
 
 __global__ void k_emission(int n, int Bl, const uint8_t *__restrict__ em, const int32_t *__restrict__ depth,
@@ -515,11 +560,7 @@ __global__ void k_emission(int n, int Bl, const uint8_t *__restrict__ em, const 
     if (i >= (int64_t)n * Bl) return;
     int p = (int)(i / Bl), b = (int)(i % Bl);
     if (!em[b]) return;
-    const float sigma = 5.6703744e-8f;
-    float e = eps[i];
-    if (depth[b] == 0 && e != 1.f) e = 1.f;
-    double T = (double)temp[p];
-    float out = (float)((double)(sigma * e) * (T * T * T * T));
+    const float out = emitted(eps[i], depth[b], temp[p]);
     ftop[i] += out;
     if (ts[p] != 0) fbot[i] += out;
 }
@@ -851,11 +892,26 @@ cudaError_t launch_to_float(const double *a, float *out, size_t n, cudaStream_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_fold_onesided(int n, int Bl, const int8_t *twosided, const double *stop, const double *sbot,
-                                 double *ftop, double *fbot, cudaStream_t s) {
-    int64_t m = (int64_t)n * Bl;
+cudaError_t launch_begin_solve(size_t m, double *rin, double *stop, double *sbot, float *otop, float *obot, double *Gt,
+                               double *Gb, unsigned long long *counter, cudaStream_t s) {
+    k_begin_solve<<<blocks_for((int64_t)(m ? m : 1), 256), 256, 0, s>>>(m, rin, stop, sbot, otop, obot, Gt, Gb, counter);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_outgoing(int n, int Bl, const int8_t *twosided, int fold, double *stop, double *sbot,
+                            const uint8_t *emission, const int32_t *depth, const float *eps, const float *temperature,
+                            float *otop, float *obot, cudaStream_t s) {
+    const int64_t m = (int64_t)n * Bl;
     if (m <= 0) return cudaSuccess;
-    k_fold<<<blocks_for(m, 256), 256, 0, s>>>(n, Bl, twosided, stop, sbot, ftop, fbot);
+    k_outgoing<<<blocks_for(m, 256), 256, 0, s>>>(n, Bl, twosided, fold, stop, sbot, emission, depth, eps, temperature,
+                                                 otop, obot);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_next_pass(size_t m, int copy, double *stop, double *sbot, float *otop, float *obot, double *Gt,
+                             double *Gb, cudaStream_t s) {
+    if (m == 0) return cudaSuccess;
+    k_next_pass<<<blocks_for((int64_t)m, 256), 256, 0, s>>>(m, copy, stop, sbot, otop, obot, Gt, Gb);
     return cudaGetLastError();
 }
 
