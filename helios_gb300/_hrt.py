@@ -581,6 +581,9 @@ class Context:
         n = int(np.asarray(surf["air_temperature"]).size)
         R = None if net_radiation is None else f32(net_radiation).ravel()
         T0 = None if temperature is None else f32(temperature).ravel()
+        # the device may read these arrays in place: a short one must not reach it
+        if any(a is not None and a.size < n for a in (*keep, R, T0)):
+            raise ValueError("surface arrays, net_radiation and temperature need a value per primitive")
         T = np.zeros(n, np.float32)
         out = np.zeros((n, 5), np.float32) if outputs else None
         self.check(self.lib.hrt_energy_balance(self.h, n, C.byref(s), ptr(R), ptr(T0), ptr(T), ptr(out)))

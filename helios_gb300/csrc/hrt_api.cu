@@ -157,6 +157,7 @@ bool find_lattice(const float *T, const std::vector<uint32_t> &vox, const float 
 struct hrt_context {
     int device = 0;
     int sms = 152;
+    bool reads_host = false;  // the device reads pageable host memory through the host's page tables
     cudaStream_t own = nullptr, stream = nullptr;
     std::string err;
     // geometry
@@ -934,8 +935,8 @@ int ensure_camera_labels(hrt_context *ctx, int W, int H) {
     return HRT_OK;
 }
 
-// Energy balance: upload the surface arrays of n primitives.
-int upload_surface(hrt_context *ctx, int n, const hrt_surface *s) {
+// The surface arrays of an energy balance are all there.
+int check_surface(hrt_context *ctx, const hrt_surface *s) {
     if (!s) return fail(ctx, HRT_EINVAL, "null surface");
     const float *a[10] = {s->air_temperature, s->air_vapor_pressure, s->air_pressure, s->bl_conductance,
                           s->moisture_conductance, s->emissivity, s->other_flux, s->heat_capacity,
@@ -944,13 +945,12 @@ int upload_surface(hrt_context *ctx, int n, const hrt_surface *s) {
         if (!x) return fail(ctx, HRT_EINVAL, "null surface array");
     if (!s->nsides) return fail(ctx, HRT_EINVAL, "null surface array");
     if (!(s->dt >= 0.f)) return fail(ctx, HRT_EINVAL, "dt must be >= 0");
+    return HRT_OK;
+}
+
+// Device buffers of an energy balance of n primitives.
+int ensure_balance(hrt_context *ctx, int n, const hrt_surface *s) {
     const size_t N = (size_t)n;
-    CU(ctx->eb_surf.ensure(ctx->stream, 10 * N * sizeof(float)));
-    CU(ctx->eb_sides.ensure(ctx->stream, N));
-    for (int k = 0; k < 10; ++k)
-        CU(cudaMemcpyAsync(ctx->eb_surf.as<float>() + k * N, a[k], N * sizeof(float), cudaMemcpyHostToDevice,
-                           ctx->stream));
-    CU(cudaMemcpyAsync(ctx->eb_sides.p, s->nsides, N, cudaMemcpyHostToDevice, ctx->stream));
     CU(ctx->eb_R.ensure(ctx->stream, N * sizeof(float)));
     CU(ctx->eb_T.ensure(ctx->stream, N * sizeof(float)));
     CU(ctx->eb_out.ensure(ctx->stream, 5 * N * sizeof(float)));
@@ -961,33 +961,88 @@ int upload_surface(hrt_context *ctx, int n, const hrt_surface *s) {
     return HRT_OK;
 }
 
-// One energy-balance solve over the uploaded surface: R (device [n]) and Tin (device [n]) to
-// ctx->eb_T; counts unconverged primitives into eb_status[0].
-int eb_solve(hrt_context *ctx, const float *R, const float *Tin, bool outputs) {
+// Upload the surface arrays of n primitives, for balances that are solved again and again.
+int upload_surface(hrt_context *ctx, int n, const hrt_surface *s) {
+    int r;
+    if ((r = check_surface(ctx, s)) || (r = ensure_balance(ctx, n, s))) return r;
+    const float *a[10] = {s->air_temperature, s->air_vapor_pressure, s->air_pressure, s->bl_conductance,
+                          s->moisture_conductance, s->emissivity, s->other_flux, s->heat_capacity,
+                          s->surface_humidity, s->stomatal_sidedness};
+    const size_t N = (size_t)n;
+    CU(ctx->eb_surf.ensure(ctx->stream, 10 * N * sizeof(float)));
+    CU(ctx->eb_sides.ensure(ctx->stream, N));
+    for (int k = 0; k < 10; ++k)
+        CU(cudaMemcpyAsync(ctx->eb_surf.as<float>() + k * N, a[k], N * sizeof(float), cudaMemcpyHostToDevice,
+                           ctx->stream));
+    CU(cudaMemcpyAsync(ctx->eb_sides.p, s->nsides, N, cudaMemcpyHostToDevice, ctx->stream));
+    return HRT_OK;
+}
+
+// One energy-balance solve of ctx->eb_n primitives: R and Tin to Tout (which may be Tin); counts
+// unconverged primitives into eb_status[0].  host: read the caller's arrays where they are (each is
+// read once), else the uploaded ones.
+int eb_solve(hrt_context *ctx, const hrt_surface *host, const float *R, const float *Tin, float *Tout, bool outputs) {
     const size_t N = (size_t)ctx->eb_n;
     EnergyParams P{};
     P.n = ctx->eb_n;
     P.R = R;
     P.Tin = Tin;
     const float *f = ctx->eb_surf.as<float>();
-    P.Ta = f;
-    P.ea = f + N;
-    P.press = f + 2 * N;
-    P.gH = f + 3 * N;
-    P.gS = f + 4 * N;
-    P.eps = f + 5 * N;
-    P.Qother = f + 6 * N;
-    P.cap = f + 7 * N;
-    P.hs = f + 8 * N;
-    P.sided = f + 9 * N;
-    P.nsides = ctx->eb_sides.as<uint8_t>();
+    P.Ta = host ? host->air_temperature : f;
+    P.ea = host ? host->air_vapor_pressure : f + N;
+    P.press = host ? host->air_pressure : f + 2 * N;
+    P.gH = host ? host->bl_conductance : f + 3 * N;
+    P.gS = host ? host->moisture_conductance : f + 4 * N;
+    P.eps = host ? host->emissivity : f + 5 * N;
+    P.Qother = host ? host->other_flux : f + 6 * N;
+    P.cap = host ? host->heat_capacity : f + 7 * N;
+    P.hs = host ? host->surface_humidity : f + 8 * N;
+    P.sided = host ? host->stomatal_sidedness : f + 9 * N;
+    P.nsides = host ? host->nsides : ctx->eb_sides.as<uint8_t>();
     P.dt = ctx->eb_dt;
     P.T_default = ctx->eb_Tdef;
-    P.Tout = ctx->eb_T.as<float>();
+    P.Tout = Tout;
     P.out = outputs ? ctx->eb_out.as<float>() : nullptr;
     P.status = ctx->eb_status.as<unsigned>();
     CU(cudaMemsetAsync(ctx->eb_status.p, 0, 2 * sizeof(unsigned), ctx->stream));
     CU(launch_energy_balance(P, ctx->stream));
+    return HRT_OK;
+}
+
+// A kernel may read these caller's arrays in place: plain host memory, aligned for its type.  Pointers
+// that CUDA knows (device, managed, registered memory) keep the route of the copies.
+bool reads_in_place(const hrt_context *ctx, const hrt_surface *s, const float *R, const float *T) {
+    if (!ctx->reads_host) return false;
+    const void *a[13] = {s->air_temperature, s->air_vapor_pressure, s->air_pressure, s->bl_conductance,
+                         s->moisture_conductance, s->emissivity, s->other_flux, s->heat_capacity,
+                         s->surface_humidity, s->stomatal_sidedness, R, T, s->nsides};
+    for (int k = 0; k < 13; ++k) {
+        if (!a[k]) continue;
+        if (k < 12 && (uintptr_t)a[k] % alignof(float)) return false;
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, a[k]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeUnregistered) return false;
+    }
+    return true;
+}
+
+// Solve a balance into emis_T, hand its results to the caller and wait for them.
+int finish_balance(hrt_context *ctx, const hrt_surface *host, const float *R, const float *Tin, float *temperature_out,
+                   float *fluxes_out) {
+    const size_t N = (size_t)ctx->eb_n;
+    cudaStream_t st = ctx->stream;
+    int r = eb_solve(ctx, host, R, Tin, ctx->emis_T.as<float>(), fluxes_out != nullptr);
+    if (r) return r;
+    CU(cudaMemcpyAsync(ctx->pinned, ctx->eb_status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    if (temperature_out) CU(cudaMemcpyAsync(temperature_out, ctx->emis_T.p, N * sizeof(float), cudaMemcpyDeviceToHost, st));
+    if (fluxes_out) CU(cudaMemcpyAsync(fluxes_out, ctx->eb_out.p, 5 * N * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CU(cudaStreamSynchronize(st));
+    unsigned bad;
+    std::memcpy(&bad, ctx->pinned, sizeof bad);
+    ctx->eb_unconverged = bad;
     return HRT_OK;
 }
 
@@ -1087,6 +1142,10 @@ int hrt_create(hrt_context **out, int device) {
         return HRT_ECUDA;
     }
     cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device);
+    int pageable = 0, tables = 0;
+    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) == cudaSuccess)
+        ctx->reads_host = pageable && tables;
     if (cudaStreamCreateWithFlags(&ctx->own, cudaStreamNonBlocking) != cudaSuccess) {
         delete ctx;
         return HRT_ECUDA;
@@ -1462,31 +1521,46 @@ int hrt_energy_balance(hrt_context *ctx, int32_t n, const hrt_surface *s, const 
     if (n == 0) return HRT_OK;
     CU(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
-    int r = upload_surface(ctx, n, s);
+    int r = check_surface(ctx, s);
     if (r) return r;
+    // Where the device reads the host's pages through its page tables, the kernel takes each input
+    // straight from the caller's arrays, once.  The link is no faster that way (172 GB/s read in place,
+    // 165 copied); what goes is the cost of thirteen copies.  A call with arrays not seen before, copied
+    // and in place: 1 primitive 76 and 54 us, 5,000 105 and 73, 50,000 252 and 113, 500,009 658 and 489,
+    // 2,000,003 2.89 and 2.70 ms.  There is no size at which copies are better.  Arrays that a kernel
+    // cannot read as they are (misaligned, or not plain host memory) are copied.
+    const hrt_surface *host = reads_in_place(ctx, s, net_radiation, temperature) ? s : nullptr;
+    if ((r = host ? ensure_balance(ctx, n, s) : upload_surface(ctx, n, s))) return r;
     const size_t N = (size_t)n;
-    if (net_radiation) {
+    const float *R = ctx->eb_R.as<float>();
+    if (net_radiation && host) {
+        R = net_radiation;
+    } else if (net_radiation) {
         CU(cudaMemcpyAsync(ctx->eb_R.p, net_radiation, N * sizeof(float), cudaMemcpyHostToDevice, st));
     } else {
         if (n != ctx->n || ctx->Bl <= 0 || !ctx->fin.p)
             return fail(ctx, HRT_EINVAL, "no device fluxes of this scene; call hrt_run_band() first or pass net_radiation");
         CU(launch_net_radiation(n, ctx->Bl, ctx->fin.as<float>(), ctx->eb_R.as<float>(), st));
     }
+    const float *Tin;
     if (temperature) {
         CU(ctx->emis_T.ensure(st, N * sizeof(float)));
-        CU(cudaMemcpyAsync(ctx->emis_T.p, temperature, N * sizeof(float), cudaMemcpyHostToDevice, st));
-        ctx->emis_T_count = N;
+        if (!host) CU(cudaMemcpyAsync(ctx->emis_T.p, temperature, N * sizeof(float), cudaMemcpyHostToDevice, st));
+        if (!host) ctx->emis_T_count = N;
+        Tin = host ? temperature : ctx->emis_T.as<float>();
     } else if (ctx->emis_T_count != N) {
         return fail(ctx, HRT_EINVAL, "no resident temperatures for these primitives; pass temperature");
+    } else {
+        Tin = ctx->emis_T.as<float>();
     }
-    if ((r = eb_solve(ctx, ctx->eb_R.as<float>(), ctx->emis_T.as<float>(), fluxes_out != nullptr))) return r;
-    CU(cudaMemcpyAsync(ctx->emis_T.p, ctx->eb_T.p, N * sizeof(float), cudaMemcpyDeviceToDevice, st));
-    unsigned bad = 0;
-    CU(cudaMemcpyAsync(&bad, ctx->eb_status.p, sizeof bad, cudaMemcpyDeviceToHost, st));
-    if (temperature_out) CU(cudaMemcpyAsync(temperature_out, ctx->eb_T.p, N * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (fluxes_out) CU(cudaMemcpyAsync(fluxes_out, ctx->eb_out.p, 5 * N * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    ctx->eb_unconverged = bad;
+    // emis_T holds no temperatures of this scene until the solve has written them
+    if (host) ctx->emis_T_count = 0;
+    r = finish_balance(ctx, host, R, Tin, temperature_out, fluxes_out);
+    if (r) {
+        cudaStreamSynchronize(st);  // no read of the caller's arrays outlives the call
+        return r;
+    }
+    ctx->emis_T_count = N;
     return HRT_OK;
 }
 
@@ -1515,7 +1589,7 @@ int hrt_run_coupled(hrt_context *ctx, const hrt_band_solve *s, const hrt_surface
         if (ctx->emis_T_count != N)
             return fail(ctx, HRT_EINVAL, "the coupled solve needs temperatures (hrt_band_solve.temperature)");
         CU(launch_net_radiation(n, ctx->Bl, ctx->fin.as<float>(), ctx->eb_R.as<float>(), st));
-        if ((r = eb_solve(ctx, ctx->eb_R.as<float>(), ctx->emis_T.as<float>(), false))) return r;
+        if ((r = eb_solve(ctx, nullptr, ctx->eb_R.as<float>(), ctx->emis_T.as<float>(), ctx->eb_T.as<float>(), false))) return r;
         CU(launch_max_abs_diff(n, ctx->eb_T.as<float>(), ctx->emis_T.as<float>(), ctx->eb_status.as<unsigned>() + 1, st));
         CU(cudaMemcpyAsync(ctx->emis_T.p, ctx->eb_T.p, N * sizeof(float), cudaMemcpyDeviceToDevice, st));
         unsigned h[2] = {0, 0};

@@ -62,6 +62,35 @@ def test_energy_balance_vs_oracle(oracle_mod):
         assert np.allclose(o1[:, 4], o2[:, 4], rtol=1e-3, atol=1e-6)
 
 
+def _misaligned(a):
+    """A copy of a float array that starts one byte off its type's alignment."""
+    raw = np.zeros(a.nbytes + 8, np.uint8)
+    v = raw[1:1 + a.nbytes].view(a.dtype)
+    v[:] = a
+    return v
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 4097, 100003])
+def test_inputs_read_in_place_equal_copied_ones(n):
+    """The kernel does the same arithmetic wherever its inputs lie, so the bytes are the same when
+    one or all arrays are misaligned (which a kernel cannot read, so they are copied)."""
+    from helios_gb300 import _hrt
+    ctx = _hrt.Context(0)
+    surf, R, To = _random_surface(n, n)
+    want = ctx.energy_balance(surf, net_radiation=R, temperature=To, outputs=True)
+    floats = [k for k, v in surf.items() if isinstance(v, np.ndarray) and v.dtype == np.float32]
+    for names in ([floats[0]], [floats[-1]], floats):
+        off = dict(surf, **{k: _misaligned(surf[k]) for k in names})
+        got = ctx.energy_balance(off, net_radiation=R, temperature=To, outputs=True)
+        assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(want, got))
+    got = ctx.energy_balance(surf, net_radiation=_misaligned(R), temperature=_misaligned(To), outputs=True)
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(want, got))
+    # resident temperatures of the call before: the same as passing its result
+    again = ctx.energy_balance(surf, net_radiation=R, outputs=True)
+    passed = ctx.energy_balance(surf, net_radiation=R, temperature=want[0], outputs=True)
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(again, passed))
+
+
 def _coupled_scene(seed=0, n_leaves=1500):
     sc = scenes.homogeneous_canopy(n_leaves=n_leaves, leaf=0.1, domain=3.0, zlo=0.5, zhi=2.0, seed=seed)
     ctx = Context()
