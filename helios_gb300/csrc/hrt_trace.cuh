@@ -696,9 +696,8 @@ __device__ __forceinline__ double sky_fd(f3 dir, const SkyParams &sky, int b) {
 // 4-wide trace took 80.5 ms with it against 78.1 ms without.  HRT_REFILL overrides (0-32).
 constexpr int kRefillDefault = 8;
 // The lean 4-wide trace (hrt_trace_w4.cuh) keeps fewer registers per lane and refills more
-// cheaply; on the same workload, per diffuse launch, with two postponed leaves and no leaf
-// vote: 8 162.5 ms, 10 160.4 ms, 12 160.2 ms, 14 161.2 ms, 16 162.7 ms, 18 161.8 ms, 20 161.1 ms,
-// 24 170.6 ms (run to run on one box within 0.02 ms).
+// cheaply.  Diffuse ms per solve at 8 / 10 / 12 / 14 / 16 lanes: 1 M orchard 810.6 / 800.6 / 798.6 / 802.3 /
+// 808.6, canopy of 20,001 15.25 / 14.93 / 14.71 / 14.64 / 14.61, periodic stand 35.3 / 34.95 / 34.93 / 35.2 / 35.7.
 constexpr int kRefillLean = 12;
 // With a lattice of voxels to march a refill costs more code: on the deep-scattering section 4 362 ms of
 // diffuse launches, 6 364 ms, 8 369 ms, 12 377 ms.
