@@ -517,12 +517,21 @@ GlassParams glass_params(hrt_context *ctx, int Bg, int Bl) {
 }
 
 // Buffers of the grids of `nsrc` collimated sources and the scene's extent (queued on the context's
-// stream); *nb: sources per batch.
+// stream); *nb: sources per batch, 0 where the device has no memory left for them (the rays then go
+// through the tree, which needs none).
 int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
     const SunCaps caps = sun_caps(ctx->n);
     *nb = std::max(1, std::min(caps.batch, nsrc));
-    CU(ctx->sg_cells.ensure(ctx->stream, (size_t)*nb * caps.cells * sizeof(uint2)));
-    CU(ctx->sg_entries.ensure(ctx->stream, (size_t)*nb * caps.entries * sizeof(uint2)));
+    cudaError_t e = ctx->sg_cells.ensure(ctx->stream, (size_t)*nb * caps.cells * sizeof(uint2));
+    if (e == cudaSuccess) e = ctx->sg_entries.ensure(ctx->stream, (size_t)*nb * caps.entries * sizeof(uint2));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ctx->sg_cells.free_on(ctx->stream);
+        ctx->sg_entries.free_on(ctx->stream);
+        *nb = 0;
+        return HRT_OK;
+    }
+    CU(e);
     CU(ctx->sg_grids.ensure(ctx->stream, (size_t)kSunBatch * sizeof(SunGrid)));
     CU(ctx->sg_done.ensure(ctx->stream, (size_t)std::max(nsrc, 1) * sizeof(uint32_t)));
     CU(ctx->sg_extent.ensure(ctx->stream, 9 * sizeof(uint32_t)));
@@ -593,11 +602,14 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
     const uint32_t per = chunk_prims(ctx, (uint64_t)dimx * (uint64_t)dimy);
     if (per == 0) return HRT_EUNSUPPORTED;
     uint32_t chunks = 0;
-    const bool grids = !cov && sun_grids_pay(ctx, (unsigned long long)count * (unsigned)(dimx * dimy)) &&
+    bool grids = !cov && sun_grids_pay(ctx, (unsigned long long)count * (unsigned)(dimx * dimy)) &&
                        std::find(ctx->h_src_type.begin(), ctx->h_src_type.end(), 0) != ctx->h_src_type.end();
     int batch = 1;
     if (grids) {
         if ((r = ensure_sun_grids(ctx, ctx->S, &batch))) return r;
+        grids = batch > 0;
+    }
+    if (grids) {
         CU(cudaMemsetAsync(ctx->sg_done.p, 0, (size_t)ctx->S * sizeof(uint32_t), ctx->stream));
         P.done = ctx->sg_done.as<uint32_t>();
     }
@@ -1382,8 +1394,13 @@ int hrt_build_accel(hrt_context *ctx) {
     // leaves (voxel codes sort last)
     const int ns = n - (int)ctx->h_voxels.size();
     ctx->use_lattice = false;
+    cudaError_t se = cudaErrorMemoryAllocation;  // no memory for it: the one tree of everything serves
     if (ctx->have_lattice && ns >= 2) {
-        CU(ctx->nodes4s.ensure(ctx->stream, bvh4_node_capacity(ns) * 4 * sizeof(float4)));
+        se = ctx->nodes4s.ensure(ctx->stream, bvh4_node_capacity(ns) * 4 * sizeof(float4));
+        if (se == cudaErrorMemoryAllocation) cudaGetLastError();
+        else CU(se);
+    }
+    if (se == cudaSuccess) {
         if ((uintptr_t)ctx->nodes4s.p & 63u) return fail(ctx, HRT_ECUDA, "node arrays are not 64-byte aligned");
         CU(ploc_build(b.leafbox, ns, ploc_nodes.as<float4>(), ploc_scratch.p, ctx->stream));
         CU(bvh4_build(ploc_nodes.as<float4>(), ns, ctx->nodes4s.as<float4>(), ctx->bvh_scratch.p,
