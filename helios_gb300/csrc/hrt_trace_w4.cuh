@@ -178,9 +178,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_diffuse_w4(const DiffuseParams 
         s_chunk[1][tid >> 5] = 0ull;
     }
     __syncwarp();
-    // ends the traversal of the lane's ray after an error
+    // ends the traversal of the lane's ray after an error, which is its own scene's (a multi-scene launch
+    // leaves P.sc empty)
     auto give_up = [&](uint32_t bit) {
-        raise(P.sc.status, bit);
+        raise(SC.status, bit);
         cur = kSentinel;
         leaf = 0;
         leaf2 = 0;

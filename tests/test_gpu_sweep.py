@@ -129,3 +129,32 @@ def test_multi_scene_sweep_equals_each_scene_alone():
             np.testing.assert_allclose(multi[k], alone[k], rtol=1e-6, atol=1e-9)
             assert c.last_stats()["rays"] == rays[k]
             assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("bad", [0, 1, 2])
+def test_multi_scene_sweep_reports_the_failing_scene(bad):
+    """A scene whose rays run out of their visit budget in the recording launch (no direct pass, which
+    has its own checks): the call fails and names the scene, and the next one is clean."""
+    from helios_gb300 import _hrt
+
+    ctxs, sweeps = [], []
+    for k, n in enumerate((900, 1500, 600)):
+        sc = scenes.mixed_canopy(n, 2.0, seed=k)
+        c = _hrt.Context(0)
+        c.update_geometry(sc.T, sc.ptype, sc.twosided)
+        c.build_accel()
+        ctxs.append(c)
+        sweeps.append(dict(sun_dir=np.array([[0.1, 0.2, 0.9]]), direct_flux=np.zeros((1, 1)), diffuse_flux=np.full((1, 1), 100.0),
+                           rho=np.full((sc.n, 1), 0.3), tau=np.full((sc.n, 1), 0.2), direct_rays=25, diffuse_rays=49,
+                           depth=1, seed=3))
+    before = _hrt.run_sweep_multi(ctxs, sweeps)
+    ctxs[bad].set_visit_budget(2)
+    with pytest.raises(_hrt.HrtError) as e:
+        _hrt.run_sweep_multi(ctxs, sweeps)
+    assert e.value.code == _hrt.HRT_EDEVICE and "visit budget" in str(e.value)
+    assert bad == 0 or f"scene {bad}" in str(e.value)
+    ctxs[bad].set_visit_budget(0)
+    after = _hrt.run_sweep_multi(ctxs, sweeps)
+    for a, b, c in zip(after, before, ctxs):
+        np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-9)
+        assert c.device_status() == 0
