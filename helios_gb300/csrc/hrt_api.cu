@@ -1107,12 +1107,11 @@ int set_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sources, b
     if (nsources > 256) return fail(ctx, HRT_EINVAL, "A maximum of 256 radiation sources are allowed.");
     CU(cudaSetDevice(ctx->device));
     std::vector<SourceDev> h((size_t)std::max(nsources, 1));
-    ctx->h_src_type.assign((size_t)nsources, 0);
+    std::vector<int> type((size_t)nsources);
     for (int k = 0; k < nsources; ++k) {
         if (sources[k].type > 4) return fail(ctx, HRT_EINVAL, "unknown source type");
         SourceDev &s = h[k];
-        s.type = (int)sources[k].type;
-        ctx->h_src_type[k] = s.type;
+        s.type = type[k] = (int)sources[k].type;
         for (int i = 0; i < 3; ++i) s.pos[i] = sources[k].position[i];
         s.w0 = sources[k].width[0];
         s.w1 = sources[k].width[1];
@@ -1120,6 +1119,7 @@ int set_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sources, b
     }
     CU(ctx->src.ensure(ctx->stream, h.size() * sizeof(SourceDev)));
     CU(cudaMemcpyAsync(ctx->src.p, h.data(), h.size() * sizeof(SourceDev), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->h_src_type.swap(type);  // with S: a refused list leaves the resident sources as they were
     ctx->S = nsources;
     if (wait) CU(cudaStreamSynchronize(ctx->stream));
     return HRT_OK;

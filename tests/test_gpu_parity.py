@@ -619,3 +619,27 @@ def test_device_matches_reference_estimator(oracle_mod):
     with oracle_mod.reference_rng():
         ref = ensemble(lambda s: run_oracle(rad, ["SW"], oracle_mod, scene=scene, seed=s + 1000)[0], seeds)
     check_statistical_parity(dev, ref, sc.area)
+
+
+@pytest.mark.parametrize("count", [3, 1, 40])
+def test_refused_sources_leave_the_resident_ones(count):
+    """An update with a source of an unknown type is refused; the solve goes on with the sources that
+    were there, a sphere among them, whether the refused list was as long, shorter or longer."""
+    from helios_gb300 import _hrt
+
+    sc = scenes.mixed_canopy(2500, 2.0, seed=1)
+    c = _hrt.Context(0)
+    c.update_geometry(sc.T, sc.ptype, sc.twosided)
+    c.build_accel()
+    sources = [{"type": 1, "position": (0.5, 0.5, 9.0), "width": (0.4, 0.0)}, {"type": 0, "position": (0.3, 0.2, 0.9)},
+               {"type": 1, "position": (1.0, 1.0, 9.0), "width": (0.4, 0.0)}]
+    d = {"band_launch": np.array([1], np.uint8), "sources": sources, "source_flux": np.full((3, 1), 100.0),
+         "rho": np.zeros((3, sc.n, 1)), "tau": np.zeros((3, sc.n, 1)), "diffuse_flux": np.array([0.0]),
+         "direct_rays": np.array([100]), "diffuse_rays": np.array([1]), "depth": np.array([0]),
+         "emission": np.array([0], np.uint8), "seed": 3}
+    want = c.run_band(d)
+    bad = [{"type": 0, "position": (0.0, 0.0, 1.0)}] * (count - 1) + [{"type": 9, "position": (0.0, 0.0, 1.0)}]
+    with pytest.raises(_hrt.HrtError):
+        c.update_sources(bad)
+    got = c.run_band(dict(d, sources=None, nsources=3))
+    np.testing.assert_allclose(got, want, rtol=1e-6)
