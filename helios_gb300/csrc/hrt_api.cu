@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -194,6 +195,8 @@ struct hrt_context {
     DevBuf io_a, io_b, io_c;  // staging for inspection calls
     uint64_t last_rays = 0, last_kernels = 0, last_iters = 0;
     unsigned long long *pinned = nullptr;  // [0] ray count, [1] device error word
+    // host arrays of queued copies, until the stream has been waited for (upload_local)
+    std::vector<std::shared_ptr<const void>> staged;
     DevBuf resid;  // scattering residual: block partials and the per-band result
     // measurement: bit 0 counts traversal work, bit 1 times trace launches
     int measure = 0;
@@ -379,6 +382,22 @@ int check_built(hrt_context *ctx) {
     return HRT_OK;
 }
 
+// Queues the copy of an array that the call has made to dst and keeps the array until the stream has
+// been waited for (waited): a copy from pageable memory may read its source as late as that.
+template <class T>
+cudaError_t upload_local(hrt_context *ctx, void *dst, std::vector<T> &&v) {
+    auto keep = std::make_shared<const std::vector<T>>(std::move(v));
+    ctx->staged.push_back(keep);
+    return cudaMemcpyAsync(dst, keep->data(), keep->size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream);
+}
+
+// Waits for the context's stream, after which no host array is read any more.
+cudaError_t waited(hrt_context *ctx) {
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    ctx->staged.clear();
+    return e;
+}
+
 int status_result(hrt_context *ctx, uint32_t st) {
     if (st) {
         CU(cudaMemsetAsync(ctx->status.p, 0, sizeof(uint32_t), ctx->stream));
@@ -397,7 +416,7 @@ int status_result(hrt_context *ctx, uint32_t st) {
 // each such wait cost a small solve some 10 us.
 int sync_and_status(hrt_context *ctx) {
     CU(cudaMemcpyAsync(ctx->pinned + 1, ctx->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
+    CU(waited(ctx));
     uint32_t st;
     std::memcpy(&st, ctx->pinned + 1, sizeof st);
     return status_result(ctx, st);
@@ -432,7 +451,7 @@ int upload_sky(hrt_context *ctx, int Bl, const float *flux, const float *K, cons
     ctx->sky_any = false;
     for (int b = 0; b < Bl; ++b) ctx->sky_any = ctx->sky_any || h[b] > 0.f;
     CU(ctx->sky.ensure(ctx->stream, h.size() * sizeof(float)));
-    CU(cudaMemcpyAsync(ctx->sky.p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    CU(upload_local(ctx, ctx->sky.p, std::move(h)));
     float *d = ctx->sky.as<float>();
     sp->flux = d;
     sp->K = d + Bn;
@@ -447,7 +466,7 @@ int upload_flags(hrt_context *ctx, int Bg, const uint8_t *flags) {
         return HRT_OK;  // on the device already
     ctx->h_flags.clear();
     CU(ctx->flags.ensure(ctx->stream, (size_t)std::max(Bg, 1)));
-    CU(cudaMemcpyAsync(ctx->flags.p, flags, (size_t)Bg, cudaMemcpyHostToDevice, ctx->stream));
+    CU(upload_local(ctx, ctx->flags.p, std::vector<uint8_t>(flags, flags + Bg)));
     ctx->h_flags.assign(flags, flags + Bg);
     return HRT_OK;
 }
@@ -492,8 +511,7 @@ int covers_for(hrt_context *ctx, int Bg, int nsrc, const uint32_t **out) {
         }
         if (any) {
             CU(ctx->cover.ensure(ctx->stream, bits.size() * sizeof(uint32_t)));
-            CU(cudaMemcpyAsync(ctx->cover.p, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                               ctx->stream));
+            CU(upload_local(ctx, ctx->cover.p, std::move(bits)));
         }
         ctx->cover_any = any;
         ctx->cover_key = key;
@@ -1088,17 +1106,16 @@ int set_materials(hrt_context *ctx, int32_t nsources, int32_t nprims, int32_t nb
                     vr[i] = h;
                     vt[i] = h;
                 }
-        rho = vr.data();
-        tau = vt.data();
-    }
-    if (m) {
+        CU(upload_local(ctx, ctx->rho.p, std::move(vr)));
+        CU(upload_local(ctx, ctx->tau.p, std::move(vt)));
+    } else if (m) {
         CU(cudaMemcpyAsync(ctx->rho.p, rho, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(ctx->tau.p, tau, m * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     }
     ctx->mS = nsources;
     ctx->mN = nprims;
     ctx->mB = nbands_global;
-    if (wait) CU(cudaStreamSynchronize(ctx->stream));
+    if (wait) CU(waited(ctx));
     return HRT_OK;
 }
 
@@ -1118,10 +1135,10 @@ int set_sources(hrt_context *ctx, int32_t nsources, const hrt_source *sources, b
         rotation3(sources[k].rotation, s.R);
     }
     CU(ctx->src.ensure(ctx->stream, h.size() * sizeof(SourceDev)));
-    CU(cudaMemcpyAsync(ctx->src.p, h.data(), h.size() * sizeof(SourceDev), cudaMemcpyHostToDevice, ctx->stream));
+    CU(upload_local(ctx, ctx->src.p, std::move(h)));
     ctx->h_src_type.swap(type);  // with S: a refused list leaves the resident sources as they were
     ctx->S = nsources;
-    if (wait) CU(cudaStreamSynchronize(ctx->stream));
+    if (wait) CU(waited(ctx));
     return HRT_OK;
 }
 
@@ -1210,7 +1227,7 @@ const char *hrt_last_error(const hrt_context *ctx) { return ctx ? ctx->err.c_str
 int hrt_set_stream(hrt_context *ctx, void *stream) {
     if (!ctx) return HRT_EINVAL;
     CU(cudaSetDevice(ctx->device));
-    CU(cudaStreamSynchronize(ctx->stream));  // buffers allocated on the old stream are ready
+    CU(waited(ctx));  // buffers allocated on the old stream are ready
     ctx->stream = stream ? (cudaStream_t)stream : ctx->own;
     return HRT_OK;
 }
@@ -1265,10 +1282,8 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
             CU(ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4)));
             CU(ctx->vg.ensure(ctx->stream, sizeof(VoxGrid)));
             vg.cells = ctx->vg_cells.as<float4>();
-            CU(cudaMemcpyAsync(ctx->vg_cells.p, cells.data(), cells.size() * sizeof(float4), cudaMemcpyHostToDevice,
-                               ctx->stream));
-            CU(cudaMemcpyAsync(ctx->vg.p, &vg, sizeof vg, cudaMemcpyHostToDevice, ctx->stream));
-            CU(cudaStreamSynchronize(ctx->stream));  // the host copies end here
+            CU(upload_local(ctx, ctx->vg_cells.p, std::move(cells)));
+            CU(upload_local(ctx, ctx->vg.p, std::vector<VoxGrid>{vg}));
             ctx->have_lattice = true;
         }
     }
@@ -1300,12 +1315,11 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
         CU(ctx->mask_offset.ensure(ctx->stream, (size_t)g->nmasks * sizeof(uint32_t)));
         CU(ctx->mask_data.ensure(ctx->stream, std::max<size_t>(total, 1)));
         CU(cudaMemcpyAsync(ctx->mask_id.p, g->mask_id, n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
-        CU(cudaMemcpyAsync(ctx->mask_uv_id.p, uvid.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
-        CU(cudaMemcpyAsync(ctx->mask_uv.p, uv.data(), 8 * n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+        CU(upload_local(ctx, ctx->mask_uv_id.p, std::move(uvid)));
+        CU(upload_local(ctx, ctx->mask_uv.p, std::move(uv)));
         CU(cudaMemcpyAsync(ctx->mask_size.p, g->mask_size, 2 * (size_t)g->nmasks * sizeof(int32_t),
                            cudaMemcpyHostToDevice, ctx->stream));
-        CU(cudaMemcpyAsync(ctx->mask_offset.p, off.data(), off.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                           ctx->stream));
+        CU(upload_local(ctx, ctx->mask_offset.p, std::move(off)));
         CU(cudaMemcpyAsync(ctx->mask_data.p, g->mask_data, total, cudaMemcpyHostToDevice, ctx->stream));
         ctx->masks = true;
     }
@@ -1333,12 +1347,12 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
         for (int i = 0; i < g->nbbox * 4; ++i)
             q[i] = make_float4(g->bbox_vertices[3 * i], g->bbox_vertices[3 * i + 1], g->bbox_vertices[3 * i + 2], 0.f);
         CU(ctx->bbox.ensure(ctx->stream, q.size() * sizeof(float4)));
-        CU(cudaMemcpyAsync(ctx->bbox.p, q.data(), q.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
+        CU(upload_local(ctx, ctx->bbox.p, std::move(q)));
     }
     ctx->n = g->n;
     ctx->have_geometry = true;
     ctx->built = false;
-    CU(cudaStreamSynchronize(ctx->stream));
+    CU(waited(ctx));
     return HRT_OK;
 }
 
@@ -1646,7 +1660,7 @@ int hrt_update_sky_model(hrt_context *ctx, int32_t nbands, const hrt_sky_model *
     for (size_t b = 0; b < B; ++b)
         for (int i = 0; i < 3; ++i) h[7 * B + 3 * b + i] = m->sun_direction[i];
     CU(ctx->cam_sky.ensure(ctx->stream, h.size() * sizeof(float)));
-    CU(cudaMemcpyAsync(ctx->cam_sky.p, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    CU(upload_local(ctx, ctx->cam_sky.p, std::move(h)));
     ctx->sky_has[4] = m->band_emission_flag != nullptr;
     if (m->band_emission_flag) {
         CU(ctx->cam_em.ensure(ctx->stream, B * sizeof(uint32_t)));
@@ -1656,7 +1670,7 @@ int hrt_update_sky_model(hrt_context *ctx, int32_t nbands, const hrt_sky_model *
     for (int i = 0; i < 3; ++i) ctx->sky_sun[i] = m->sun_direction[i];
     ctx->sky_cos = m->solar_disk_cos_angle;
     ctx->sky_B = nbands;
-    CU(cudaStreamSynchronize(ctx->stream));
+    CU(waited(ctx));
     return HRT_OK;
 }
 
@@ -2007,7 +2021,7 @@ static int run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) 
     CU(cudaMemcpyAsync(ctx->pinned + 1, ctx->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     // the fluxes last: a copy to pageable memory waits for all before it
     if (flux_out) CU(cudaMemcpyAsync(flux_out, ctx->fin.p, m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
+    CU(waited(ctx));
     uint32_t word;
     std::memcpy(&word, ctx->pinned + 1, sizeof word);
     ctx->last_rays = ctx->pinned[0];
@@ -2018,7 +2032,7 @@ static int run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) 
 extern "C" int hrt_run_band(hrt_context *ctx, const hrt_band_solve *s, float *flux_out) {
     const int r = run_band(ctx, s, flux_out);
     // a call that failed on its way may have uploads from the caller's arrays in flight
-    if (r != HRT_OK && ctx) cudaStreamSynchronize(ctx->stream);
+    if (r != HRT_OK && ctx) waited(ctx);
     return r;
 }
 
@@ -2108,8 +2122,8 @@ int sweep_prepare(hrt_context *ctx, const hrt_sweep *s, bool tune, SweepPlan *pl
         std::copy(s->diffuse_flux, s->diffuse_flux + C, h.begin() + 3 * nsun + C);
         std::vector<uint8_t> mk8;
         for (auto *v : {&all, &fold, &diffuse, &copy0, &active, &rundirect}) mk8.insert(mk8.end(), v->begin(), v->end());
-        CU(cudaMemcpyAsync(P.d_sun, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-        CU(cudaMemcpyAsync(d_masks, mk8.data(), mk8.size(), cudaMemcpyHostToDevice, st));
+        CU(upload_local(ctx, P.d_sun, std::move(h)));
+        CU(upload_local(ctx, d_masks, std::move(mk8)));
     }
     P.m_all = d_masks;
     P.m_fold = d_masks + C;
@@ -2402,7 +2416,7 @@ int hrt_run_sweep_multi(hrt_context *const *ctxs, const hrt_sweep *sweeps, int32
         if (ctxs[k]->n4 <= 0) return fail(ctx, HRT_EUNSUPPORTED, "multi-scene sweeps trace 4-wide trees");
         key += "|" + sweep_key(plans[k], &sweeps[k]);
     }
-    for (int k = 1; k < nscenes; ++k) CU(cudaStreamSynchronize(ctxs[k]->stream));  // their uploads
+    for (int k = 1; k < nscenes; ++k) CU(waited(ctxs[k]));  // their uploads
     cudaStream_t st = ctx->stream;
     // slot tables of the recording passes: pass 0 = primary diffuse, pass 1 + it = scattering it;
     // a pass lists the primitive chunks of every scene that traces it
@@ -2438,12 +2452,12 @@ int hrt_run_sweep_multi(hrt_context *const *ctxs, const hrt_sweep *sweeps, int32
             return fail(ctx, HRT_EUNSUPPORTED, "a multi-scene pass holds at most 32 scene chunks");
     }
     CU(ctx->sw_slots.ensure(st, std::max<size_t>(slots.size(), 1) * sizeof(SceneSlot)));
-    CU(cudaMemcpyAsync(ctx->sw_slots.p, slots.data(), slots.size() * sizeof(SceneSlot), cudaMemcpyHostToDevice, st));
     {
         char more[64];
         std::snprintf(more, sizeof more, "|slots %p %zu", ctx->sw_slots.p, slots.size());
         key += more;
     }
+    CU(upload_local(ctx, ctx->sw_slots.p, std::move(slots)));
     if (!ctx->mw_exec || ctx->mw_key != key) {
         int nk = 0;
         std::vector<SweepStages> S;
@@ -2493,7 +2507,7 @@ int hrt_run_sweep_multi(hrt_context *const *ctxs, const hrt_sweep *sweeps, int32
             CU(cudaMemcpyAsync(flux_out[k], plans[k].fin, plans[k].m * sizeof(float), cudaMemcpyDeviceToHost, st));
         CU(cudaMemcpyAsync(&rays[k], ctxs[k]->counter.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     }
-    CU(cudaStreamSynchronize(st));
+    CU(waited(ctx));
     int status = HRT_OK;
     unsigned long long total = 0;
     for (int k = 0; k < nscenes; ++k) {

@@ -209,6 +209,12 @@ __global__ void k_collapse_init(int2 *queue, unsigned *counters) {
     if (i < kWaves + 2) counters[i] = i == 0 ? 2u : (i == 1 ? 1u : 0u);
 }
 
+// Counters of a further batch of waves: its first wave has `left` items.
+__global__ void k_collapse_more(unsigned left, unsigned *counters) {
+    const int i = threadIdx.x;
+    if (i >= 1 && i < kWaves + 2) counters[i] = i == 1 ? left : 0u;
+}
+
 cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratch, uint32_t *status, int *count_out,
                        cudaStream_t s) {
     *count_out = 0;
@@ -248,9 +254,7 @@ cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratc
         if (h[1] > 0) {
             if (done >= kMaxWaves) return cudaErrorInvalidValue;
             waves = std::min(waves, kMaxWaves - done);
-            const unsigned left = h[1];
-            if ((e = cudaMemsetAsync(counters + 1, 0, (kWaves + 1) * sizeof(unsigned), s)) != cudaSuccess) return e;
-            if ((e = cudaMemcpyAsync(counters + 1, &left, sizeof left, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
+            k_collapse_more<<<1, 128, 0, s>>>(h[1], counters);
         }
     } while (h[1] > 0);
     *count_out = (int)std::min<unsigned>(h[0], (unsigned)cap);
