@@ -351,6 +351,22 @@ __host__ __device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv 
     const uint32_t t = (uint32_t)(((uint64_t)f.m * n) >> 32);  // umulhi
     return (t + ((n - t) >> f.s1)) >> f.s2;
 }
+// Cells of a grid over [-hu, hu] x [-hv, hv] with cells of side *side or more: at most cap of them and
+// at most 2^15 a side; false where no such grid exists (extents that are not finite).  Counted in
+// integers: products above 2^24 round as floats, which let a grid have a cell more than its buffer.
+__host__ __device__ __forceinline__ bool sun_cells(float hu, float hv, uint32_t cap, float *side, int *nu, int *nv) {
+    float h = *side;
+    for (int it = 0; it < 64; ++it, h *= 1.1f) {  // rounding up to whole cells may pass the limit by a little
+        const float fu = floorf(2.f * hu / h) + 1.f, fv = floorf(2.f * hv / h) + 1.f;
+        if (!(fu >= 1.f && fv >= 1.f)) return false;
+        if (fu > 32768.f || fv > 32768.f || (uint64_t)fu * (uint64_t)fv > (uint64_t)cap) continue;
+        *side = h;
+        *nu = (int)fu;
+        *nv = (int)fv;
+        return true;
+    }
+    return false;
+}
 // The four float4 of a 64-byte node (binary or 4-wide) in two 256-bit read-only loads; node
 // arrays start on a 256-byte boundary, so every node is 64-byte aligned.
 __device__ __forceinline__ void load_node64(const float4 *nodes, int32_t i, float4 &q0, float4 &q1, float4 &q2,

@@ -105,7 +105,7 @@ struct SunGrid {
     float u0, v0, inv_h, pad;
     int nu, nv;
     uint32_t total;        // entries
-    uint32_t ok;           // 0: the source's rays go through the tree
+    uint32_t ok;           // 0: no frame; the source's rays go through the tree
     uint32_t nlarge;
     uint2 large[kSunLarge];
 };

@@ -16,8 +16,8 @@
 // 200,004-primitive canopy 6.5 -> 1.7 ms, 6.3 M of a periodic stand 5.6 -> 1.1 ms, 2 M of the
 // 20,001-patch canopy 0.69 -> 0.21 ms; 96 suns over a 100 k orchard block 344 -> 121 ms per sweep.
 // A source whose grid would not pay (entries over the buffer, more than kSunLarge primitives that
-// cover over kSunWide cells, a direction that is not finite) clears its flag on the device and its
-// rays go through the tree (k_direct / k_direct_sweep skip the sources done here).
+// cover over kSunWide cells, a direction that is not finite) is not marked as done on the device and
+// its rays go through the tree (k_direct / k_direct_sweep skip the sources done here).
 #include "hrt_trace.cuh"
 
 namespace hrt {
@@ -137,22 +137,22 @@ __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stri
     const float area = 4.f * hu * hv;
     h = fmaxf(h, 1.01f * sqrtf(area / (float)cells_cap));
     h = fmaxf(h, 2.f * fmaxf(hu, hv) / 30000.f);
-    float fu = 0.f, fv = 0.f;
-    for (int it = 0; it < 64; ++it) {  // rounding up to whole cells may pass the limit by a little
-        fu = floorf(2.f * hu / h) + 1.f;
-        fv = floorf(2.f * hv / h) + 1.f;
-        if (!(fu * fv > (float)cells_cap)) break;
-        h *= 1.1f;
-    }
+    int nu = 1, nv = 1;
+    const bool fits = sun_cells(hu, hv, cells_cap, &h, &nu, &nv);
     g.inv_h = 1.f / h;
-    const bool fine = fu >= 1.f && fv >= 1.f && fu * fv <= (float)cells_cap && g.inv_h > 0.f && isfinite(g.inv_h) &&
-                      isfinite(g.u0) && isfinite(g.v0);
-    g.nu = fine ? (int)fu : 1;
-    g.nv = fine ? (int)fv : 1;
+    const bool fine = fits && g.inv_h > 0.f && isfinite(g.inv_h) && isfinite(g.u0) && isfinite(g.v0);
+    g.nu = fine ? nu : 1;
+    g.nv = fine ? nv : 1;
     g.ok = fine ? 1u : 0u;
     g.total = 0u;
     g.nlarge = 0u;
     grids[b] = g;
+}
+
+// Whether a binned source is traced by its grid: its entries fit and few primitives are wide.  The
+// flag of the frame is written once, by k_sun_setup, so that all threads of a block agree on it.
+__device__ __forceinline__ bool sun_served(const SunGrid &g, uint32_t entries_cap) {
+    return g.ok && g.nlarge <= (uint32_t)kSunLarge && g.total <= entries_cap;
 }
 
 struct CellRect {
@@ -222,8 +222,9 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
                                                          uint32_t entries_cap, uint32_t *done) {
     SunGrid *G = grids + blockIdx.y;
     const SunGrid &g = *G;
-    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) done[blockIdx.y] = g.ok;
-    if (!g.ok) return;
+    const bool on = FILL ? sun_served(g, entries_cap) : g.ok != 0u;
+    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) done[blockIdx.y] = on ? 1u : 0u;
+    if (!on) return;
     uint2 *cl = cells + (size_t)blockIdx.y * cells_cap;
     uint2 *en = entries + (size_t)blockIdx.y * entries_cap;
     const int i = blockIdx.x * kSunThreads + threadIdx.x;
@@ -232,10 +233,10 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
     if (!c.any) return;
     const int nc = (c.u1 - c.u0 + 1) * (c.v1 - c.v0 + 1);
     if (nc > kSunWide) {
-        if (FILL) return;
+        // past the limit the source is dropped, and its other wide primitives need not queue up here
+        if (FILL || *(volatile const uint32_t *)&G->nlarge > (uint32_t)kSunLarge) return;
         const uint32_t k = atomicAdd(&G->nlarge, 1u);
         if (k < kSunLarge) G->large[k] = make_uint2((uint32_t)i, __float_as_uint(c.wmax));
-        else G->ok = 0u;
         return;
     }
     for (int v = c.v0; v <= c.v1; ++v)
@@ -252,8 +253,7 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
 
 // First entry of every cell: a scan within the block's cells from one range of the entries per block
 // (cells of different blocks need no order).
-__global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uint2 *cells, uint32_t cells_cap,
-                                                             uint32_t entries_cap) {
+__global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uint2 *cells, uint32_t cells_cap) {
     SunGrid *G = grids + blockIdx.y;
     if (!G->ok) return;
     const uint32_t ncell = (uint32_t)G->nu * (uint32_t)G->nv;
@@ -286,8 +286,7 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uin
             sh[w] = t;
             t += s;
         }
-        first = t ? atomicAdd(&G->total, t) : 0u;
-        if (first + t > entries_cap || first + t < first) G->ok = 0u;
+        first = t ? atomicAdd(&G->total, t) : 0u;  // at most kSunWide entries of 2^25 primitives: no wrap
     }
     __syncthreads();
     uint32_t at = first + sh[warp] + x - sum;
@@ -344,6 +343,11 @@ __global__ void __launch_bounds__(kSunThreads, 4) k_direct_sun(const SunDirectPa
         uint32_t *dst = reinterpret_cast<uint32_t *>(s_grid);
         for (uint32_t i = threadIdx.x; i < (uint32_t)P.nb * (sizeof(SunGrid) / sizeof(uint32_t)); i += kSunThreads)
             dst[i] = src[i];
+        __syncthreads();
+        if (threadIdx.x < (unsigned)P.nb) {
+            SunGrid &g = s_grid[threadIdx.x];
+            g.ok = sun_served(g, P.entries_cap) ? 1u : 0u;
+        }
         __syncthreads();
     }
     unsigned long long nrays = 0;
@@ -448,7 +452,7 @@ cudaError_t launch_direct_sun(const SunDirectParams &p, const float *dirs, int d
     const dim3 gp((unsigned)((n + kSunThreads - 1) / kSunThreads), (unsigned)p.nb);
     k_sun_bin<false><<<gp, kSunThreads, 0, s>>>(n, p.sc.rec, p.grids, p.cells, p.cells_cap, p.entries, p.entries_cap, done);
     const dim3 gc((unsigned)((p.cells_cap + kSunTile - 1) / kSunTile), (unsigned)p.nb);
-    k_sun_offsets<<<gc, kSunThreads, 0, s>>>(p.grids, p.cells, p.cells_cap, p.entries_cap);
+    k_sun_offsets<<<gc, kSunThreads, 0, s>>>(p.grids, p.cells, p.cells_cap);
     k_sun_bin<true><<<gp, kSunThreads, 0, s>>>(n, p.sc.rec, p.grids, p.cells, p.cells_cap, p.entries, p.entries_cap, done);
     SunDirectParams Q = p;
     for (uint32_t at = 0; at < p.count; at += Q.count) {
