@@ -7,6 +7,7 @@
 // sequence of RadiationModel::runBand (src/RadiationModel.cpp:3470-4663)
 // without returning to the host between passes.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -166,6 +167,7 @@ struct hrt_context {
     float px = 0.f, py = 0.f;
     float wall_scale = 0.f;  // TraceScene::wall_scale
     bool have_geometry = false, built = false;
+    uint64_t version = 0;  // of the geometry and its trees, unique among all contexts (new_version)
     std::vector<int8_t> h_twosided;
     std::vector<uint32_t> h_voxels;  // original indices of voxel primitives
     DevBuf T, type, twosided, bbox, rec, rgen, nodes, codes, perm, bvh_scratch, lad, area, nodes4;
@@ -1232,6 +1234,12 @@ int hrt_set_stream(hrt_context *ctx, void *stream) {
     return HRT_OK;
 }
 
+// The next version of a scene.
+static uint64_t new_version() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
+}
+
 int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     if (!ctx || !g) return HRT_EINVAL;
     if (g->n < 0) return fail(ctx, HRT_EINVAL, "negative primitive count");
@@ -1240,6 +1248,7 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     if (!(g->nbbox == 0 || g->nbbox == 2 || g->nbbox == 4) || (g->nbbox > 0 && !g->bbox_vertices))
         return fail(ctx, HRT_EINVAL, "periodic walls must be 0, 2 or 4 quads");
     ctx->cover_key.clear();
+    ctx->version = new_version();
     std::vector<uint32_t> voxels;
     for (int i = 0; i < g->n; ++i) {
         if (g->type[i] > 4) return fail(ctx, HRT_EUNSUPPORTED, "unsupported primitive type " + std::to_string(g->type[i]));
@@ -1360,6 +1369,7 @@ int hrt_build_accel(hrt_context *ctx) {
     if (!ctx) return HRT_EINVAL;
     if (!ctx->have_geometry) return fail(ctx, HRT_EINVAL, "hrt_update_geometry() has not been called");
     CU(cudaSetDevice(ctx->device));
+    ctx->version = new_version();
     int n = ctx->n;
     if (n == 0) {
         ctx->built = true;
@@ -2184,16 +2194,18 @@ int sweep_prepare(hrt_context *ctx, const hrt_sweep *s, bool tune, SweepPlan *pl
     return HRT_OK;
 }
 
-// Shape and buffers of a prepared sweep: a captured graph is valid while these stay the same.
+// Everything that a captured sweep holds by value: shapes, settings, buffers and the scene, whose version
+// stands for its tree, walls and masks.  The graph is valid while these stay the same.
 std::string sweep_key(const SweepPlan &P, const hrt_sweep *s) {
     hrt_context *ctx = P.ctx;
-    char key[384];
-    std::snprintf(key, sizeof key, "%d/%d/%d/%d/%d/%d/%u/%d%d%d%d/%p/%p/%p/%p/%p/%p/%p/v%d/c%u/%u/g%d/%p/%p/%p/%p", P.n, P.nsun, P.Bl,
+    char key[512];
+    std::snprintf(key, sizeof key,
+                  "%d/%d/%d/%d/%d/%d/%u/%d%d%d%d/%p/%p/%p/%p/%p/%p/%p/v%d/c%u/%u/g%d/%p/%p/%p/%p/s%llu/%u/%u", P.n, P.nsun, P.Bl,
                   s->direct_rays, s->diffuse_rays, s->scattering_depth, s->seed, (int)P.any_direct,
                   (int)P.any_diffuse, (int)P.any_copy0, (int)P.any_active, ctx->sw_acc.p, ctx->sw_hits.p,
                   ctx->sw_in.p, ctx->sw_mat.p, ctx->sw_out.p, ctx->Gd.p, (void *)ctx->stream, P.rec_variant,
                   P.rec_per, P.dir_per, P.sun_batch, ctx->sg_cells.p, ctx->sg_entries.p, ctx->sg_grids.p,
-                  ctx->sg_done.p);
+                  ctx->sg_done.p, (unsigned long long)ctx->version, ctx->visit_budget, ctx->lane_budget);
     return key;
 }
 

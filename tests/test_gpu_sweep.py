@@ -158,3 +158,36 @@ def test_multi_scene_sweep_reports_the_failing_scene(bad):
     for a, b, c in zip(after, before, ctxs):
         np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-9)
         assert c.device_status() == 0
+
+
+def test_sweep_follows_a_changed_scene():
+    """A sweep of the same shape after the scene got periodic walls, after the walls moved, after the
+    leaves moved, with another visit budget and without walls again: what a fresh context gives."""
+    from helios_gb300 import _hrt
+
+    sc = scenes.mixed_canopy(1500, 2.0, seed=1)
+    side = float(np.sqrt(1500 * 0.0025 / 2))
+    kw = dict(sun_dir=np.array([[0.6, 0.2, 0.4]]), direct_flux=np.full((1, 1), 500.0), diffuse_flux=np.full((1, 1), 80.0),
+              rho=np.full((sc.n, 1), 0.3), tau=np.full((sc.n, 1), 0.2), direct_rays=64, diffuse_rays=64, depth=1, seed=9)
+
+    def walls(out):
+        z0, z1, a, b = -1.0, 3.2, -0.1 - out, side + 0.1 + out
+        return np.array([[(a, a, z0), (a, b, z0), (a, b, z1), (a, a, z1)], [(b, a, z0), (b, b, z0), (b, b, z1), (b, a, z1)],
+                         [(a, a, z0), (b, a, z0), (b, a, z1), (a, a, z1)], [(a, b, z0), (b, b, z0), (b, b, z1), (a, b, z1)]],
+                        np.float32)
+
+    moved = sc.T.copy()
+    moved[1:, 11] *= 0.5
+    ctx = _hrt.Context(0)
+    for T, bb in ((sc.T, None), (sc.T, walls(0.0)), (sc.T, walls(1.0)), (moved, walls(1.0)), (moved, None)):
+        fresh = _hrt.Context(0)
+        for c in (ctx, fresh):
+            c.update_geometry(T, sc.ptype, sc.twosided, bb, (0.0, 0.0) if bb is None else (1.0, 1.0))
+            c.build_accel()
+        np.testing.assert_allclose(ctx.run_sweep(**kw), fresh.run_sweep(**kw), rtol=1e-6, atol=1e-9)
+        assert ctx.last_stats()["rays"] == fresh.last_stats()["rays"]
+    ctx.set_visit_budget(2)
+    with pytest.raises(_hrt.HrtError, match="visit budget"):
+        ctx.run_sweep(**kw)
+    ctx.set_visit_budget(0)
+    np.testing.assert_allclose(ctx.run_sweep(**kw), fresh.run_sweep(**kw), rtol=1e-6, atol=1e-9)
