@@ -166,6 +166,7 @@ struct hrt_context {
     int n = 0, nbbox = 0;
     float px = 0.f, py = 0.f;
     float wall_scale = 0.f;  // TraceScene::wall_scale
+    float wall_far = 0.f;    // largest coordinate of the walls
     bool have_geometry = false, built = false;
     uint64_t version = 0;  // of the geometry and its trees, unique among all contexts (new_version)
     std::vector<int8_t> h_twosided;
@@ -575,6 +576,7 @@ void fill_sun_params(hrt_context *ctx, SunDirectParams *D) {
     D->entries = ctx->sg_entries.as<uint2>();
     D->cells_cap = caps.cells;
     D->entries_cap = caps.entries;
+    D->wall_far = ctx->wall_far;
 }
 
 // Direct pass + epilogue (__raygen__direct / __miss__direct).
@@ -1280,6 +1282,7 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     // primitive areas (voxels: leaf area) weight the scattering residual
     CU(launch_prim_area((int)n, ctx->T.as<float>(), ctx->type.as<uint32_t>(), ctx->lad.as<float>(),
                         ctx->area.as<double>(), ctx->stream));
+    ctx->wall_far = largest_coordinate(g->bbox_vertices, 12 * (size_t)g->nbbox);
     ctx->have_lattice = ctx->use_lattice = false;
     if (!voxels.empty() && voxels.size() + 2 <= n) {
         float far = 0.f;  // periodic wraps stay within the walls, which hold the scene
@@ -1340,16 +1343,14 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     ctx->wall_scale = 0.f;
     if (g->nbbox) {
         bool planes = g->nbbox == 4 ? (g->periodic_x == 1.f) : true;
-        float scale = 0.f;
         const int nx = g->periodic_x == 1.f ? 2 : 0;
         for (int b = 0; b < g->nbbox; ++b)
             for (int k = 0; k < 4; ++k) {
                 const float *v = g->bbox_vertices + 3 * (4 * b + k), *v0 = g->bbox_vertices + 12 * b;
                 const int a = b < nx ? 0 : 1;
                 planes = planes && v[a] == v0[a];
-                for (int i = 0; i < 3; ++i) scale = std::max(scale, std::fabs(v[i]));
             }
-        if (planes && std::isfinite(scale)) ctx->wall_scale = 2.f * scale;
+        if (planes && std::isfinite(ctx->wall_far)) ctx->wall_scale = 2.f * ctx->wall_far;
     }
     if (g->nbbox) {
         std::vector<float4> q((size_t)g->nbbox * 4);

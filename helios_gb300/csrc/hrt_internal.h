@@ -1,5 +1,6 @@
 // hrt_internal.h -- structures shared by the CUDA translation units of libhrt.
 #pragma once
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -15,6 +16,17 @@ struct VoxGrid {
     float tol, tolf[3];             // closeness to a cell face: a length, and per axis in cells
     const float4 *cells;            // [n0*n1*n2*2] (lo.xyz, extinction), (hi.xyz, original index); extinction 0: empty
 };
+
+// Largest absolute value of `count` coordinates; infinite where one is not a number.
+inline float largest_coordinate(const float *v, size_t count) {
+    float far = 0.f;
+    for (size_t i = 0; i < count; ++i) far = std::isnan(v[i]) ? INFINITY : std::fmax(far, std::fabs(v[i]));
+    return far;
+}
+// Walls farther than this many times the primitives' coordinates: a ray that comes back from one starts
+// where coordinates are too coarse for bounds padded by the scene's, and what such a ray meets depends on
+// the form of the search.  The grids across the suns then give way to the tree.
+constexpr float kWallsFar = 4.f;
 
 // Scene as the trace kernels see it.
 struct TraceScene {
@@ -124,6 +136,7 @@ struct SunDirectParams {
     uint2 *cells;             // [nb * cells_cap] end of the cell's entries, count
     uint2 *entries;           // [nb * entries_cap] record slot, largest depth
     uint32_t cells_cap, entries_cap;
+    float wall_far;           // largest coordinate of the periodic walls (0: none)
     double *G;                // [n*S*2] as DirectParams::G, without the factor 1 / rays of a primitive
 };
 // Scene bounds and extent sums of the records (once per geometry), 9 words.

@@ -16,7 +16,7 @@
 // 200,004-primitive canopy 6.5 -> 1.7 ms, 6.3 M of a periodic stand 5.6 -> 1.1 ms, 2 M of the
 // 20,001-patch canopy 0.69 -> 0.21 ms; 96 suns over a 100 k orchard block 344 -> 121 ms per sweep.
 // A source whose grid would not pay (entries over the buffer, more than kSunLarge primitives that
-// cover over kSunWide cells, a direction that is not finite) is not marked as done on the device and
+// cover over kSunWide cells, a direction that is not finite, walls far beyond the scene) is not marked as done on the device and
 // its rays go through the tree (k_direct / k_direct_sweep skip the sources done here).
 #include "hrt_trace.cuh"
 
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kSunThreads) k_scene_extent(int n, const float
 
 // One thread per source: direction, plane axes, ray set-up and the grid's frame.
 __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stride, const uint32_t *__restrict__ extent,
-                            int n, uint32_t cells_cap, SunGrid *grids) {
+                            int n, uint32_t cells_cap, float wall_far, SunGrid *grids) {
     const int b = threadIdx.x;
     if (b >= nb) return;
     SunGrid g;
@@ -118,9 +118,10 @@ __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stri
         ext = fmaxf(ext, hi[k] - lo[k]);
         far = fmaxf(far, fmaxf(fabsf(lo[k]), fabsf(hi[k])));
     }
-    // The projections round by about 2^-22 of the coordinates, the primitive tests by 2^-22 of the
-    // distances; 2^-19 of both covers them.
-    g.pad = (far + ext) * 1.9073486328125e-06f;
+    // The projections round by about 2^-22 of the coordinates (of a wrapped ray: the walls'), the primitive
+    // tests by 2^-22 of the distances; 2^-19 of both covers them.
+    g.pad = (fmaxf(far, wall_far) + ext) * 1.9073486328125e-06f;
+    const bool near = !(wall_far > kWallsFar * (far + ext));
     const f3 c = mk(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]));
     const f3 half = mk(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]));
     const float hu = fabsf(e1.x) * half.x + fabsf(e1.y) * half.y + fabsf(e1.z) * half.z + 2.f * g.pad;
@@ -140,7 +141,7 @@ __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stri
     int nu = 1, nv = 1;
     const bool fits = sun_cells(hu, hv, cells_cap, &h, &nu, &nv);
     g.inv_h = 1.f / h;
-    const bool fine = fits && g.inv_h > 0.f && isfinite(g.inv_h) && isfinite(g.u0) && isfinite(g.v0);
+    const bool fine = fits && near && g.inv_h > 0.f && isfinite(g.inv_h) && isfinite(g.u0) && isfinite(g.v0);
     g.nu = fine ? nu : 1;
     g.nv = fine ? nv : 1;
     g.ok = fine ? 1u : 0u;
@@ -448,7 +449,7 @@ cudaError_t launch_direct_sun(const SunDirectParams &p, const float *dirs, int d
     if (n <= 0 || p.nb <= 0 || p.nb > kSunBatch) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(p.cells, 0, (size_t)p.nb * p.cells_cap * sizeof(uint2), s);
     if (e != cudaSuccess) return e;
-    k_sun_setup<<<1, kSunBatch, 0, s>>>(p.nb, dirs, dir_stride, extent, n, p.cells_cap, p.grids);
+    k_sun_setup<<<1, kSunBatch, 0, s>>>(p.nb, dirs, dir_stride, extent, n, p.cells_cap, p.wall_far, p.grids);
     const dim3 gp((unsigned)((n + kSunThreads - 1) / kSunThreads), (unsigned)p.nb);
     k_sun_bin<false><<<gp, kSunThreads, 0, s>>>(n, p.sc.rec, p.grids, p.cells, p.cells_cap, p.entries, p.entries_cap, done);
     const dim3 gc((unsigned)((p.cells_cap + kSunTile - 1) / kSunTile), (unsigned)p.nb);

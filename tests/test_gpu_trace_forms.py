@@ -308,3 +308,28 @@ def test_trees_of_all_sizes_hit_what_the_binary_tree_hits(gpu, n, spread):
     gpu.set_tuning(1)
     assert gpu.last_stats()["rays"] == rays and gpu.device_status() == 0
     assert np.all(np.abs(wide - binary) <= 2.4e-7 * np.abs(binary))
+
+
+@pytest.mark.parametrize("scale", [1.0, 6.0, 4.0e4])
+def test_binned_shadow_rays_from_far_walls(hrt_lib, scale):
+    """A horizontal sun through periodic walls as wide as the scene, several times and 40,000 times wider
+    (where the tree serves the sun): rays that come back from a wall start where coordinates are
+    coarser, and find what the tree finds.  Leaves face the sun, so that many end at the edges of cells."""
+    rng = np.random.default_rng(3)
+    n, sun = 3000, np.array([0.6, 0.8, 0.0])
+    T = scenes.frame_T(rng.uniform(0.0, 1.7, (n, 3)), np.full(n, 0.05), np.full(n, 0.05), np.tile(sun, (n, 1)), np.zeros(n))
+    h, z = 2.0 * scale, 3.0
+    walls = np.array([[(-h, -h, -z), (-h, h, -z), (-h, h, z), (-h, -h, z)], [(h, -h, -z), (h, h, -z), (h, h, z), (h, -h, z)],
+                      [(-h, -h, -z), (h, -h, -z), (h, -h, z), (-h, -h, z)], [(-h, h, -z), (h, h, -z), (h, h, z), (-h, h, z)]],
+                     np.float32)
+    c = _hrt.Context(0)
+    c.update_geometry(T, np.zeros(n, np.uint32), np.ones(n, np.int8), walls, (1.0, 1.0))
+    c.build_accel()
+    d = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 0, "position": tuple(sun)}],
+         "source_flux": np.array([[100.0]]), "rho": np.zeros((1, n, 1)), "tau": np.zeros((1, n, 1)),
+         "diffuse_flux": np.array([0.0]), "direct_rays": np.array([400]), "diffuse_rays": np.array([1]),
+         "depth": np.array([0]), "emission": np.array([0], np.uint8), "seed": 3}
+    binned = c.run_band(d).astype(np.float64)
+    c.set_visit_budget(1 << 30)
+    tree = c.run_band(d).astype(np.float64)
+    assert np.all(np.abs(binned - tree) <= 2.4e-7 * np.abs(tree))
