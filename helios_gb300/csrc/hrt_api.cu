@@ -1285,12 +1285,12 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     ctx->wall_far = largest_coordinate(g->bbox_vertices, 12 * (size_t)g->nbbox);
     ctx->have_lattice = ctx->use_lattice = false;
     if (!voxels.empty() && voxels.size() + 2 <= n) {
-        float far = 0.f;  // periodic wraps stay within the walls, which hold the scene
-        for (size_t i = 0; i < n; ++i)
-            for (int a = 0; a < 3; ++a) far = std::max(far, std::fabs(g->transform[16 * i + 4 * a + 3]));
+        // rays start on primitives and, wrapped, on the walls
+        const float reach = primitives_reach(g->transform, n);
         std::vector<float4> cells;
         VoxGrid vg{};
-        if (find_lattice(g->transform, voxels, g->voxel_lad, far, &vg, &cells)) {
+        if (!(ctx->wall_far > kWallsFar * reach) &&
+            find_lattice(g->transform, voxels, g->voxel_lad, std::max(reach, ctx->wall_far), &vg, &cells)) {
             CU(ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4)));
             CU(ctx->vg.ensure(ctx->stream, sizeof(VoxGrid)));
             vg.cells = ctx->vg_cells.as<float4>();

@@ -23,9 +23,21 @@ inline float largest_coordinate(const float *v, size_t count) {
     for (size_t i = 0; i < count; ++i) far = std::isnan(v[i]) ? INFINITY : std::fmax(far, std::fabs(v[i]));
     return far;
 }
+// A bound on the coordinates of n primitives: of an affine image of the cube [-1, 1]^3, which holds every
+// primitive's canonical form.
+inline float primitives_reach(const float *T, size_t n) {
+    float far = 0.f;
+    for (size_t i = 0; i < n; ++i)
+        for (int a = 0; a < 3; ++a) {
+            const float *t = T + 16 * i + 4 * a;
+            const float r = std::fabs(t[0]) + std::fabs(t[1]) + std::fabs(t[2]) + std::fabs(t[3]);
+            far = std::isnan(r) ? INFINITY : std::fmax(far, r);
+        }
+    return far;
+}
 // Walls farther than this many times the primitives' coordinates: a ray that comes back from one starts
 // where coordinates are too coarse for bounds padded by the scene's, and what such a ray meets depends on
-// the form of the search.  The grids across the suns then give way to the tree.
+// the form of the search.  The grids across the suns and the march of a lattice then give way to the tree.
 constexpr float kWallsFar = 4.f;
 
 // Scene as the trace kernels see it.

@@ -1,5 +1,5 @@
-"""Cell counts of the grids across collimated sources (hrt_device.cuh sun_cells): the shipped header
-compiled for the host; a grid never has more cells than its buffer."""
+"""Host checks of the shipped headers: a grid across a collimated source never has more cells than its
+buffer (sun_cells), and the bounds on ray origins hold the primitives' edges and the walls."""
 import os
 import subprocess
 
@@ -11,9 +11,10 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.skipif(_nvcc() is None, reason="nvcc not available")
-def test_grid_cells_fit_their_buffer(tmp_path):
-    exe = str(tmp_path / "suncells_check")
-    src = os.path.join(ROOT, "tests", "cpp", "suncells_check.cu")
+@pytest.mark.parametrize("check", ["suncells", "reach"])
+def test_host_check(tmp_path, check):
+    exe = str(tmp_path / check)
+    src = os.path.join(ROOT, "tests", "cpp", check + "_check.cu")
     r = subprocess.run([_nvcc(), "-O2", "-std=c++17", "-I" + os.path.join(ROOT, "helios_gb300", "csrc"), src, "-o", exe],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
