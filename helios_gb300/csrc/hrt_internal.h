@@ -121,6 +121,17 @@ constexpr int kSunWide = 64;
 // with it and 50 us through the tree, 0.25 M of 2,501 primitives 65 and 95 us.
 constexpr unsigned long long kSunMinRays = 200000;
 constexpr float kSunCell = 0.6f; // cell side in halves of the mean box extent
+// Entries of the cell of a mean entry (sum of squared counts over their sum) from which the tree serves a
+// source: a ray scans its cell from end to end, and one plant on a wide ground has its leaves in a few
+// cells.  Grid and tree, ms of 100 rays a leaf (1 M leaves: 25) under a vertical sun, at the mean given:
+// 5,000 leaves 0.27 and 0.33 at 85, 0.39 and 0.33 at 177; 20,000 0.43 and 0.83 at 31, 0.77 and 0.84 at 79,
+// 1.63 and 0.84 at 195; 100,000 2.6 and 4.4 at 69, 4.0 and 4.4 at 118, 11.5 and 4.4 at 374; 200,000
+// 9.7 and 9.9 just below 192; 1 M 9.6 and 18.8 at 97, 17.9 and 19.1 at 231 (a large tree misses the caches).  Uniform canopies have 3-30, at a
+// leaf area index of 5 up to 84.  A source that is dropped has cost its counting: 40-50 us with 5,000 and
+// 20,000 leaves, 0.1 ms with 100,000, 0.3 ms with 1 M.
+__host__ __device__ inline unsigned long long sun_crowd(int n) {
+    return n < (96 << 10) ? 96ull : (n > (192 << 10) ? 192ull : (unsigned long long)(n >> 10));
+}
 struct SunGrid {
     f3 s, e1, e2;          // direction toward the source, plane axes
     f3 inv;                // the rays' inverse direction and watertight-test set-up
@@ -129,6 +140,7 @@ struct SunGrid {
     float u0, v0, inv_h, pad;
     int nu, nv;
     uint32_t total;        // entries
+    unsigned long long sq; // sum over the cells of their squared counts
     uint32_t ok;           // 0: no frame; the source's rays go through the tree
     uint32_t nlarge;
     uint2 large[kSunLarge];

@@ -16,7 +16,7 @@
 // 200,004-primitive canopy 6.5 -> 1.7 ms, 6.3 M of a periodic stand 5.6 -> 1.1 ms, 2 M of the
 // 20,001-patch canopy 0.69 -> 0.21 ms; 96 suns over a 100 k orchard block 344 -> 121 ms per sweep.
 // A source whose grid would not pay (entries over the buffer, more than kSunLarge primitives that
-// cover over kSunWide cells, a direction that is not finite, walls far beyond the scene) is not marked as done on the device and
+// cover over kSunWide cells, a direction that is not finite, walls far beyond the scene, crowded cells) is not marked as done on the device and
 // its rays go through the tree (k_direct / k_direct_sweep skip the sources done here).
 #include "hrt_trace.cuh"
 
@@ -146,14 +146,16 @@ __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stri
     g.nv = fine ? nv : 1;
     g.ok = fine ? 1u : 0u;
     g.total = 0u;
+    g.sq = 0ull;
     g.nlarge = 0u;
     grids[b] = g;
 }
 
-// Whether a binned source is traced by its grid: its entries fit and few primitives are wide.  The
+// Whether a binned source is traced by its grid: its entries fit, few primitives are wide and the cells
+// are not crowded.  The
 // flag of the frame is written once, by k_sun_setup, so that all threads of a block agree on it.
-__device__ __forceinline__ bool sun_served(const SunGrid &g, uint32_t entries_cap) {
-    return g.ok && g.nlarge <= (uint32_t)kSunLarge && g.total <= entries_cap;
+__device__ __forceinline__ bool sun_served(const SunGrid &g, uint32_t entries_cap, int n) {
+    return g.ok && g.nlarge <= (uint32_t)kSunLarge && g.total <= entries_cap && g.sq <= sun_crowd(n) * g.total;
 }
 
 struct CellRect {
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
                                                          uint32_t entries_cap, uint32_t *done) {
     SunGrid *G = grids + blockIdx.y;
     const SunGrid &g = *G;
-    const bool on = FILL ? sun_served(g, entries_cap) : g.ok != 0u;
+    const bool on = FILL ? sun_served(g, entries_cap, n) : g.ok != 0u;
     if (FILL && blockIdx.x == 0 && threadIdx.x == 0) done[blockIdx.y] = on ? 1u : 0u;
     if (!on) return;
     uint2 *cl = cells + (size_t)blockIdx.y * cells_cap;
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
         }
 }
 
-// First entry of every cell: a scan within the block's cells from one range of the entries per block
+// First entry of every cell and the sum of squared counts: a scan within the block's cells from one range of the entries per block
 // (cells of different blocks need no order).
 __global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uint2 *cells, uint32_t cells_cap) {
     SunGrid *G = grids + blockIdx.y;
@@ -263,12 +265,17 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uin
     uint2 *cl = cells + (size_t)blockIdx.y * cells_cap;
     constexpr int kPer = kSunTile / kSunThreads;
     uint32_t v[kPer], sum = 0;
+    unsigned long long sq = 0;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
         const uint32_t i = base + threadIdx.x * kPer + j;
         v[j] = i < ncell ? cl[i].y : 0u;
         sum += v[j];
+        sq += (unsigned long long)v[j] * v[j];
     }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, d);
+    if ((threadIdx.x & 31) == 0 && sq) atomicAdd(&G->sq, sq);
     __shared__ uint32_t sh[kSunThreads / 32];
     __shared__ uint32_t first;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -347,7 +354,7 @@ __global__ void __launch_bounds__(kSunThreads, 4) k_direct_sun(const SunDirectPa
         __syncthreads();
         if (threadIdx.x < (unsigned)P.nb) {
             SunGrid &g = s_grid[threadIdx.x];
-            g.ok = sun_served(g, P.entries_cap) ? 1u : 0u;
+            g.ok = sun_served(g, P.entries_cap, P.sc.n) ? 1u : 0u;
         }
         __syncthreads();
     }

@@ -333,3 +333,44 @@ def test_binned_shadow_rays_from_far_walls(hrt_lib, scale):
     c.set_visit_budget(1 << 30)
     tree = c.run_band(d).astype(np.float64)
     assert np.all(np.abs(binned - tree) <= 2.4e-7 * np.abs(tree))
+
+
+def _direct_ms(c, d, k=7):
+    import time
+
+    c.run_band(d, out=False)
+    t = []
+    for _ in range(k):
+        a = time.perf_counter()
+        c.run_band(d, out=False)
+        t.append(time.perf_counter() - a)
+    return 1e3 * sorted(t)[k // 2]
+
+
+@pytest.mark.parametrize("ground", [0.0, 50.0, 400.0, 5000.0])
+def test_shadow_rays_of_clumped_leaves(hrt_lib, ground):
+    """One plant of 20,000 leaves alone and on ever wider grounds, where the cells of a sun's grid hold
+    hundreds or thousands of leaves: same fluxes as through the tree and not much slower than it."""
+    rng = np.random.default_rng(0)
+    n = 20000
+    at = scenes.uniform_sphere(rng, n) * (rng.uniform(0, 1, n) ** (1 / 3))[:, None] * 1.25
+    at[:, 2] += 1.75
+    T = scenes.frame_T(at, np.full(n, 0.03), np.full(n, 0.03), scenes.uniform_sphere(rng, n), rng.uniform(0, 6, n))
+    if ground:
+        one = np.ones(1)
+        T = np.concatenate([scenes.frame_T(np.zeros((1, 3)), ground * one, ground * one, np.array([[0.0, 0.0, 1.0]]), 0 * one), T])
+    n = T.shape[0]
+    c = _hrt.Context(0)
+    c.update_geometry(T, np.zeros(n, np.uint32), np.ones(n, np.int8))
+    c.build_accel()
+    for sun in ((0.0, 0.0, 1.0), (0.6, 0.3, 0.5)):
+        d = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 0, "position": sun}], "source_flux": np.array([[100.0]]),
+             "rho": np.zeros((1, n, 1)), "tau": np.zeros((1, n, 1)), "diffuse_flux": np.array([0.0]),
+             "direct_rays": np.array([100]), "diffuse_rays": np.array([1]), "depth": np.array([0]),
+             "emission": np.array([0], np.uint8), "seed": 3}
+        got, ms = c.run_band(d).astype(np.float64), _direct_ms(c, d)
+        c.set_visit_budget(1 << 30)
+        tree, tree_ms = c.run_band(d).astype(np.float64), _direct_ms(c, d)
+        c.set_visit_budget(0)
+        assert np.all(np.abs(got - tree) <= 2.4e-7 * np.abs(tree))
+        assert ms <= 1.5 * tree_ms, (sun, ms, tree_ms)
