@@ -566,7 +566,7 @@ int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
 // Whether a direct pass of `rays` rays per source bins its collimated sources (hrt_sungrid.cu).
 // Statistics launches count the tree's visits and a lowered visit budget is meant for the tree.
 bool sun_grids_pay(hrt_context *ctx, unsigned long long rays) {
-    return !(ctx->measure & 1) && ctx->visit_budget == 0 && rays >= kSunMinRays;
+    return !(ctx->measure & 1) && ctx->visit_budget == 0 && rays >= kSunMinRays && rays >= (unsigned long long)ctx->n;
 }
 
 void fill_sun_params(hrt_context *ctx, SunDirectParams *D) {

@@ -118,7 +118,10 @@ constexpr int kSunBatch = 32;    // sources binned and traced together
 constexpr int kSunLarge = 32;    // primitives over kSunWide cells, which every ray tests
 constexpr int kSunWide = 64;
 // Rays per source from which the binning pays: 0.1 M rays of the 1,001-primitive canopy take 53 us
-// with it and 50 us through the tree, 0.25 M of 2,501 primitives 65 and 95 us.
+// with it and 50 us through the tree, 0.25 M of 2,501 primitives 65 and 95 us.  A range of a large scene
+// also needs a ray per primitive of the whole, since all are binned: of 1 M primitives, 0.25 M rays of a
+// range take 246 and 168 us, 0.5 M 255 and 243, 1 M 268 and 357; whole scenes at one ray each 0.34 and
+// 0.40 ms with 200,000 primitives, 1.0 and 1.25 with 1 M, 3.9 and 5.7 with 4 M.
 constexpr unsigned long long kSunMinRays = 200000;
 constexpr float kSunCell = 0.6f; // cell side in halves of the mean box extent
 // Entries of the cell of a mean entry (sum of squared counts over their sum) from which the tree serves a

@@ -374,3 +374,26 @@ def test_shadow_rays_of_clumped_leaves(hrt_lib, ground):
         c.set_visit_budget(0)
         assert np.all(np.abs(got - tree) <= 2.4e-7 * np.abs(tree))
         assert ms <= 1.5 * tree_ms, (sun, ms, tree_ms)
+
+
+def test_direct_range_of_a_large_scene(hrt_lib):
+    """A range with fewer rays than the scene has primitives is not worth binning them all: it makes the
+    launches that it makes through the tree, and a range with more rays makes the grid's."""
+    sc = scenes.mixed_canopy(300000, 2.0, seed=1)
+    c = _hrt.Context(0)
+    c.update_geometry(sc.T, sc.ptype, sc.twosided)
+    c.build_accel()
+    c.update_materials(np.zeros((1, sc.n, 1)), np.zeros((1, sc.n, 1)), 1, 1)
+    c.update_sources([{"type": 0, "position": (0.3, 0.2, 0.9)}])
+    c.zero_radiation_buffers(1)
+    c.upload_source_fluxes([100.0])
+
+    def launches(count):
+        before = c.last_stats()["kernels"]
+        c.launch_direct(launch_offset=5, launch_count=count, rays_per_primitive=25, random_seed=3, pass_id=0, nbands_global=1,
+                        nbands_launch=1, band_launch_flag=np.ones(1, np.uint8))
+        return c.last_stats()["kernels"] - before
+
+    few, many = launches(10000), launches(20000)
+    c.set_visit_budget(1 << 30)
+    assert few == launches(10000) and many > launches(20000)
