@@ -191,3 +191,35 @@ def test_sweep_follows_a_changed_scene():
         ctx.run_sweep(**kw)
     ctx.set_visit_budget(0)
     np.testing.assert_allclose(ctx.run_sweep(**kw), fresh.run_sweep(**kw), rtol=1e-6, atol=1e-9)
+
+
+def _median_ms(f, k=9):
+    import time
+
+    f()
+    t = []
+    for _ in range(k):
+        a = time.perf_counter()
+        f()
+        t.append(time.perf_counter() - a)
+    return 1e3 * sorted(t)[k // 2]
+
+
+def test_suns_of_a_small_scene_run_together():
+    """The shadow rays of 192 suns over 50 primitives, 1 M in all, fill the device together: no longer
+    than one sun over 192 times the primitives, whose rays wander through a larger tree."""
+    from helios_gb300 import _hrt
+
+    ms = []
+    for n, suns in ((50, 192), (9600, 1)):
+        sc = scenes.mixed_canopy(n, 2.0, seed=1)
+        c = _hrt.Context(0)
+        c.update_geometry(sc.T, sc.ptype, sc.twosided)
+        c.build_accel()
+        d = scenes.uniform_sphere(np.random.default_rng(1), suns)
+        d[:, 2] = np.abs(d[:, 2]) + 0.1
+        kw = dict(sun_dir=d, direct_flux=np.full((suns, 1), 500.0), diffuse_flux=np.zeros((suns, 1)), rho=np.zeros((sc.n, 1)),
+                  tau=np.zeros((sc.n, 1)), direct_rays=100, diffuse_rays=4, depth=0, seed=9)
+        c.set_visit_budget(1 << 30)  # through the tree
+        ms.append(_median_ms(lambda: c.run_sweep(**kw, out=False)))
+    assert ms[0] <= ms[1], ms
