@@ -194,6 +194,7 @@ struct hrt_context {
     // (ordered bounds and extent sums of the records, once per geometry)
     DevBuf sg_cells, sg_entries, sg_grids, sg_extent, sg_done;
     bool sg_extent_ready = false;
+    size_t sg_limit = SIZE_MAX;  // bytes that the cells and entries may take (limit_sun_grids)
     std::vector<int> h_src_type;
     DevBuf io_a, io_b, io_c;  // staging for inspection calls
     uint64_t last_rays = 0, last_kernels = 0, last_iters = 0;
@@ -538,11 +539,12 @@ GlassParams glass_params(hrt_context *ctx, int Bg, int Bl) {
 }
 
 // Buffers of the grids of `nsrc` collimated sources and the scene's extent (queued on the context's
-// stream); *nb: sources per batch, 0 where the device has no memory left for them (the rays then go
-// through the tree, which needs none).
+// stream); *nb: sources per batch, 0 where the context's limit or the device leaves no memory for them
+// (the rays then go through the tree, which needs none).
 int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
     const SunCaps caps = sun_caps(ctx->n);
-    *nb = std::max(1, std::min(caps.batch, nsrc));
+    *nb = (int)std::min<size_t>(std::max(1, std::min(caps.batch, nsrc)), ctx->sg_limit / sun_grid_bytes(ctx->n, 1));
+    if (*nb == 0) return HRT_OK;
     cudaError_t e = ctx->sg_cells.ensure(ctx->stream, (size_t)*nb * caps.cells * sizeof(uint2));
     if (e == cudaSuccess) e = ctx->sg_entries.ensure(ctx->stream, (size_t)*nb * caps.entries * sizeof(uint2));
     if (e == cudaErrorMemoryAllocation) {
@@ -1158,6 +1160,13 @@ int set_source_fluxes(hrt_context *ctx, const float *fluxes, size_t count, bool 
 }
 
 }  // namespace
+
+void hrt::limit_sun_grids(hrt_context *ctx, size_t bytes) {
+    ctx->sg_limit = bytes;
+    if (ctx->sg_cells.cap + ctx->sg_entries.cap <= bytes || cudaSetDevice(ctx->device) != cudaSuccess) return;
+    ctx->sg_cells.free_on(ctx->stream);
+    ctx->sg_entries.free_on(ctx->stream);
+}
 
 // ============================================================== C ABI ===
 extern "C" {

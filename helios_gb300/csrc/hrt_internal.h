@@ -7,6 +7,8 @@
 
 #include "hrt_device.cuh"
 
+struct hrt_context;
+
 namespace hrt {
 
 // Voxels that are cells of one lattice (hrt_voxgrid.cuh).
@@ -153,6 +155,10 @@ struct SunCaps {
     int batch;                // sources per batch
 };
 SunCaps sun_caps(int n);
+// Bytes of the grids of `nsrc` sources, and the most that a context may hold of them (default: what they
+// take; buffers above it are released; 0: suns go through the tree).  The context must be idle.
+size_t sun_grid_bytes(int n, int nsrc);
+void limit_sun_grids(hrt_context *ctx, size_t bytes);
 struct SunDirectParams {
     TraceScene sc;
     int dimx, dimy;

@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/hrt.h"
+#include "hrt_internal.h"
 
 namespace {
 
@@ -60,6 +61,7 @@ struct Scene {
     cudaStream_t stream = nullptr;  // priority stream of this scene's solves
     bool busy = false;
     size_t bytes = 0;
+    size_t grids = 0;  // granted to the grids of its suns, out of memory that no scene needs
     uint64_t last_use = 0;
 };
 
@@ -102,11 +104,12 @@ struct Request {
 };
 
 // Device bytes of a resident scene solved with Bl bands (records, binary and 4-wide BVH,
-// origins, transforms, areas, radiation buffers, BVH scratch).
+// origins, transforms, areas, radiation buffers, BVH scratch).  The grids of its suns are not in it: a
+// solve does without them, and grant_grids gives them what is left of the budget.
 size_t footprint(int32_t n, int32_t Bl) {
     size_t nn = (size_t)std::max(n, 1);
     return nn * (64 + 64 + 64 + 64 + 64 + 8 + 1) + nn * (size_t)std::max(Bl, 1) * (7 * 8 + 3 * 4) + nn * 200 +
-           nn * 192 + (8u << 20);  // 192: the grid of one sun (hrt_sungrid.cu)
+           (8u << 20);
 }
 
 }  // namespace
@@ -114,6 +117,7 @@ size_t footprint(int32_t n, int32_t Bl) {
 struct hrt_server {
     int device = 0;
     size_t budget = 0, used = 0;
+    size_t grids = 0;  // granted to grids of suns; used + grids <= budget
     std::mutex mu;
     std::condition_variable cv_dispatch, cv_work, cv_done;
     std::map<uint32_t, std::unique_ptr<Scene>> scenes;
@@ -141,11 +145,18 @@ bool ensure_resident(hrt_server *s, Scene *sc, int32_t Bl, std::string &err) {
     size_t need = footprint(sc->n, Bl);
     if (sc->ctx && need <= sc->bytes) return true;
     size_t extra = need - (sc->ctx ? sc->bytes : 0);
-    while (s->used + extra > s->budget) {
-        Scene *victim = nullptr;
+    while (s->used + s->grids + extra > s->budget) {
+        Scene *victim = nullptr, *lender = nullptr;
         for (auto &kv : s->scenes) {
             Scene *c = kv.second.get();
+            if (c->ctx && !c->busy && c->grids && (!lender || c->last_use < lender->last_use)) lender = c;
             if (c != sc && c->ctx && !c->busy && (!victim || c->last_use < victim->last_use)) victim = c;
+        }
+        if (lender) {  // grids first: no scene is evicted for them
+            hrt::limit_sun_grids(lender->ctx, 0);
+            s->grids -= lender->grids;
+            lender->grids = 0;
+            continue;
         }
         if (!victim) return false;  // wait for a busy scene to finish
         hrt_destroy(victim->ctx);
@@ -163,6 +174,18 @@ bool ensure_resident(hrt_server *s, Scene *sc, int32_t Bl, std::string &err) {
     sc->bytes = need;
     (void)err;
     return true;
+}
+
+// Lets the context of a busy scene hold grids for the batch's suns as far as the budget has room.
+void grant_grids(hrt_server *s, Scene *sc, const std::vector<Request *> &batch) {
+    if ((double)sc->n * (double)batch[0]->direct_rays < (double)hrt::kSunMinRays) return;  // too few rays for grids
+    std::lock_guard<std::mutex> lk(s->mu);
+    const size_t want = hrt::sun_grid_bytes(sc->n, (int)batch.size());
+    const size_t spare = s->budget - std::min(s->budget, s->used + s->grids);
+    const size_t more = want > sc->grids ? std::min(want - sc->grids, spare) : 0;
+    sc->grids += more;
+    s->grids += more;
+    hrt::limit_sun_grids(sc->ctx, sc->grids);
 }
 
 bool same_batch(const Request *a, const Request *b) {
@@ -369,6 +392,7 @@ void worker_loop(hrt_server *s) {
         for (Scene *sc : scs)
             if (rc == HRT_OK) rc = prepare_scene(s, sc);
         if (rc == HRT_OK && item.size() > 1) {
+            for (size_t i = 0; i < scs.size(); ++i) grant_grids(s, scs[i], item[i]);
             rc = solve_group(scs, item);
         } else if (rc == HRT_OK) {
             Scene *sc = scs[0];
@@ -395,6 +419,7 @@ void worker_loop(hrt_server *s) {
                     }
                 }
             }
+            grant_grids(s, sc, batch);
             rc = batch.size() == 1 ? solve_one(sc, batch[0], Bl) : solve_batch(sc, batch);
         }
         {

@@ -450,6 +450,12 @@ SunCaps sun_caps(int n) {
     return c;
 }
 
+size_t sun_grid_bytes(int n, int nsrc) {
+    const SunCaps c = sun_caps(n);
+    const int nb = nsrc < 1 ? 1 : (nsrc < c.batch ? nsrc : c.batch);
+    return (size_t)nb * ((size_t)c.cells + c.entries) * sizeof(uint2);
+}
+
 cudaError_t launch_direct_sun(const SunDirectParams &p, const float *dirs, int dir_stride, const uint32_t *extent,
                               uint32_t *done, bool shared, uint32_t chunk, int max_blocks, cudaStream_t s) {
     const int n = p.sc.n;

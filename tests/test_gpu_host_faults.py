@@ -27,6 +27,16 @@ def fake_lib_path(hrt_lib, tmp_path_factory):
     return out
 
 
+@pytest.fixture
+def fakes(fake_lib_path, monkeypatch):
+    monkeypatch.setattr(_hrt, "_lib", None)
+    lib = _hrt.load(fake_lib_path)
+    lib.fake_fail_allocations.argtypes = [_hrt.C.c_size_t, _hrt.C.c_size_t]
+    yield lib
+    lib.fake_fail_allocations(0, 0)
+    lib.fake_late_copies(0)
+
+
 def _solve(n, sources, nb=1, **k):
     S = len(sources)
     d = {"band_launch": np.ones(nb, np.uint8), "sources": sources, "source_flux": np.full((S, nb), 300.0),
@@ -44,6 +54,29 @@ def _voxel_context():
                       np.concatenate([leaves.twosided, vox.twosided]), None, (0.0, 0.0),
                       np.concatenate([np.zeros(leaves.n), vox.lad]))
     return c, leaves.n
+
+
+@pytest.mark.parametrize("spare", [0, 1 << 30])
+def test_server_grids_take_what_the_budget_leaves(fakes, spare):
+    """With a budget of just the scene's footprint the server makes no grids of its suns, and with room it
+    does (their allocation fails here, which changes nothing): the fluxes are those of the scene alone."""
+    sc = scenes.mixed_canopy(4000, 2.0, seed=1)
+    n = sc.n
+    sun = (0.3, 0.2, 0.9)
+    c = _hrt.Context(0)
+    c.update_geometry(sc.T, sc.ptype, sc.twosided)
+    c.build_accel()
+    want = c.run_band(_solve(n, [{"type": 0, "position": sun}], direct_rays=np.array([100]))).astype(np.float64)
+    fakes.fake_fail_allocations(8 * 16 * n, 0)  # the entries of one sun
+    srv = _hrt.Server(device=0, workers=1, hbm_budget=n * (529 + 68) + (8 << 20) + spare)
+    srv.add_scene(0, sc.T, sc.ptype, sc.twosided, np.full((n, 1), 0.3), np.full((n, 1), 0.2))
+    srv.submit(0, 0, 0.0, [1], sun, [300.0], [100.0], 100, 64, 1, 3, keep=True)
+    srv.start()
+    srv.wait()
+    got = srv.result(0, n)["flux"].reshape(n, 1).astype(np.float64)
+    srv.close()
+    assert (fakes.fake_failed() > 0) == (spare > 0)
+    assert np.all(np.abs(got - want) <= 1e-5 * np.maximum(np.abs(want), 1e-3 * np.abs(want).mean()))
 
 
 LATE = """
