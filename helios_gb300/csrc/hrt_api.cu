@@ -15,6 +15,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1298,14 +1299,24 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
         const float reach = primitives_reach(g->transform, n);
         std::vector<float4> cells;
         VoxGrid vg{};
-        if (!(ctx->wall_far > kWallsFar * reach) &&
-            find_lattice(g->transform, voxels, g->voxel_lad, std::max(reach, ctx->wall_far), &vg, &cells)) {
-            CU(ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4)));
-            CU(ctx->vg.ensure(ctx->stream, sizeof(VoxGrid)));
-            vg.cells = ctx->vg_cells.as<float4>();
-            CU(upload_local(ctx, ctx->vg_cells.p, std::move(cells)));
-            CU(upload_local(ctx, ctx->vg.p, std::vector<VoxGrid>{vg}));
-            ctx->have_lattice = true;
+        // without memory for the cells, here or on the device, the voxels stay leaves of the tree
+        try {
+            ctx->have_lattice = !(ctx->wall_far > kWallsFar * reach) &&
+                                find_lattice(g->transform, voxels, g->voxel_lad, std::max(reach, ctx->wall_far), &vg, &cells);
+        } catch (const std::bad_alloc &) {
+        }
+        if (ctx->have_lattice) {
+            const cudaError_t e = ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4));
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                ctx->have_lattice = false;
+            } else {
+                CU(e);
+                CU(ctx->vg.ensure(ctx->stream, sizeof(VoxGrid)));
+                vg.cells = ctx->vg_cells.as<float4>();
+                CU(upload_local(ctx, ctx->vg_cells.p, std::move(cells)));
+                CU(upload_local(ctx, ctx->vg.p, std::vector<VoxGrid>{vg}));
+            }
         }
     }
     ctx->h_voxels.swap(voxels);

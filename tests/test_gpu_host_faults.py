@@ -56,6 +56,27 @@ def _voxel_context():
     return c, leaves.n
 
 
+@pytest.mark.parametrize("what", ["cells", "second tree", "sun cells", "sun entries"])
+def test_optional_buffers_without_memory(fakes, what):
+    """Buffers that a call can do without: the cells of a voxel lattice, the tree of the surfaces beside
+    it, and the grids of a direct pass.  Without memory for them the call gives the same fluxes."""
+    c, ns = _voxel_context()
+    c.build_accel()
+    n = c.n
+    d = _solve(n, [{"type": 0, "position": (0.3, 0.2, 0.9)}])
+    want = c.run_band(d).astype(np.float64)
+    size = {"cells": 2 * 16 * 6 * 5 * 4, "second tree": 64 * (ns - 1 + 8), "sun cells": 8 * 8 * n, "sun entries": 8 * 16 * n}
+    sun = what.startswith("sun")  # cells are as large as the transforms: fail them from the solve on
+    fakes.fake_fail_allocations(0 if sun else size[what], 0)
+    c, _ = _voxel_context()
+    c.build_accel()
+    failed = fakes.fake_failed()
+    fakes.fake_fail_allocations(size[what] if sun else 0, 0)
+    got = c.run_band(d).astype(np.float64)
+    assert failed + fakes.fake_failed() > 0
+    assert np.all(np.abs(got - want) <= 2.4e-7 * np.abs(want))
+
+
 @pytest.mark.parametrize("spare", [0, 1 << 30])
 def test_server_grids_take_what_the_budget_leaves(fakes, spare):
     """With a budget of just the scene's footprint the server makes no grids of its suns, and with room it
