@@ -41,7 +41,10 @@ constexpr int32_t kMore = kSentinel + 2;
 template <int SD, int BLOCK>
 struct LaneStack {
     uint32_t base, top;         // shared addresses: entry 0, and the next free entry
-    int32_t spill[kStack4 + 1]; // [0] entries held (while entry 0 is kMore), then the entries
+    // Entries move in blocks, so local memory has room for the shared ones besides kStack4 more: a ray
+    // whose stack fitted in both together still does.
+    static constexpr int kSpill = kStack4 + SD;
+    int32_t spill[kSpill + 1];  // [0] entries held (while entry 0 is kMore), then the entries
     static constexpr uint32_t kStep = 4u * BLOCK, kFull = (uint32_t)SD * kStep;
     __device__ __forceinline__ static void put(uint32_t at, int32_t v) {
         asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(v));
@@ -78,7 +81,7 @@ struct LaneStack {
     __device__ __noinline__ bool spill_out() {
         int held = take(base) == kMore ? spill[0] : 0;
         const int n = (int)((top - base) / kStep) - 1;
-        if (held + n > kStack4) return false;
+        if (held + n > kSpill) return false;
         for (int i = 0; i < n; ++i) spill[1 + held + i] = take(base + kStep * (uint32_t)(1 + i));
         spill[0] = held + n;
         put(base, kMore);

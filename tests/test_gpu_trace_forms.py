@@ -397,3 +397,31 @@ def test_direct_range_of_a_large_scene(hrt_lib):
     few, many = launches(10000), launches(20000)
     c.set_visit_budget(1 << 30)
     assert few == launches(10000) and many > launches(20000)
+
+
+@pytest.mark.parametrize("variant,n", [(6, 133), (8, 140), (8, 144), (13, 151), (13, 159)])
+def test_deep_stacks_that_fit(hrt_lib, oracle_mod, variant, n):
+    """Coincident patches make a chain of nodes whose children are all pushed.  As deep as the stacks in
+    shared and local memory together, each lean shape gives the oracle's fluxes and no error."""
+    from helpers import oracle_solve
+
+    T = np.concatenate([np.tile(scenes.frame_T(np.full((1, 3), 0.5), np.array([0.1]), np.array([0.1]), np.array([[0.0, 0.0, 1.0]]),
+                                               np.zeros(1)), (n, 1)),
+                        scenes.frame_T(np.array([[0.5, 0.5, 0.3]]), np.array([0.3]), np.array([0.3]), np.array([[0.0, 0.0, 1.0]]),
+                                       np.zeros(1))]).astype(np.float32)
+    n += 1
+    ty, ts = np.zeros(n, np.uint32), np.ones(n, np.int8)
+    c = _hrt.Context(0)
+    c.update_geometry(T, ty, ts)
+    c.build_accel()
+    d = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 0, "position": (0.0, 0.0, 1.0), "width": (0.0, 0.0)}],
+         "source_flux": np.zeros((1, 1)), "rho": np.full((1, n, 1), 0.3), "tau": np.full((1, n, 1), 0.2),
+         "diffuse_flux": np.array([100.0]), "direct_rays": np.array([0]), "diffuse_rays": np.array([64]),
+         "depth": np.array([1]), "emission": np.array([0], np.uint8), "seed": 3}
+    c.set_tuning(16 + variant)
+    got = c.run_band(d).astype(np.float64)
+    full = dict({k: None for k in ("diffuse_ext", "diffuse_norm", "diffuse_peak", "prague", "eps", "temperature")}, **d)
+    ref, _ = oracle_mod.OracleScene(T, ty, ts).run_band(oracle_solve(full))
+    floor = 1e-3 * float(np.abs(ref).mean())
+    assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
+    assert c.device_status() == 0
