@@ -84,9 +84,9 @@ void keep_pool(int device) {
 }
 
 // Do the voxels form a regular lattice?  Boxes as the records hold them (make_records, FP32): equal
-// sides, corners on the planes of one lattice within a thousandth of a cell, no cell twice, and not
-// so sparse that the table of cells outgrows them 16 times.  Fills g but for its device pointer and
-// the cells [x fastest] as the march reads them.
+// sides, corners on the planes of one lattice within a thousandth of a cell, no cell twice, and at least
+// half of the cells in use: at one in ten the march took 0.91 to 1.79 times the time of the tree of
+// everything.  Fills g but for its device pointer and the cells [x fastest] as the march reads them.
 bool find_lattice(const float *T, const std::vector<uint32_t> &vox, const float *lad, float far, VoxGrid *g,
                   std::vector<float4> *cells) {
     if (vox.empty()) return false;
@@ -119,7 +119,7 @@ bool find_lattice(const float *T, const std::vector<uint32_t> &vox, const float 
         cellsn *= n;
         ext = std::max(ext, end[a] - org[a]);
     }
-    if (cellsn > 16.0 * (double)nv + 64.0) return false;
+    if (cellsn > 2.0 * (double)nv + 64.0) return false;
     double off = 0.0;
     cells->assign(2 * (size_t)cellsn, make_float4(0.f, 0.f, 0.f, 0.f));
     for (size_t i = 0; i < nv; ++i) {
@@ -148,11 +148,24 @@ bool find_lattice(const float *T, const std::vector<uint32_t> &vox, const float 
         g->org[a] = (float)org[a];
         g->size[a] = (float)size[a];
         g->inv[a] = (float)(1.0 / size[a]);
-        g->tolf[a] = (float)(tol / size[a]);
-        if (!(g->tolf[a] < 0.1f)) return false;
+        if (!(tol < 0.1 * size[a])) return false;  // close to a face must not mean anywhere in the cell
     }
     g->tol = (float)tol;
     return true;
+}
+
+// Whether passes too short to time both forms march a lattice: one of at most 64 cells an axis that is full
+// (seven of eight cells in use) beside 8,192 surfaces or more or at most two for each voxel, or half full
+// beside 65,536.  Time of the march over the generic trace's, open and periodic, full lattices of 3 to 24 cells an
+// axis under a leaf area density of 1: 100,000 leaves 0.69-0.78 and 0.71-0.88, 16,000 0.70-0.89 and
+// 0.73-0.97, 4,000 and 3 to 10 cells 0.94-1.02 and 0.98-1.14, 14 and 24 cells 0.74-0.85 and 0.76-0.89, 2,000
+// 0.96-1.00 and 1.01-1.17, 0.74-0.88 and 0.73-0.91.  Half-full ones 0.84-0.93 and 0.97-1.02 with 100,000,
+// 0.92-0.99 and 0.99-1.11 with 16,000.  Under a density of 18, where rays end on leaves before the cells
+// that were marched, 1.07-1.18 and 1.14-1.21.  A line of 1,024 cells: 7.
+bool march_pays(size_t voxels, size_t cells, size_t surfaces, int axis) {
+    const bool full = 8 * voxels >= 7 * cells;
+    const bool half = 2 * voxels >= cells;
+    return axis <= 64 && ((full && (surfaces >= 8192 || 2 * voxels >= surfaces)) || (half && surfaces >= 65536));
 }
 
 }  // namespace
@@ -178,6 +191,7 @@ struct hrt_context {
     int n4 = 0;  // compressed 4-wide nodes built
     // a lattice of voxels: its description, cells and the 4-wide nodes over the other primitives
     bool have_lattice = false, use_lattice = false;
+    bool march = false;  // TraceScene::march
     DevBuf vg, vg_cells, nodes4s;
     int n4s = 0;
     // materials and sources
@@ -282,6 +296,7 @@ TraceScene scene_of(hrt_context *ctx) {
     sc.nodes4s = ctx->use_lattice ? ctx->nodes4s.as<float4>() : nullptr;
     sc.n4s = ctx->use_lattice ? ctx->n4s : 0;
     sc.vgrid = ctx->use_lattice ? ctx->vg.as<VoxGrid>() : nullptr;
+    sc.march = ctx->march ? 1 : 0;
     sc.rgen = ctx->rgen.as<float4>();
     sc.bbox = ctx->nbbox ? ctx->bbox.as<float4>() : nullptr;
     sc.n = ctx->n;
@@ -710,6 +725,10 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
 // per (mode, n, count, rays per face, faces, bands, voxels); passes under kTuneMinRays
 // rays keep the default.  Choices differ only in the order of the FP64 atomic sums.
 constexpr long long kTuneMinRays = 20000000;
+// Passes over a lattice of voxels are timed from here on, the march against the generic trace, on a sample
+// of 1 M rays (a wave of the device is 0.16 M): which is faster depends on the density of leaves and cells,
+// and the one costs up to 1.4 times the other.
+constexpr long long kTuneMinRaysLattice = 8000000;
 
 const char *variant_name(int v) {
     switch (v) {
@@ -739,8 +758,8 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
         if (!(record && v == DV_SIMPLE)) *variant = v;
         return HRT_OK;
     }
-    if (!ctx->tune || rays < kTuneMinRays) return HRT_OK;
-    if (!record && P0.sc.vgrid) return HRT_OK;  // a marched lattice has one kernel
+    const bool lattice = !record && P0.sc.vgrid;
+    if (!ctx->tune || rays < (lattice ? kTuneMinRaysLattice : kTuneMinRays)) return HRT_OK;
     char key[160];
     std::snprintf(key, sizeof key, "%s n=%d count=%u rays_per_face=%d faces=%d bands=%d voxels=%d",
                   record ? "record" : "accumulate", ctx->n, P0.count, P0.dimx * P0.dimy, P0.faces, P0.Bc,
@@ -757,12 +776,13 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
     // periodic stand's first solve.  hrt_set_tuning still forces any of them.
     std::vector<int> cand;
     const bool w4 = P0.sc.nodes4 != nullptr;
-    if (!record && P0.sc.voxels) cand = w4 ? std::vector<int>{DV_W4, DV_PS4} : std::vector<int>{DV_PS4, DV_SIMPLE};
+    if (lattice) cand = {DV_W4S4D16, DV_W4};  // the march and the one tree of everything
+    else if (!record && P0.sc.voxels) cand = w4 ? std::vector<int>{DV_W4, DV_PS4} : std::vector<int>{DV_PS4, DV_SIMPLE};
     else if (w4) cand = {DV_W4S4D16, DV_W4S4D32, DV_W4S4};
     else if (record) cand = {DV_PS3, DV_PS4};
     else cand = {DV_PS4, DV_PS3, DV_SIMPLE};
     DiffuseParams P = P0;
-    P.count = std::min(P0.count, std::max(P0.count / 32u, 4096u));
+    P.count = std::min(P0.count, std::max(P0.count / 32u, lattice ? (uint32_t)(1000000 / (P0.dimx * P0.dimy * nf)) + 1u : 4096u));
     // the sample is one launch: keep it within the per-launch ray limit
     P.count = std::min(P.count, std::max(launch_chunk_prims((uint64_t)P0.dimx * P0.dimy * nf, ctx->ray_limit), 1u));
     P.sc.rays = nullptr;
@@ -1293,7 +1313,7 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
     CU(launch_prim_area((int)n, ctx->T.as<float>(), ctx->type.as<uint32_t>(), ctx->lad.as<float>(),
                         ctx->area.as<double>(), ctx->stream));
     ctx->wall_far = largest_coordinate(g->bbox_vertices, 12 * (size_t)g->nbbox);
-    ctx->have_lattice = ctx->use_lattice = false;
+    ctx->have_lattice = ctx->use_lattice = ctx->march = false;
     if (!voxels.empty() && voxels.size() + 2 <= n) {
         // rays start on primitives and, wrapped, on the walls
         const float reach = primitives_reach(g->transform, n);
@@ -1306,6 +1326,7 @@ int hrt_update_geometry(hrt_context *ctx, const hrt_geometry *g) {
         } catch (const std::bad_alloc &) {
         }
         if (ctx->have_lattice) {
+            ctx->march = march_pays(voxels.size(), cells.size() / 2, n - voxels.size(), std::max({vg.n[0], vg.n[1], vg.n[2]}));
             const cudaError_t e = ctx->vg_cells.ensure(ctx->stream, cells.size() * sizeof(float4));
             if (e == cudaErrorMemoryAllocation) {
                 cudaGetLastError();

@@ -15,7 +15,7 @@ namespace hrt {
 struct VoxGrid {
     float org[3], size[3], inv[3];  // lower corner, cell sides and their inverses
     int n[3];                       // cells per axis
-    float tol, tolf[3];             // closeness to a cell face: a length, and per axis in cells
+    float tol;                      // closeness to a cell face
     const float4 *cells;            // [n0*n1*n2*2] (lo.xyz, extinction), (hi.xyz, original index); extinction 0: empty
 };
 
@@ -51,6 +51,7 @@ struct TraceScene {
     const float4 *nodes4s; // [n4s*4] 4-wide nodes over the surfaces alone (scenes with a voxel lattice)
     int n4s;
     const VoxGrid *vgrid; // the lattice (null: none; voxels are leaves of the tree)
+    int march;            // default diffuse passes march the lattice
     const float4 *rgen;   // [n*4] ray-origin records, original order
     const float4 *bbox;   // [nbbox*4] periodic wall corners (xyz, w unused)
     int n;

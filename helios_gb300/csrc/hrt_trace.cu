@@ -797,9 +797,12 @@ template <bool STATS>
 static cudaError_t diffuse_impl(const DiffuseParams &p, int variant, int max_blocks, cudaStream_t s) {
     int64_t total = (int64_t)p.count * p.dimx * p.dimy;
     if (total <= 0 || p.Bc <= 0) return cudaSuccess;
-    if (variant == DV_DEFAULT) variant = default_variant();
+    if (variant == DV_DEFAULT) {
+        variant = default_variant();
+        if (is_w4s_variant(variant) && p.sc.vgrid && !p.sc.march) variant = DV_W4;
+    }
     if ((variant == DV_W4 || variant == DV_W43 || is_w4s_variant(variant)) && !p.sc.nodes4) variant = DV_PS4;
-    // voxels that form a lattice: the lean trace marches them; others are leaves of the generic one
+    // voxels that form a lattice: the lean shapes stand for its march; others are leaves of the generic trace
     if (is_w4s_variant(variant) && p.sc.voxels) {
         if (!STATS && p.sc.vgrid && p.fetch) return launch_w4s_voxels(p, s);
         variant = DV_W4;

@@ -425,3 +425,60 @@ def test_deep_stacks_that_fit(hrt_lib, oracle_mod, variant, n):
     floor = 1e-3 * float(np.abs(ref).mean())
     assert float((np.abs(got - ref) / np.maximum(np.abs(ref), floor)).max()) <= 1e-4
     assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("form", ["full", "half", "sparse", "line", "dense leaves"])
+def test_lattices_are_marched_where_it_pays(hrt_lib, form):
+    """Lattices of voxels that are full, half full, one cell in sixteen, a line of a thousand cells, and
+    full among dense leaves: a diffuse pass takes no longer than a quarter more than the generic trace."""
+    div, occupied, ext = {"full": ((10, 10, 10), 1.0, 4.0), "half": ((10, 10, 10), 0.5, 4.0), "sparse": ((40, 40, 40), 1 / 15.5, 4.0),
+                          "line": ((1024, 1, 1), 1.0, 4.0), "dense leaves": ((24, 24, 24), 1.0, 1.5)}[form]
+    rng = np.random.default_rng(5)
+    lv = scenes.mixed_canopy(16000, 16000 * 0.0025 / ext ** 2, seed=2, height=1.0)
+    v = scenes.voxel_grid((0.0, 0.0, 0.05), (ext, ext, 1.0), div, rng.uniform(0.0, 2.0, int(np.prod(div))))
+    keep = rng.random(v.n) < occupied
+    keep[0] = keep[-1] = True
+    T, lad = np.concatenate([lv.T, v.T[keep]]), np.concatenate([np.zeros(lv.n), v.lad[keep]])
+    n = T.shape[0]
+    c = _hrt.Context(0)
+    c.update_geometry(T, np.concatenate([lv.ptype, v.ptype[keep]]), np.concatenate([lv.twosided, v.twosided[keep]]), None,
+                      (0.0, 0.0), lad)
+    c.build_accel()
+    d = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 0, "position": (0.0, 0.0, 1.0)}],
+         "source_flux": np.zeros((1, 1)), "rho": np.zeros((1, n, 1)), "tau": np.zeros((1, n, 1)), "diffuse_flux": np.array([100.0]),
+         "direct_rays": np.array([0]), "diffuse_rays": np.array([100]), "depth": np.array([0]),
+         "emission": np.array([0], np.uint8), "seed": 3}
+    got, ms = c.run_band(d).astype(np.float64), _direct_ms(c, d)
+    c.set_tuning(16 + 4)
+    generic, generic_ms = c.run_band(d).astype(np.float64), _direct_ms(c, d)
+    assert np.all(np.abs(got - generic) <= 2.4e-7 * np.abs(generic))
+    assert ms <= 1.25 * generic_ms, (ms, generic_ms)
+
+
+@pytest.mark.parametrize("form", ["full", "holes", "layer", "shifted", "far"])
+@pytest.mark.parametrize("walls", [False, True])
+def test_march_equals_the_tree_of_everything(hrt_lib, form, walls):
+    """The march and the generic trace, each forced, give the same fluxes and ray counts; passes of scenes
+    of this size run the generic one by themselves."""
+    T, ty, ts, lad = _voxel_scene(form)
+    n = T.shape[0]
+    c = _hrt.Context(0)
+    lo, hi = T.reshape(-1, 16)[:, [3, 7, 11]].min(0) - 0.6, T.reshape(-1, 16)[:, [3, 7, 11]].max(0) + 0.6
+    (x0, y0, z0), (x1, y1, z1) = lo, hi
+    bb = np.array([[(x0, y0, z0), (x0, y1, z0), (x0, y1, z1), (x0, y0, z1)], [(x1, y0, z0), (x1, y1, z0), (x1, y1, z1), (x1, y0, z1)],
+                   [(x0, y0, z0), (x1, y0, z0), (x1, y0, z1), (x0, y0, z1)], [(x0, y1, z0), (x1, y1, z0), (x1, y1, z1), (x0, y1, z1)]],
+                  np.float32)
+    c.update_geometry(T, ty, ts, bb if walls else None, (1.0, 1.0) if walls else (0.0, 0.0), lad)
+    c.build_accel()
+    d = {"band_launch": np.array([1], np.uint8), "sources": [{"type": 0, "position": (0.0, 0.0, 1.0)}],
+         "source_flux": np.zeros((1, 1)), "rho": np.full((1, n, 1), 0.4), "tau": np.full((1, n, 1), 0.3),
+         "diffuse_flux": np.array([100.0]), "direct_rays": np.array([0]), "diffuse_rays": np.array([400]), "depth": np.array([2]),
+         "emission": np.array([0], np.uint8), "seed": 3}
+    got = []
+    for mode in (16 + 8, 16 + 4, 0):
+        c.set_tuning(mode)
+        got.append((c.run_band(d).astype(np.float64), c.last_stats()["rays"]))
+    for flux, rays in got[1:]:
+        assert rays == got[0][1]
+        assert np.all(np.abs(flux - got[0][0]) <= 2.4e-7 * np.abs(got[0][0]))
+    assert c.device_status() == 0
