@@ -725,10 +725,6 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
 // per (mode, n, count, rays per face, faces, bands, voxels); passes under kTuneMinRays
 // rays keep the default.  Choices differ only in the order of the FP64 atomic sums.
 constexpr long long kTuneMinRays = 20000000;
-// Passes over a lattice of voxels are timed from here on, the march against the generic trace, on a sample
-// of 1 M rays (a wave of the device is 0.16 M): which is faster depends on the density of leaves and cells,
-// and the one costs up to 1.4 times the other.
-constexpr long long kTuneMinRaysLattice = 8000000;
 
 const char *variant_name(int v) {
     switch (v) {
@@ -759,7 +755,7 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
         return HRT_OK;
     }
     const bool lattice = !record && P0.sc.vgrid;
-    if (!ctx->tune || rays < (lattice ? kTuneMinRaysLattice : kTuneMinRays)) return HRT_OK;
+    if (!ctx->tune || rays < kTuneMinRays) return HRT_OK;
     char key[160];
     std::snprintf(key, sizeof key, "%s n=%d count=%u rays_per_face=%d faces=%d bands=%d voxels=%d",
                   record ? "record" : "accumulate", ctx->n, P0.count, P0.dimx * P0.dimy, P0.faces, P0.Bc,
@@ -782,6 +778,7 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
     else if (record) cand = {DV_PS3, DV_PS4};
     else cand = {DV_PS4, DV_PS3, DV_SIMPLE};
     DiffuseParams P = P0;
+    // (a lattice's: 1 M rays, some six waves of the device; its kernels are several times slower)
     P.count = std::min(P0.count, std::max(P0.count / 32u, lattice ? (uint32_t)(1000000 / (P0.dimx * P0.dimy * nf)) + 1u : 4096u));
     // the sample is one launch: keep it within the per-launch ray limit
     P.count = std::min(P.count, std::max(launch_chunk_prims((uint64_t)P0.dimx * P0.dimy * nf, ctx->ray_limit), 1u));
