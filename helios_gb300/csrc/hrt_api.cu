@@ -2568,10 +2568,12 @@ int hrt_run_sweep_multi(hrt_context *const *ctxs, const hrt_sweep *sweeps, int32
         total += rays[k];
         uint32_t word = 0;  // each scene's device error word (the graph ran on ctx's stream)
         CU(cudaMemcpy(&word, ctxs[k]->status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-        if (word && status == HRT_OK) {
-            int rk = sync_and_status(ctxs[k]);
-            status = rk;
-            if (k > 0) fail(ctx, rk, std::string("scene ") + std::to_string(k) + ": " + ctxs[k]->err);
+        if (word) {  // every failing scene's word is cleared, the first one is reported
+            const std::string first = ctx->err;
+            const int rk = sync_and_status(ctxs[k]);
+            if (status != HRT_OK) ctx->err = first;
+            else if (k > 0) fail(ctx, rk, std::string("scene ") + std::to_string(k) + ": " + ctxs[k]->err);
+            if (status == HRT_OK) status = rk;
         }
     }
     ctx->multi_rays = total;

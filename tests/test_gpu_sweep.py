@@ -131,10 +131,10 @@ def test_multi_scene_sweep_equals_each_scene_alone():
             assert c.device_status() == 0
 
 
-@pytest.mark.parametrize("bad", [0, 1, 2])
+@pytest.mark.parametrize("bad", [(0,), (1,), (2,), (1, 2)])
 def test_multi_scene_sweep_reports_the_failing_scene(bad):
-    """A scene whose rays run out of their visit budget in the recording launch (no direct pass, which
-    has its own checks): the call fails and names the scene, and the next one is clean."""
+    """Scenes whose rays run out of their visit budget in the recording launch (no direct pass, which
+    has its own checks): the call fails and names the first of them, and the next one is clean."""
     from helios_gb300 import _hrt
 
     ctxs, sweeps = [], []
@@ -148,12 +148,14 @@ def test_multi_scene_sweep_reports_the_failing_scene(bad):
                            rho=np.full((sc.n, 1), 0.3), tau=np.full((sc.n, 1), 0.2), direct_rays=25, diffuse_rays=49,
                            depth=1, seed=3))
     before = _hrt.run_sweep_multi(ctxs, sweeps)
-    ctxs[bad].set_visit_budget(2)
+    for k in bad:
+        ctxs[k].set_visit_budget(2)
     with pytest.raises(_hrt.HrtError) as e:
         _hrt.run_sweep_multi(ctxs, sweeps)
     assert e.value.code == _hrt.HRT_EDEVICE and "visit budget" in str(e.value)
-    assert bad == 0 or f"scene {bad}" in str(e.value)
-    ctxs[bad].set_visit_budget(0)
+    assert bad[0] == 0 or f"scene {bad[0]}" in str(e.value)
+    for k in bad:
+        ctxs[k].set_visit_budget(0)
     after = _hrt.run_sweep_multi(ctxs, sweeps)
     for a, b, c in zip(after, before, ctxs):
         np.testing.assert_allclose(a, b, rtol=1e-6, atol=1e-9)
