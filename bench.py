@@ -413,7 +413,8 @@ def run_stress(args, stream, device=0):
     st = ctx.last_stats()
     tuning = [x for x in ctx.tuning_report().splitlines() if x.startswith("accumulate")]
     # traversal counts (untimed) on the same workload scaled to 5 % of the primitives, with
-    # the kernel variant and tree the tuner chose for the full workload
+    # the kernel variant and tree the tuner chose for the full workload (the march of a voxel
+    # lattice has no statistics form: the generic 4-wide trace counts for it)
     small, _ = stress_model(0.05 * args.stress_scale, device=device)
     small.setSeed(99)
     small.updateGeometry()
@@ -431,7 +432,7 @@ def run_stress(args, stream, device=0):
             "primitives": int(sc.n), "s_per_solve": t, "rays_per_solve": st["rays"], "rays_per_s": st["rays"] / t,
             "scattering_iterations": st["iterations"], "kernels": st["kernels"], "setup_build_s": t_build,
             "node_visits_per_ray_5pct": meas["node_visits"] / small_rays,
-            "prim_tests_per_ray_5pct": meas["prim_tests"] / small_rays, "counted_variant": chosen,
+            "prim_tests_per_ray_5pct": meas["prim_tests"] / small_rays, "counted_variant": chosen if chosen in TUNER_VARIANTS else "wide4",
             "autotune": tuning}
 
 
@@ -565,12 +566,13 @@ def run_gpu(args):
                    "parallelism": "replicas" if world > 1 else "single",
                    "l2": "working set (BVH 64 MB + records 128 MB + buffers) larger than the 129 MB L2; no flush",
                    "setup_s": setup_s},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
+        "roofline": {"bound": "sm issue", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_kind": peak_kind, "traffic": traffic,
                      "kernel": "k_diffuse_w4" if chosen and chosen[0].startswith("lean") else "k_diffuse_ps",
                      "variant": chosen[0] if chosen else None,
-                     "limiter": "SM issue and L1/L2 hit latency of the node fetches, not DRAM: the algorithmic "
-                                "bytes are logical fetches, almost all served by L1/L2 (traffic = DRAM bytes)",
+                     "limiter": "SM issue and L1/L2 hit latency of the node fetches, not DRAM: achieved and frac are "
+                                "logical fetches over the measured HBM copy rate, almost all of them served by L1/L2 "
+                                "(traffic = DRAM bytes)",
                      "ncu": dict(PROFILE, sources_now=digest, stale=not fresh),
                      "kernel_ms": diff_ms, "kernel_share": diff_share, "bytes_per_launch": bytes_per_launch,
                      "rays_per_launch": rays_per_launch,

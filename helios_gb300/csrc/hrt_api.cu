@@ -723,7 +723,7 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
 // first max(count/32, 4096) primitives, written to scratch sums (or the hit buffer of a
 // recorded pass, rewritten by the real pass) and not counted.  The choice is cached
 // per (mode, n, count, rays per face, faces, bands, voxels); passes under kTuneMinRays
-// rays keep the default.  Choices differ only in the order of the FP64 atomic sums.
+// rays keep the default.  Over a lattice of voxels the candidates are its march and the generic trace.  Choices differ only in the order of the FP64 atomic sums.
 constexpr long long kTuneMinRays = 20000000;
 
 const char *variant_name(int v) {

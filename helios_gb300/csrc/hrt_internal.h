@@ -319,10 +319,10 @@ size_t bvh4_scratch_bytes(int n);
 size_t bvh4_node_capacity(int n);
 cudaError_t bvh4_build(const float4 *nodes2, int n, float4 *nodes4, void *scratch, uint32_t *status, int *count_out,
                        cudaStream_t s);
-// lad: [n] leaf area density of voxels (original order), or null (voxels then hold no leaves).
 // Primitive areas (voxels: leaf area), T 16-byte aligned; lad read for voxels.
 cudaError_t launch_prim_area(int n, const float *T, const uint32_t *type, const float *lad, double *area,
                              cudaStream_t s);
+// lad: [n] leaf area density of voxels (original order), or null (voxels then hold no leaves).
 cudaError_t bvh_build(const float *T, const uint32_t *type, const float *lad, int n, BvhBuffers &b, cudaStream_t s);
 constexpr int kSortTile = 2048;
 
@@ -335,9 +335,10 @@ cudaError_t launch_diffuse(const DiffuseParams &p, int max_blocks, cudaStream_t 
 enum DiffuseVariant {
     DV_DEFAULT = 0, DV_PS4 = 1, DV_PS3 = 2, DV_SIMPLE = 3, DV_W4 = 4, DV_W43 = 5,
     // lean 4-wide trace (k_diffuse_w4): threads per block x resident blocks per SM, shared
-    // stack entries per lane (r: a ring over local memory, l: the bottom entries), ray ids a
-    // warp takes per fetch (32 x batch) -- 256 x 4, 8r, 1; 256 x 5, 8r, 1; 256 x 4, 16l, 1;
-    // 128 x 8, 8r, 1; 512 x 2, 8r, 1; 256 x 4, 8r, 4; 256 x 4, 8r, 16; 256 x 4, 32l, 1
+    // stack entries per lane, ray ids a warp takes per fetch (32 x batch) -- 256 x 4, 8, 1;
+    // 256 x 5, 8, 1; 256 x 4, 16, 1; 128 x 8, 8, 1; 512 x 2, 8, 1; 256 x 4, 8, 4; 256 x 4, 8, 16;
+    // 256 x 4, 32, 1.  The tuner tries W4S4, W4S4D16 and W4S4D32; the others, W43 among them, are
+    // reached by hrt_set_tuning alone
     DV_W4S4 = 6, DV_W4S5 = 7, DV_W4S4D16 = 8, DV_W4B128 = 9, DV_W4B512 = 10, DV_W4K4 = 11, DV_W4K16 = 12,
     DV_W4S4D32 = 13, DV_LAST = DV_W4S4D32
 };

@@ -41,7 +41,10 @@ constexpr int32_t kSentinel = 0x7FFFFFF0;  // no node (empty stack, missed child
 constexpr int kStack4 = 128;               // a 4-wide node pushes up to three children
 
 // Slab offsets of a compressed 4-wide node for a ray: b = (p - o) * inv per axis, p the origin of
-// the node's frame (q0.xyz).
+// the node's frame (q0.xyz), one frame extent S below the node box.  A slab plane then is offset by S more
+// than its distance asks for and rounds by up to 2^-24 S |inv| more: S is at most twice the node box's side,
+// so in space 2^-23 of the scene's extent at the root and less below, an eighth of the leaf-box
+// padding ((|x| + extent) 2^-20, extent the scene's).
 __device__ __forceinline__ f3 node4_offset(const float4 q0, f3 o, f3 inv) {
     return mk((q0.x - o.x) * inv.x, (q0.y - o.y) * inv.y, (q0.z - o.z) * inv.z);
 }

@@ -20,6 +20,9 @@
 // the 32 lanes of a warp always hit 32 different banks); they move to local memory all at once when
 // they run out (LaneStack).  Local memory is touched only by rays whose stack is deeper than SD.
 //
+// Scenes with a lattice of voxels run it as the march (VG) where that is the faster form (march_pays and
+// the tuner, hrt_api.cu).
+//
 // Hits equal those of trace_bvh / k_diffuse_ps: the same node and primitive tests, the same
 // tie rule (closest, then smaller original index); only the order of work differs.
 #pragma once
@@ -102,7 +105,7 @@ struct LaneStack {
 };
 
 // BLOCK: threads per block; MINB: resident blocks per SM the register allocation must allow.
-// SD: stack entries per lane in shared memory (a power of two).  KB: ray-id batch -- a warp
+// SD: stack entries per lane in shared memory.  KB: ray-id batch -- a warp
 // takes 32 x KB consecutive ray ids from the global counter at a time and hands them to its
 // idle lanes from shared memory (KB = 1: every refill takes exactly the idle lanes' count).
 // MULTI (recording mode only): the launch traces several scenes -- P.slots[0..P.nslots) each

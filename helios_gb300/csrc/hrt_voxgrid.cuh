@@ -2,9 +2,11 @@
 //
 // Voxels are large boxes over the leaves, so a tree that holds both has overlapping nodes and a ray
 // visits most of the voxels it crosses through several of them.  Where the voxels of a scene are
-// cells of one regular lattice (the host checks it, find_lattice in hrt_api.cu), a ray steps through
-// the cells in order and stops at its first interception, which then bounds the walk through a tree
-// of the other primitives alone.  Each cell makes the test of the tree's leaves (voxel_hit: the same
+// cells of one regular lattice (the host checks it, find_lattice in hrt_api.cu), a ray can step through
+// the cells in order (after Amanatides and Woo, "A Fast Voxel Traversal Algorithm for Ray Tracing",
+// Eurographics 1987) and stop at its first interception, which then bounds the walk through a tree
+// of the other primitives alone.  Sparse lattices, few surfaces and dense leaves are faster in the one tree
+// (march_pays in hrt_api.cu has both sides).  Each cell makes the test of the tree's leaves (voxel_hit: the same
 // box, extinction and random number), so the closest interception is the tree's.  Measured on a section
 // of the deep-scattering scene (16,001 leaves and 1,000 voxels, periodic, 285 M diffuse rays): 59.8 node
 // visits and 11.6 tests per ray in one tree, 39.7 visits, 2.8 tests and 9.7 cells here; 422 -> 362 ms
