@@ -146,10 +146,11 @@ struct SunGrid {
     float u0, v0, inv_h, pad;
     int nu, nv;
     uint32_t total;        // entries
-    unsigned long long sq; // sum over the cells of their squared counts
     uint32_t ok;           // 0: no frame; the source's rays go through the tree
     uint32_t nlarge;
     uint2 large[kSunLarge];
+    uint32_t served;       // the grid traces its source: written as the entries are filled, from counts that are final
+    unsigned long long sq; // sum over the cells of their squared counts
 };
 struct SunCaps {
     uint32_t cells, entries;  // buffer sizes per source

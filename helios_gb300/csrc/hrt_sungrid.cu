@@ -146,14 +146,15 @@ __global__ void k_sun_setup(int nb, const float *__restrict__ dirs, int dir_stri
     g.nv = fine ? nv : 1;
     g.ok = fine ? 1u : 0u;
     g.total = 0u;
+    g.served = 0u;
     g.sq = 0ull;
     g.nlarge = 0u;
     grids[b] = g;
 }
 
 // Whether a binned source is traced by its grid: its entries fit, few primitives are wide and the cells
-// are not crowded.  The
-// flag of the frame is written once, by k_sun_setup, so that all threads of a block agree on it.
+// are not crowded.  The flag of the frame is written once, by k_sun_setup, and this once, by one thread of
+// the filling launch, so that the threads of a block agree on both.
 __device__ __forceinline__ bool sun_served(const SunGrid &g, uint32_t entries_cap, int n) {
     return g.ok && g.nlarge <= (uint32_t)kSunLarge && g.total <= entries_cap && g.sq <= sun_crowd(n) * g.total;
 }
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_bin(int n, const float4 *__
     SunGrid *G = grids + blockIdx.y;
     const SunGrid &g = *G;
     const bool on = FILL ? sun_served(g, entries_cap, n) : g.ok != 0u;
-    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) done[blockIdx.y] = on ? 1u : 0u;
+    if (FILL && blockIdx.x == 0 && threadIdx.x == 0) done[blockIdx.y] = G->served = on ? 1u : 0u;
     if (!on) return;
     uint2 *cl = cells + (size_t)blockIdx.y * cells_cap;
     uint2 *en = entries + (size_t)blockIdx.y * entries_cap;
@@ -275,8 +276,8 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uin
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, d);
-    if ((threadIdx.x & 31) == 0 && sq) atomicAdd(&G->sq, sq);
     __shared__ uint32_t sh[kSunThreads / 32];
+    __shared__ unsigned long long sh_sq[kSunThreads / 32];
     __shared__ uint32_t first;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = sum;
@@ -286,14 +287,18 @@ __global__ void __launch_bounds__(kSunThreads) k_sun_offsets(SunGrid *grids, uin
         if (lane >= d) x += y;
     }
     if (lane == 31) sh[warp] = x;
+    if (lane == 0) sh_sq[warp] = sq;
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t t = 0;
+        sq = 0;
         for (int w = 0; w < kSunThreads / 32; ++w) {
             const uint32_t s = sh[w];
             sh[w] = t;
             t += s;
+            sq += sh_sq[w];
         }
+        if (sq) atomicAdd(&G->sq, sq);
         first = t ? atomicAdd(&G->total, t) : 0u;  // at most kSunWide entries of 2^25 primitives: no wrap
     }
     __syncthreads();
@@ -352,11 +357,6 @@ __global__ void __launch_bounds__(kSunThreads, 4) k_direct_sun(const SunDirectPa
         for (uint32_t i = threadIdx.x; i < (uint32_t)P.nb * (sizeof(SunGrid) / sizeof(uint32_t)); i += kSunThreads)
             dst[i] = src[i];
         __syncthreads();
-        if (threadIdx.x < (unsigned)P.nb) {
-            SunGrid &g = s_grid[threadIdx.x];
-            g.ok = sun_served(g, P.entries_cap, P.sc.n) ? 1u : 0u;
-        }
-        __syncthreads();
     }
     unsigned long long nrays = 0;
     for (uint32_t base = blockIdx.x * kSunThreads + (threadIdx.x & ~31u); base < total; base += stride) {
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kSunThreads, 4) k_direct_sun(const SunDirectPa
         }
         for (int b = 0; b < P.nb; ++b) {
             const SunGrid &g = s_grid[b];
-            if (!g.ok) continue;
+            if (!g.served) continue;
             const uint32_t k = (uint32_t)(P.first + b);
             const uint32_t c2 = SHARED ? 0u : (k << 1);
             const bool face = vox || dot(g.s, nrm) > 0.f;
