@@ -563,6 +563,9 @@ int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
     if (*nb == 0) return HRT_OK;
     cudaError_t e = ctx->sg_cells.ensure(ctx->stream, (size_t)*nb * caps.cells * sizeof(uint2));
     if (e == cudaSuccess) e = ctx->sg_entries.ensure(ctx->stream, (size_t)*nb * caps.entries * sizeof(uint2));
+    if (e == cudaSuccess) e = ctx->sg_grids.ensure(ctx->stream, (size_t)kSunBatch * sizeof(SunGrid));
+    if (e == cudaSuccess) e = ctx->sg_done.ensure(ctx->stream, (size_t)std::max(nsrc, 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = ctx->sg_extent.ensure(ctx->stream, 9 * sizeof(uint32_t));
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         ctx->sg_cells.free_on(ctx->stream);
@@ -571,9 +574,6 @@ int ensure_sun_grids(hrt_context *ctx, int nsrc, int *nb) {
         return HRT_OK;
     }
     CU(e);
-    CU(ctx->sg_grids.ensure(ctx->stream, (size_t)kSunBatch * sizeof(SunGrid)));
-    CU(ctx->sg_done.ensure(ctx->stream, (size_t)std::max(nsrc, 1) * sizeof(uint32_t)));
-    CU(ctx->sg_extent.ensure(ctx->stream, 9 * sizeof(uint32_t)));
     if (!ctx->sg_extent_ready) {
         CU(launch_scene_extent(ctx->n, ctx->rec.as<float4>(), ctx->sg_extent.as<uint32_t>(), ctx->stream));
         ctx->sg_extent_ready = true;

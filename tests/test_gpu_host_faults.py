@@ -56,7 +56,7 @@ def _voxel_context():
     return c, leaves.n
 
 
-@pytest.mark.parametrize("what", ["cells", "second tree", "sun cells", "sun entries"])
+@pytest.mark.parametrize("what", ["cells", "second tree", "sun cells", "sun entries", "sun frames"])
 def test_optional_buffers_without_memory(fakes, what):
     """Buffers that a call can do without: the cells of a voxel lattice, the tree of the surfaces beside
     it, and the grids of a direct pass.  Without memory for them the call gives the same fluxes."""
@@ -65,7 +65,8 @@ def test_optional_buffers_without_memory(fakes, what):
     n = c.n
     d = _solve(n, [{"type": 0, "position": (0.3, 0.2, 0.9)}])
     want = c.run_band(d).astype(np.float64)
-    size = {"cells": 2 * 16 * 6 * 5 * 4, "second tree": 64 * (ns - 1 + 8), "sun cells": 8 * 8 * n, "sun entries": 8 * 16 * n}
+    size = {"cells": 2 * 16 * 6 * 5 * 4, "second tree": 64 * (ns - 1 + 8), "sun cells": 8 * 8 * n, "sun entries": 8 * 16 * n,
+            "sun frames": 32 * 384}
     sun = what.startswith("sun")  # cells are as large as the transforms: fail them from the solve on
     fakes.fake_fail_allocations(0 if sun else size[what], 0)
     c, _ = _voxel_context()
