@@ -351,7 +351,8 @@ int hrt_run_sweep_multi(hrt_context *const *ctxs, const hrt_sweep *sweeps, int32
  * after hrt_server_start) and one runBand's parameters; a dispatcher thread admits them
  * in arrival order when the scene's device context is idle and its footprint fits in
  * hbm_budget_bytes (least-recently-used idle scenes are evicted; resident scenes keep
- * their BVH and buffers).  Arrived requests of the same scene with the same band set,
+ * their BVH and buffers).  Memory that no scene needs serves the grids of the batches'
+ * suns, which solves can do without.  Arrived requests of the same scene with the same band set,
  * ray counts, depth and seed are batched (up to 64 requests, 256 channels) into one
  * hrt_run_sweep: direct rays per request sun, diffuse and scattering passes traced once.
  * Worker threads run the batches on per-scene CUDA streams, so solves of different
