@@ -430,7 +430,7 @@ def test_deep_stacks_that_fit(hrt_lib, oracle_mod, variant, n):
 @pytest.mark.parametrize("form", ["full", "half", "sparse", "line", "dense leaves"])
 def test_lattices_are_marched_where_it_pays(hrt_lib, form):
     """Lattices of voxels that are full, half full, one cell in sixteen, a line of a thousand cells, and
-    full among dense leaves: a diffuse pass takes no longer than a quarter more than the generic trace."""
+    full among dense leaves: a diffuse pass takes at most 1.4 times as long as the generic trace."""
     div, occupied, ext = {"full": ((10, 10, 10), 1.0, 4.0), "half": ((10, 10, 10), 0.5, 4.0), "sparse": ((40, 40, 40), 1 / 15.5, 4.0),
                           "line": ((1024, 1, 1), 1.0, 4.0), "dense leaves": ((24, 24, 24), 1.0, 1.5)}[form]
     rng = np.random.default_rng(5)
@@ -452,7 +452,7 @@ def test_lattices_are_marched_where_it_pays(hrt_lib, form):
     c.set_tuning(16 + 4)
     generic, generic_ms = c.run_band(d).astype(np.float64), _direct_ms(c, d)
     assert np.all(np.abs(got - generic) <= 2.4e-7 * np.abs(generic))
-    assert ms <= 1.25 * generic_ms, (ms, generic_ms)
+    assert ms <= 1.4 * generic_ms, (ms, generic_ms)
 
 
 @pytest.mark.parametrize("form", ["full", "holes", "layer", "shifted", "far"])
