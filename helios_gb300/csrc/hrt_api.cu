@@ -723,7 +723,8 @@ int direct_pass(hrt_context *ctx, uint32_t offset, uint32_t count, uint32_t rpp,
 // first max(count/32, 4096) primitives, written to scratch sums (or the hit buffer of a
 // recorded pass, rewritten by the real pass) and not counted.  The choice is cached
 // per (mode, n, count, rays per face, faces, bands, voxels); passes under kTuneMinRays
-// rays keep the default.  Over a lattice of voxels the candidates are its march and the generic trace.  Choices differ only in the order of the FP64 atomic sums.
+// rays keep the default.  Over a lattice of voxels the candidates are its march and the generic
+// trace.  Choices differ only in the order of the FP64 atomic sums.
 constexpr long long kTuneMinRays = 20000000;
 
 const char *variant_name(int v) {
@@ -779,7 +780,8 @@ int tuned_variant(hrt_context *ctx, const DiffuseParams &P0, bool record, int *v
     else cand = {DV_PS4, DV_PS3, DV_SIMPLE};
     DiffuseParams P = P0;
     // (a lattice's: 1 M rays, some six waves of the device; its kernels are several times slower)
-    P.count = std::min(P0.count, std::max(P0.count / 32u, lattice ? (uint32_t)(1000000 / (P0.dimx * P0.dimy * nf)) + 1u : 4096u));
+    const uint32_t least = lattice ? (uint32_t)(1000000 / (P0.dimx * P0.dimy * nf)) + 1u : 4096u;
+    P.count = std::min(P0.count, std::max(P0.count / 32u, least));
     // the sample is one launch: keep it within the per-launch ray limit
     P.count = std::min(P.count, std::max(launch_chunk_prims((uint64_t)P0.dimx * P0.dimy * nf, ctx->ray_limit), 1u));
     P.sc.rays = nullptr;
